@@ -324,6 +324,9 @@ __device__ __forceinline__ T till_temperature(const DevMat &m, T E, T rho)
     const double *t = m.tl;
     const double step = t[12];
     int dl = (int)(wind(floor(val(rho) / step), 0, m.cold_n - 2));
+    // a NaN density passes through wind, and its conversion to int is the most negative one:
+    // clamped once more as an index, so that the lookup stays inside the curve (the result is NaN)
+    dl = dl < 0 ? 0 : (dl > m.cold_n - 2 ? m.cold_n - 2 : dl);
     T dxl = dl + 1.0 - rho / step;
     T dxr = 1.0 - dxl;
     T ecold = dxl * m.cold_yeng[dl] + dxr * m.cold_yeng[dl + 1];
