@@ -63,7 +63,26 @@ enum StepKernel {
 };
 
 #ifdef __CUDACC__
-// flux: a0 = pass (0 interior, 1 pad); remap: a0..a3 = remap, damping, ejecta drag, EOS switches
+// Launch of a kernel that begins with grid_dependency() (salec_step.cu): programmatic stream
+// serialisation lets its blocks become resident before the previous kernel of the stream has
+// finished. In a captured graph the edge becomes a programmatic one. Errors are reported by
+// cudaGetLastError, as for any launch.
+template <class... P, class... A>
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// flux: a0 = pass (see k_flux), a1 = the tracers move in the same launch; remap: a0..a3 = remap, damping, ejecta drag, EOS switches
 // blk is the block shape of the 2-D sweeps (cells, faces, vertices); the surface profile, the
 // Laplacian mask, the tracer and the single-thread kernels use their own fixed shapes.
 template <class R>

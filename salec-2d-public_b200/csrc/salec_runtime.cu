@@ -161,16 +161,11 @@ struct salec_gpu {
     // tracer arrays, so changing either drops the graph)
     cudaGraphExec_t cycle_graph = nullptr;
     long long cycle_graph_launches = 0;
-    // in the captured cycle the tracer sweep runs on a side stream beside the flux sweep (it
-    // reads nothing the flux writes and writes only tracer arrays); joined before phase 13
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
     // its completion event and whether it is in flight
     Scal *report_scal[2] = {nullptr, nullptr};
     cudaEvent_t report_ev[2] = {nullptr, nullptr};
     bool report_pending[2] = {false, false};
-    bool fork_tracers = false;
     void *output = nullptr;     // output writer state (salec_output.cu)
     void *conserve = nullptr;   // scratch of the conservation sums (salec_conserve.cu)
     // prescribed time steps (salec_gpu_set_dt_schedule)
@@ -318,10 +313,10 @@ int run_gather(salec_gpu *h, const Gather &g)
     const int tb = 256, nb = (g.batch.total + tb - 1) / tb;
     h->launches += g.two_pass ? 2 : 1;
     if (!g.two_pass) {
-        k_gather<<<nb, tb, 0, h->stream>>>(g.batch, 0, nullptr);
+        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 0, nullptr);
     } else {
-        k_gather<<<nb, tb, 0, h->stream>>>(g.batch, 1, h->scratch);
-        k_gather<<<nb, tb, 0, h->stream>>>(g.batch, 2, h->scratch);
+        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 1, h->scratch);
+        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 2, h->scratch);
     }
     CUDA_TRY(cudaGetLastError());
     return SALEC_OK;
@@ -372,21 +367,13 @@ int run_phase_t(salec_gpu *h, int ph, bool fused)
         if (!fused) launch_step_kernel(SK_ENERGY, c, s, h->blk[SK_ENERGY]);
         break;
     case 11:
-        if (h->fork_tracers && h->tr.n > 0) {
-            CUDA_TRY(cudaEventRecord(h->ev_fork, s));
-            CUDA_TRY(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
-            launch_step_kernel(SK_TRACERS, c, h->side, h->blk[SK_TRACERS]);
-            CUDA_TRY(cudaEventRecord(h->ev_join, h->side));
-        } else {
-            launch_step_kernel(SK_TRACERS, c, s, h->blk[SK_TRACERS]);
-        }
+        launch_step_kernel(SK_TRACERS, c, s, h->blk[SK_TRACERS]);
         break;
     case 12:   // ghost fills of the donor state, then the fluxes of every cell in one launch
         rc = run_gather(h, h->g_flux_state);
         launch_step_kernel(SK_FLUX, c, s, h->blk[SK_FLUX], 3);
         break;
     case 13:   // strength condition: count the lubricating tracers of every cell in e_cnd
-        if (h->fork_tracers && h->tr.n > 0) CUDA_TRY(cudaStreamWaitEvent(s, h->ev_join, 0));
         if (h->rp.tracer_lubrication > 0) {
             const int fid = field_by_name("e_cnd");
             CUDA_TRY(cudaMemsetAsync(field_ptr(h, fid), 0, (size_t)h->d.PL * field_elem(h, fid), s));
@@ -411,6 +398,25 @@ int run_phase(salec_gpu *h, int ph, bool fused = false)
 {
     return h->mixed ? run_phase_t<float>(h, ph, fused) : run_phase_t<double>(h, ph, fused);
 }
+
+// The whole cycle as the cycle graph holds it: the phases in order, with the energy update inside
+// the stress sweep and the tracers in the flux launch.
+template <class R>
+int run_cycle_t(salec_gpu *h)
+{
+    for (int p = 0; p <= 10; ++p)
+        if (int rc = run_phase(h, p, true)) return rc;
+    // phases 11 and 12: the tracers move in the flux launch
+    if (int rc = run_gather(h, h->g_flux_state)) return rc;
+    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 3, 1);
+    h->launches += 1;
+    CUDA_TRY(cudaGetLastError());
+    for (int p = 13; p <= 15; ++p)
+        if (int rc = run_phase(h, p, true)) return rc;
+    return SALEC_OK;
+}
+
+int run_cycle(salec_gpu *h) { return h->mixed ? run_cycle_t<float>(h) : run_cycle_t<double>(h); }
 
 int build_gathers(salec_gpu *h)
 {
@@ -736,13 +742,10 @@ void release(salec_gpu *h)
     if (h->cycle_graph) cudaGraphExecDestroy(h->cycle_graph);
     for (auto e : h->ev_a) cudaEventDestroy(e);
     for (auto e : h->ev_b) cudaEventDestroy(e);
-    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     for (int k = 0; k < 2; ++k) {
         if (h->report_scal[k]) cudaFreeHost(h->report_scal[k]);
         if (h->report_ev[k]) cudaEventDestroy(h->report_ev[k]);
     }
-    if (h->ev_join) cudaEventDestroy(h->ev_join);
-    if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -891,10 +894,6 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     rp.tracer_lub_frac = run->tracer_lub_frac; rp.max_dt = run->max_dt;
 
     auto bail = [&](int rc) { release(h); return rc; };
-    if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess)
-        return bail(fail(SALEC_ERR_CUDA, "side stream or events"));
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(SALEC_ERR_CUDA, "cudaStreamCreate failed"));
 
@@ -1045,10 +1044,7 @@ void capture_cycle_graph(salec_gpu *h)
         cudaGetLastError();
         return;
     }
-    int rc = SALEC_OK;
-    h->fork_tracers = true;
-    for (int p = 0; p <= 15 && rc == SALEC_OK; ++p) rc = run_phase(h, p, true);
-    h->fork_tracers = false;
+    const int rc = run_cycle(h);
     const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     h->launches = before;
     if (rc != SALEC_OK || e != cudaSuccess || !g) {

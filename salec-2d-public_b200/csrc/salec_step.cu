@@ -15,6 +15,16 @@
 
 namespace salec {
 
+// Programmatic dependent launch: every kernel of this file starts with grid_dependency() and is
+// launched with programmatic stream serialisation (launch_dependent in salec_kernels.h), so the
+// next kernel's blocks are set up and resident while the previous kernel's last blocks drain. The
+// wait returns when the previous grid has completed and its writes are visible; as every thread
+// waits before it touches memory, a completed grid implies that all grids before it have completed.
+__device__ __forceinline__ void grid_dependency()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #define KIDX(i, j) ((long long)(i) + (long long)c.d.P * (long long)(j))
 #define PLN(ptr, comp) ((ptr) + (long long)(comp) * c.d.PL)
 // component comp of a row-tabled geometry field at the thread's own point (i, j)
@@ -159,6 +169,7 @@ __device__ __forceinline__ double cfl_candidate(const C &c, long long p, double 
 template <class R>
 __global__ void k_profile_reset(const CtxT<R> c)
 {
+    grid_dependency();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < c.d.enx) c.f.y_profile[i] = __longlong_as_double((long long)ord_encode(c.rp.threshold_z * 2.0));
 }
@@ -166,6 +177,7 @@ __global__ void k_profile_reset(const CtxT<R> c)
 template <class R>
 __global__ void k_trace_profile(const CtxT<R> c)
 {
+    grid_dependency();
     __shared__ unsigned long long smin[8][32];
     const int i = blockIdx.x * 32 + threadIdx.x;
     const int j0 = blockIdx.y * 64 + threadIdx.y;
@@ -204,6 +216,7 @@ __global__ void k_trace_profile(const CtxT<R> c)
 template <class R>
 __global__ void k_profile_decode(const CtxT<R> c)
 {
+    grid_dependency();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < c.d.enx) {
         unsigned long long u = (unsigned long long)__double_as_longlong(c.f.y_profile[i]);
@@ -279,6 +292,7 @@ __device__ __forceinline__ void vertex_momentum(const C &c, int i, int j)
 template <class R>
 __global__ void SALEC_BOUNDS_VOFMOM k_vertex_vof_momentum(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!vert_active(c, i, j)) return;
     vertex_vof(c, i, j);
@@ -290,6 +304,7 @@ __global__ void SALEC_BOUNDS_VOFMOM k_vertex_vof_momentum(const CtxT<R> c)
 template <class R>
 __global__ void k_cell_velocity(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
@@ -331,6 +346,7 @@ __global__ void k_cell_velocity(const CtxT<R> c)
 template <class R>
 __global__ void k_void_vertices(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!vert_active(c, i, j)) return;
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
@@ -361,6 +377,7 @@ __global__ void k_void_vertices(const CtxT<R> c)
 template <class R>
 __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
 {
+    grid_dependency();
     using A = R;   // arithmetic of the gradient and the viscosity: FP64, or FP32 in the mixed form
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     unsigned long long cand = ~0ULL;
@@ -433,6 +450,7 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
 template <class R>
 __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const CtxT<R> c)
 {
+    grid_dependency();
     if (c.dt_sched) {
         const long long k = c.scal->i_step - c.dt_sched_i0;
         if (k >= 0 && k < c.dt_sched_n) {
@@ -487,6 +505,7 @@ __device__ __forceinline__ void energy_cell(const CtxT<R> &c, long long p, doubl
 template <class R, int NM, bool POR, bool EN = false>
 __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
 {
+    grid_dependency();
     using A = R;   // arithmetic of stress, strength and damage: FP64, or FP32 in the mixed form
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -697,6 +716,7 @@ __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
 template <class R>
 __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
 {
+    grid_dependency();
     using A = R;   // arithmetic of the stress divergence: FP64, or FP32 in the mixed form
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!vert_active(c, i, j)) return;
@@ -804,6 +824,7 @@ __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
 template <class R>
 __global__ void k_vertex_displacement(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
@@ -879,6 +900,7 @@ __device__ __forceinline__ void energy_cell(const CtxT<R> &c, long long p, doubl
 template <class R, int NM, bool POR>
 __global__ void SALEC_BOUNDS_ENERGY k_energy(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
@@ -905,9 +927,8 @@ __device__ __forceinline__ double bilinear4(const double *v, double xi, double e
 }
 
 template <class R>
-__global__ void k_tracers(const CtxT<R> c)
+__device__ __forceinline__ void move_tracer(const CtxT<R> &c, int t)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const Tracers &T = c.tr;
     if (t >= T.n || !T.alive[t]) return;
     const int k = T.cx[t], j = T.cy[t];
@@ -966,6 +987,13 @@ __global__ void k_tracers(const CtxT<R> c)
     if (!(nk >= 2 && nk <= c.d.enx - 3 && nj >= 2 && nj <= c.d.eny - 3)) T.alive[t] = 0;
 }
 
+template <class R>
+__global__ void k_tracers(const CtxT<R> c)
+{
+    grid_dependency();
+    move_tracer(c, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // ============================================================ phase 13: strength condition
 // update_strength_condition (src/strength.c:351-376): e_cnd (cleared before the launch) counts
 // the live tracers of the lubricating rows gy0 <= gy < gy1 in every cell. The counts are small
@@ -973,6 +1001,7 @@ __global__ void k_tracers(const CtxT<R> c)
 template <class R>
 __global__ void k_strength_condition(const CtxT<R> c)
 {
+    grid_dependency();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const Tracers &T = c.tr;
     if (t >= T.n || !T.alive[t]) return;
@@ -1044,18 +1073,26 @@ __device__ __forceinline__ void pad_ring_cell(int t, int enx, int eny, int &i, i
 // pass 3: every cell, after the ghost fills. No cell's flux reads a ghost member the fills write
 // except the pad cells' own, and no flux writes what the fills read, so pass 3 computes what
 // passes 0 and 2 around the fills compute, in one launch whose pad cells hide in the interior's
-// waves.
+// waves. The first `tracer_rows` rows of blocks move the tracers instead (they read nothing the
+// fluxes write and write only tracer arrays), so that their chain of dependent loads runs beside
+// the fluxes: as a launch of their own they cost 41 us of the 2048x2048 impact's cycle.
 template <class R, int NM, bool POR>
-__global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass)
+__global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass, int tracer_rows)
 {
+    grid_dependency();
     int i, j;
+    if ((int)blockIdx.y < tracer_rows) {
+        const int block = blockIdx.y * gridDim.x + blockIdx.x;
+        move_tracer(c, (block * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x);
+        return;
+    }
     if (pass == 2) {
         const int t = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
         if (t >= 4 * c.d.enx + 4 * (c.d.eny - 4)) return;
         pad_ring_cell(t, c.d.enx, c.d.eny, i, j);
     } else {
         i = blockIdx.x * blockDim.x + threadIdx.x;
-        j = blockIdx.y * blockDim.y + threadIdx.y;
+        j = (blockIdx.y - tracer_rows) * blockDim.y + threadIdx.y;
         if (i >= c.d.enx || j >= c.d.eny) return;
         if (pass != 3 && (pass == 0) != cell_interior(c, i, j)) return;
     }
@@ -1706,6 +1743,7 @@ __device__ __forceinline__ void state_cell(const CtxT<R> &c, long long p, const 
 template <class R, int NM, bool POR, bool P3>
 __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_remap, int do_damp, int do_ejecta, int do_state)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= c.d.enx || j >= c.d.eny) return;
     const long long p = KIDX(i, j);
@@ -1735,6 +1773,7 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
 template <class R>
 __global__ void k_cycle(const CtxT<R> c)
 {
+    grid_dependency();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         Scal *s = c.scal;
         s->time += s->dt;
@@ -1750,6 +1789,7 @@ __global__ void k_cycle(const CtxT<R> c)
 template <class R>
 __global__ void k_record_reference_state(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     unsigned long long cand = 0ULL;
     if (i < c.d.enx && j < c.d.eny) {
@@ -1775,6 +1815,7 @@ __global__ void k_record_reference_state(const CtxT<R> c)
 template <class R>
 __global__ void k_init_vertex_velocity(const CtxT<R> c)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
@@ -1807,6 +1848,7 @@ __global__ void k_init_vertex_velocity(const CtxT<R> c)
 template <class R>
 __global__ void k_laplace_mask(const CtxT<R> c, unsigned *mask)
 {
+    grid_dependency();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     bool nz = false;
     if (i < c.d.vnx && j < c.d.vny) {
@@ -1877,11 +1919,10 @@ __device__ __forceinline__ void gather_component(const GatherField &gf, int a, i
     }
 }
 
-__global__ void k_gather(GatherBatch g, int mode, double *scratch)
+// mode 0: in place, one entry (or one component, where the field has them) per thread;
+// 1: gather into scratch; 2: scatter from scratch
+__device__ __forceinline__ void gather_item(const GatherBatch &g, int t, int mode, double *scratch)
 {
-    // mode 0: in place, one entry (or one component, where the field has them) per thread;
-    // 1: gather into scratch; 2: scatter from scratch
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.total) return;
     int f = 0;
     while (f + 1 < g.nfield && t >= g.start[f + 1]) ++f;
@@ -1894,6 +1935,12 @@ __global__ void k_gather(GatherBatch g, int mode, double *scratch)
     }
     if (gf.f32) gather_one<float>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
     else gather_one<double>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
+}
+
+__global__ void k_gather(GatherBatch g, int mode, double *scratch)
+{
+    grid_dependency();
+    gather_item(g, blockIdx.x * blockDim.x + threadIdx.x, mode, scratch);
 }
 
 // ============================================================ layout conversion
@@ -1960,11 +2007,11 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
     do {                                                                                                       \
         const bool por_ = c.rp.porosity_model != 0;                                                            \
         switch (c.d.nmat) {                                                                                    \
-        case 2: if (por_) KERNEL<R, 2, true><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 2, false><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 3: if (por_) KERNEL<R, 3, true><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 3, false><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 4: if (por_) KERNEL<R, 4, true><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 4, false><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 5: if (por_) KERNEL<R, 5, true><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 5, false><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        default: if (por_) KERNEL<R, 0, true><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 0, false><<<g, b, 0, s>>>(__VA_ARGS__); break; \
+        case 2: if (por_) launch_dependent(KERNEL<R, 2, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false>, g, b, s, __VA_ARGS__); break; \
+        case 3: if (por_) launch_dependent(KERNEL<R, 3, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false>, g, b, s, __VA_ARGS__); break; \
+        case 4: if (por_) launch_dependent(KERNEL<R, 4, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false>, g, b, s, __VA_ARGS__); break; \
+        case 5: if (por_) launch_dependent(KERNEL<R, 5, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false>, g, b, s, __VA_ARGS__); break; \
+        default: if (por_) launch_dependent(KERNEL<R, 0, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false>, g, b, s, __VA_ARGS__); break; \
         }                                                                                                      \
     } while (0)
 
@@ -1972,11 +2019,11 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
     do {                                                                                                       \
         const bool por_ = c.rp.porosity_model != 0;                                                            \
         switch (c.d.nmat) {                                                                                    \
-        case 2: if (por_) KERNEL<R, 2, true, X><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 2, false, X><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 3: if (por_) KERNEL<R, 3, true, X><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 3, false, X><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 4: if (por_) KERNEL<R, 4, true, X><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 4, false, X><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        case 5: if (por_) KERNEL<R, 5, true, X><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 5, false, X><<<g, b, 0, s>>>(__VA_ARGS__); break; \
-        default: if (por_) KERNEL<R, 0, true, X><<<g, b, 0, s>>>(__VA_ARGS__); else KERNEL<R, 0, false, X><<<g, b, 0, s>>>(__VA_ARGS__); break; \
+        case 2: if (por_) launch_dependent(KERNEL<R, 2, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false, X>, g, b, s, __VA_ARGS__); break; \
+        case 3: if (por_) launch_dependent(KERNEL<R, 3, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false, X>, g, b, s, __VA_ARGS__); break; \
+        case 4: if (por_) launch_dependent(KERNEL<R, 4, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false, X>, g, b, s, __VA_ARGS__); break; \
+        case 5: if (por_) launch_dependent(KERNEL<R, 5, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false, X>, g, b, s, __VA_ARGS__); break; \
+        default: if (por_) launch_dependent(KERNEL<R, 0, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false, X>, g, b, s, __VA_ARGS__); break; \
         }                                                                                                      \
     } while (0)
 
@@ -1988,29 +2035,33 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, 
     const dim3 gv((c.d.vnx + b.x - 1) / b.x, (c.d.vny + b.y - 1) / b.y);  // vertices
     const int ncol = (c.d.enx + 255) / 256;
     switch (k) {
-    case SK_PROFILE_RESET: k_profile_reset<R><<<ncol, 256, 0, s>>>(c); break;
-    case SK_TRACE_PROFILE: k_trace_profile<R><<<dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, 0, s>>>(c); break;
-    case SK_PROFILE_DECODE: k_profile_decode<R><<<ncol, 256, 0, s>>>(c); break;
-    case SK_VERTEX_VOF_MOMENTUM: k_vertex_vof_momentum<R><<<gv, b, 0, s>>>(c); break;
-    case SK_CELL_VELOCITY: k_cell_velocity<R><<<g, b, 0, s>>>(c); break;
-    case SK_VOID_VERTICES: k_void_vertices<R><<<gv, b, 0, s>>>(c); break;
-    case SK_GRADIENT: k_gradient_viscosity_cfl<R><<<g, b, 0, s>>>(c); break;
-    case SK_FINALIZE_DT: k_finalize_dt<R><<<148, SALEC_FINALIZE_THREADS, 0, s>>>(c); break;
+    case SK_PROFILE_RESET: launch_dependent(k_profile_reset<R>, ncol, 256, s, c); break;
+    case SK_TRACE_PROFILE: launch_dependent(k_trace_profile<R>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
+    case SK_PROFILE_DECODE: launch_dependent(k_profile_decode<R>, ncol, 256, s, c); break;
+    case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, gv, b, s, c); break;
+    case SK_CELL_VELOCITY: launch_dependent(k_cell_velocity<R>, g, b, s, c); break;
+    case SK_VOID_VERTICES: launch_dependent(k_void_vertices<R>, gv, b, s, c); break;
+    case SK_GRADIENT: launch_dependent(k_gradient_viscosity_cfl<R>, g, b, s, c); break;
+    case SK_FINALIZE_DT: launch_dependent(k_finalize_dt<R>, 148, SALEC_FINALIZE_THREADS, s, c); break;
     case SK_STRESS: SALEC_NM_DISPATCH(k_stress, c); break;
     case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, true, c); break;
-    case SK_ACCELERATION: k_vertex_acceleration<R><<<gv, b, 0, s>>>(c); break;
-    case SK_DISPLACEMENT: k_vertex_displacement<R><<<gv, b, 0, s>>>(c); break;
+    case SK_ACCELERATION: launch_dependent(k_vertex_acceleration<R>, gv, b, s, c); break;
+    case SK_DISPLACEMENT: launch_dependent(k_vertex_displacement<R>, gv, b, s, c); break;
     case SK_ENERGY: SALEC_NM_DISPATCH(k_energy, c); break;
     case SK_TRACERS:
-        if (c.tr.n > 0) k_tracers<R><<<(c.tr.n + 127) / 128, 128, 0, s>>>(c);
+        if (c.tr.n > 0) launch_dependent(k_tracers<R>, (c.tr.n + 127) / 128, 128, s, c);
         break;
     case SK_FLUX:
         if (a0 == 2) {   // pad ring, 1-D
             const long long ring = 4LL * c.d.enx + 4LL * (c.d.eny - 4);
             const dim3 g((unsigned)((ring + b.x * b.y - 1) / (b.x * b.y)));
-            SALEC_NM_DISPATCH(k_flux, c, a0);
+            SALEC_NM_DISPATCH(k_flux, c, a0, 0);
         } else {
-            SALEC_NM_DISPATCH(k_flux, c, a0);
+            dim3 gt = g;   // a1: the tracers' blocks come first
+            const int per_row = (int)(g.x * b.x * b.y), rows = a1 && c.tr.n > 0 ? (c.tr.n + per_row - 1) / per_row : 0;
+            gt.y += rows;
+            const dim3 g = gt;
+            SALEC_NM_DISPATCH(k_flux, c, a0, rows);
         }
         break;
     case SK_REMAP_DAMP_STATE:
@@ -2019,14 +2070,14 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, 
         else SALEC_NM_DISPATCH_P3(k_remap_damp_state, false, c, a0, a1, a2, a3);
         break;
     case SK_LAPLACE_MASK:
-        k_laplace_mask<R><<<dim3(c.d.P / 32, (c.d.vny + 7) / 8), b8, 0, s>>>(c, const_cast<unsigned *>(c.lap_mask));
+        launch_dependent(k_laplace_mask<R>, dim3(c.d.P / 32, (c.d.vny + 7) / 8), b8, s, c, const_cast<unsigned *>(c.lap_mask));
         break;
     case SK_STRENGTH_CONDITION:
-        if (c.tr.n > 0) k_strength_condition<R><<<(c.tr.n + 127) / 128, 128, 0, s>>>(c);
+        if (c.tr.n > 0) launch_dependent(k_strength_condition<R>, (c.tr.n + 127) / 128, 128, s, c);
         break;
-    case SK_CYCLE: k_cycle<R><<<1, 32, 0, s>>>(c); break;
-    case SK_RECORD_REFERENCE: k_record_reference_state<R><<<g, b, 0, s>>>(c); break;
-    case SK_INIT_VERTEX_VELOCITY: k_init_vertex_velocity<R><<<gv, b, 0, s>>>(c); break;
+    case SK_CYCLE: launch_dependent(k_cycle<R>, 1, 32, s, c); break;
+    case SK_RECORD_REFERENCE: launch_dependent(k_record_reference_state<R>, g, b, s, c); break;
+    case SK_INIT_VERTEX_VELOCITY: launch_dependent(k_init_vertex_velocity<R>, gv, b, s, c); break;
     }
 }
 
