@@ -118,6 +118,16 @@ struct FieldsT {
 using Fields = FieldsT<double>;
 static_assert(sizeof(FieldsT<float>) == sizeof(FieldsT<double>), "field tables share one layout");
 
+// The donor state: the cell fields that the remap rewrites and that a face's flow carries from the
+// cell it leaves (e_vel, carried too, is not rewritten). The cycle graph keeps two copies: the
+// remap reads the state before it from one, its neighbours' included, and stores into the other,
+// so that no face needs a record of its donor.
+template <class R>
+struct DonorT {
+    double *m_den, *m_eng, *m_pty, *e_cvs;
+    R *e_ste, *e_dam, *e_tps, *e_vib, *e_ejt;
+};
+
 // Lagrangian tracers as structure-of-arrays in the reference's list order
 // (tracer_t of src/mpi_vec/linked_list.h:17-27 plus the cell index and a live flag).
 struct Tracers {
@@ -142,6 +152,7 @@ struct CtxT {
     using real = R;
     Dims d;
     FieldsT<R> f;
+    DonorT<R> o;         // where the remap stores the donor state: f's own planes, or the other copy
     RunParams rp;
     const DevMat *mat;
     Scal *scal;

@@ -59,7 +59,7 @@ enum StepKernel {
     SK_PROFILE_RESET, SK_TRACE_PROFILE, SK_PROFILE_DECODE, SK_VERTEX_VOF_MOMENTUM, SK_CELL_VELOCITY,
     SK_VOID_VERTICES, SK_GRADIENT, SK_FINALIZE_DT, SK_STRESS, SK_ACCELERATION, SK_DISPLACEMENT, SK_ENERGY,
     SK_TRACERS, SK_FLUX, SK_REMAP_DAMP_STATE, SK_CYCLE, SK_RECORD_REFERENCE, SK_INIT_VERTEX_VELOCITY,
-    SK_STRENGTH_CONDITION, SK_LAPLACE_MASK, SK_STRESS_ENERGY, SK_COUNT
+    SK_STRENGTH_CONDITION, SK_LAPLACE_MASK, SK_STRESS_ENERGY, SK_REMAP_DUAL, SK_FACE_RECORDS, SK_COUNT
 };
 
 #ifdef __CUDACC__
@@ -82,7 +82,8 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// flux: a0 = pass (see k_flux), a1 = the tracers move in the same launch; remap: a0..a3 = remap, damping, ejecta drag, EOS switches
+// flux: a0 = pass (see k_flux), a1 = the tracers move in the same launch,
+// a2 = face volumes only; remap: a0..a3 = remap, damping, ejecta drag, EOS switches
 // blk is the block shape of the 2-D sweeps (cells, faces, vertices); the surface profile, the
 // Laplacian mask, the tracer and the single-thread kernels use their own fixed shapes.
 template <class R>

@@ -106,6 +106,7 @@ struct Gather {
     GatherBatch batch{};
     bool two_pass = false;
     int ncomp_max = 0;
+    int fid[SALEC_MAX_GATHER_FIELDS] = {0};       // the fields: their planes can move (salec_gpu::flip)
     int entries[SALEC_MAX_GATHER_FIELDS] = {0};   // map entries per field (the adjoint walks entries)
 };
 
@@ -159,8 +160,16 @@ struct salec_gpu {
     dim3 blk[SK_COUNT];         // block shape of each 2-D sweep (salec_gpu_autotune picks them)
     // one full cycle captured as a CUDA graph (kernel arguments hold the run parameters and the
     // tracer arrays, so changing either drops the graph)
-    cudaGraphExec_t cycle_graph = nullptr;
-    long long cycle_graph_launches = 0;
+    cudaGraphExec_t cycle_graph[2] = {nullptr, nullptr};   // by flip
+    long long cycle_graph_launches[2] = {0, 0};
+    // The cycle graph's remap reads one copy of the donor state (DonorT) and stores into the other;
+    // f then points at the new copy and alt at the state before the remap. flip counts the swaps
+    // modulo two: 0 when f's donor planes are the pool's. settle() brings everything back to the
+    // pool for the phase-by-phase path and the adjoint, which work in place with full face records.
+    Fields alt{};
+    char *alt_pool = nullptr;
+    int flip = 0;
+    bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
     // its completion event and whether it is in flight
     Scal *report_scal[2] = {nullptr, nullptr};
@@ -174,12 +183,16 @@ struct salec_gpu {
     int dt_sched_n = 0;
     struct AdjointState *adj = nullptr;   // adjoint buffers (salec_gpu_adjoint_*)
 
+    // other: the remap's output (c.o) is the other copy of the donor state
     template <class R>
-    CtxT<R> ctx_t() const
+    CtxT<R> ctx_t(bool other = false) const
     {
         CtxT<R> c;
         c.d = d;
         memcpy(&c.f, &f, sizeof(c.f));   // same pointers; relaxed ones address floats in the mixed form
+        FieldsT<R> out;
+        memcpy(&out, other ? &alt : &f, sizeof(out));
+        c.o = {out.m_den, out.m_eng, out.m_pty, out.e_cvs, out.e_ste, out.e_dam, out.e_tps, out.e_vib, out.e_ejt};
         c.rp = rp;
         c.mat = mat;
         c.scal = scal;
@@ -299,6 +312,7 @@ int make_gather(salec_gpu *h, Gather &g, const std::vector<std::pair<int, Gather
         if (comp && (rc = upload_vec(h, cstart[k], &gf.cstart))) return rc;
         g.batch.start[k] = total;
         g.entries[k] = (int)m.dst.size();
+        g.fid[k] = fid;
         total += comp ? (int)cstart[k].size() - 1 : (int)m.dst.size();
     }
     g.batch.start[maps.size()] = total;
@@ -312,11 +326,13 @@ int run_gather(salec_gpu *h, const Gather &g)
     if (g.batch.total == 0) return SALEC_OK;
     const int tb = 256, nb = (g.batch.total + tb - 1) / tb;
     h->launches += g.two_pass ? 2 : 1;
+    GatherBatch b = g.batch;
+    for (int k = 0; k < b.nfield; ++k) b.field[k].base = field_ptr(h, g.fid[k]);
     if (!g.two_pass) {
-        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 0, nullptr);
+        launch_dependent(k_gather, nb, tb, h->stream, b, 0, nullptr);
     } else {
-        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 1, h->scratch);
-        launch_dependent(k_gather, nb, tb, h->stream, g.batch, 2, h->scratch);
+        launch_dependent(k_gather, nb, tb, h->stream, b, 1, h->scratch);
+        launch_dependent(k_gather, nb, tb, h->stream, b, 2, h->scratch);
     }
     CUDA_TRY(cudaGetLastError());
     return SALEC_OK;
@@ -399,8 +415,80 @@ int run_phase(salec_gpu *h, int ph, bool fused = false)
     return h->mixed ? run_phase_t<float>(h, ph, fused) : run_phase_t<double>(h, ph, fused);
 }
 
+// Fields of the donor state (DonorT) that the remap of this handle rewrites.
+std::vector<int> donor_fields(const salec_gpu *h)
+{
+    std::vector<int> v;
+    for (const char *n : {"m_den", "m_eng", "e_ste", "e_dam", "e_tps", "e_vib", "e_ejt"}) v.push_back(field_by_name(n));
+    if (h->rp.porosity_model)
+        for (const char *n : {"m_pty", "e_cvs"}) v.push_back(field_by_name(n));
+    return v;
+}
+
+double *&alt_ptr(salec_gpu *h, int k)
+{
+    return *reinterpret_cast<double **>(reinterpret_cast<char *>(&h->alt) + kFields[k].off);
+}
+
+// The second copy of the donor state. The pml3 remap works in place, and so does a handle whose
+// second copy does not fit on the device.
+void allocate_donor_copy(salec_gpu *h)
+{
+    h->alt = h->f;
+    if (h->rp.damp_type == SALEC_DAMP_PML3) return;
+    size_t bytes = 0;
+    for (int k : donor_fields(h)) bytes += (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k);
+    if (cudaMalloc(&h->alt_pool, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        h->alt_pool = nullptr;
+        return;
+    }
+    size_t off = 0;
+    for (int k : donor_fields(h)) {
+        alt_ptr(h, k) = reinterpret_cast<double *>(h->alt_pool + off);
+        off += (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k);
+    }
+    // points outside the cells (the plane padding) are never stored by the remap
+    cudaMemsetAsync(h->alt_pool, 0, bytes, h->stream);
+}
+
+// The donor members of the face records, where the last cycle stored only their volumes. They come
+// from the state before its remap, so this runs before anything changes that, e_vel or v_dis.
+int complete_records(salec_gpu *h)
+{
+    if (!h->volumes_only) return SALEC_OK;
+    h->volumes_only = false;
+    if (h->mixed) launch_step_kernel(SK_FACE_RECORDS, h->ctx_t<float>(true), h->stream, dim3(32, 4));
+    else launch_step_kernel(SK_FACE_RECORDS, h->ctx_t<double>(true), h->stream, dim3(32, 4));
+    CUDA_TRY(cudaGetLastError());
+    return SALEC_OK;
+}
+
+// Full face records, and the donor state in the pool's own planes.
+int settle(salec_gpu *h)
+{
+    if (int rc = complete_records(h)) return rc;
+    if (!h->flip) return SALEC_OK;
+    for (int k : donor_fields(h)) {
+        CUDA_TRY(cudaMemcpyAsync(alt_ptr(h, k), field_ptr(h, k), (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k),
+                                 cudaMemcpyDeviceToDevice, h->stream));
+        std::swap(field_ptr(h, k), alt_ptr(h, k));
+    }
+    h->flip = 0;
+    return SALEC_OK;
+}
+
+void destroy_cycle_graphs(salec_gpu *h)
+{
+    for (auto &g : h->cycle_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
 // The whole cycle as the cycle graph holds it: the phases in order, with the energy update inside
-// the stress sweep and the tracers in the flux launch.
+// the stress sweep, the tracers in the flux launch and, with a second copy of the donor state, face
+// volumes instead of records and the remap from one copy into the other.
 template <class R>
 int run_cycle_t(salec_gpu *h)
 {
@@ -408,12 +496,18 @@ int run_cycle_t(salec_gpu *h)
         if (int rc = run_phase(h, p, true)) return rc;
     // phases 11 and 12: the tracers move in the flux launch
     if (int rc = run_gather(h, h->g_flux_state)) return rc;
-    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 3, 1);
-    h->launches += 1;
+    const bool dual = h->alt_pool != nullptr;
+    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 3, 1, dual ? 1 : 0);
     CUDA_TRY(cudaGetLastError());
-    for (int p = 13; p <= 15; ++p)
-        if (int rc = run_phase(h, p, true)) return rc;
-    return SALEC_OK;
+    if (int rc = run_phase(h, 13, true)) return rc;
+    if (!dual) {
+        if (int rc = run_phase(h, 14, true)) return rc;
+    } else {
+        const int ejecta = (h->rp.flow_resistance > 0. || h->rp.flow_friction > 0.) ? 1 : 0;
+        launch_step_kernel(SK_REMAP_DUAL, h->ctx_t<R>(true), h->stream, h->blk[SK_REMAP_DAMP_STATE], 1, 1, ejecta, 1);
+        CUDA_TRY(cudaGetLastError());
+    }
+    return run_phase(h, 15, true);
 }
 
 int run_cycle(salec_gpu *h) { return h->mixed ? run_cycle_t<float>(h) : run_cycle_t<double>(h); }
@@ -571,7 +665,7 @@ int build_geo_table(salec_gpu *h, int slot, int fid, int nx, int ny, int nc)
     const long long row_words = (long long)nx * nc;
     if (g.compact) { cudaFree(g.tab); cudaFree(g.row); }
     g = salec_gpu::GeoSlot();
-    if (h->cycle_graph) { cudaGraphExecDestroy(h->cycle_graph); h->cycle_graph = nullptr; }
+    destroy_cycle_graphs(h);
     const auto *src = reinterpret_cast<const unsigned long long *>(h->staging);
 
     // temporaries are stream-ordered (cudaMallocAsync / cudaFreeAsync): freeing them does not
@@ -694,6 +788,8 @@ int transfer(salec_gpu *h, int fid, double *host, long long n, bool to_device)
     void *base = field_ptr(h, fid);
     const bool f32 = field_f32(h, fid);
     const long long plane = kFields[fid].loc == L_COL ? 0 : h->d.PL;
+    if (to_device || kFields[fid].nck == NC_PHI)
+        if (int rc = complete_records(h)) return rc;
     if (to_device) {
         CUDA_TRY(cudaMemcpyAsync(h->staging, host, need * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         launch_aos_to_planes(h->staging, base, f32, plane, h->d.P, nx, ny, nc, h->stream);
@@ -739,7 +835,8 @@ void release(salec_gpu *h)
     for (auto &g : h->geo)
         if (g.compact) { cudaFree(g.tab); cudaFree(g.row); }
     if (h->row_identity) cudaFree(h->row_identity);
-    if (h->cycle_graph) cudaGraphExecDestroy(h->cycle_graph);
+    destroy_cycle_graphs(h);
+    if (h->alt_pool) cudaFree(h->alt_pool);
     for (auto e : h->ev_a) cudaEventDestroy(e);
     for (auto e : h->ev_b) cudaEventDestroy(e);
     for (int k = 0; k < 2; ++k) {
@@ -914,6 +1011,7 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
         off += kFields[k].loc == L_COL ? col * sizeof(double) : (size_t)field_ncomp(h, k) * d.PL * field_elem(h, k);
     }
 
+    allocate_donor_copy(h);
     {
         const size_t words = (size_t)(d.P / 32) * d.R;
         if (cudaMalloc(&h->lap_mask, words * sizeof(unsigned)) != cudaSuccess)
@@ -1001,6 +1099,7 @@ int salec_gpu_phases(salec_gpu *h, int first, int last)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
     if (first < 0 || last > 15 || first > last) return fail(SALEC_ERR_ARG, "phase range must lie in [0, 15]");
+    if (int rc = settle(h)) return rc;
     for (int p = first; p <= last; ++p) {
         if (h->profiling) {
             if (h->ev_used == h->ev_a.size()) {
@@ -1029,8 +1128,7 @@ namespace {
 
 void drop_cycle_graph(salec_gpu *h)
 {
-    if (h->cycle_graph) cudaGraphExecDestroy(h->cycle_graph);
-    h->cycle_graph = nullptr;
+    destroy_cycle_graphs(h);
     adjoint_drop_graphs(h);
 }
 
@@ -1054,7 +1152,7 @@ void capture_cycle_graph(salec_gpu *h)
     }
     cudaGraphExec_t exec = nullptr;
     if (cudaGraphInstantiate(&exec, g, 0) == cudaSuccess) {
-        h->cycle_graph = exec;
+        h->cycle_graph[h->flip] = exec;
         size_t n = 0;
         cudaGraphGetNodes(g, nullptr, &n);
         std::vector<cudaGraphNode_t> nodes(n);
@@ -1064,7 +1162,7 @@ void capture_cycle_graph(salec_gpu *h)
                 cudaGraphNodeType ty;
                 if (cudaGraphNodeGetType(nodes[k], &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel) ++kernels;
             }
-        h->cycle_graph_launches = kernels;
+        h->cycle_graph_launches[h->flip] = kernels;
     }
     cudaGraphDestroy(g);
     cudaGetLastError();
@@ -1076,11 +1174,16 @@ int salec_gpu_step(salec_gpu *h, int nsteps)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
     if (nsteps < 0) return fail(SALEC_ERR_ARG, "negative step count");
-    if (!h->profiling && nsteps > 0 && !h->cycle_graph) capture_cycle_graph(h);
     for (int k = 0; k < nsteps; ++k) {
-        if (!h->profiling && h->cycle_graph) {
-            CUDA_TRY(cudaGraphLaunch(h->cycle_graph, h->stream));
-            h->launches += h->cycle_graph_launches;
+        if (!h->profiling && !h->cycle_graph[h->flip]) capture_cycle_graph(h);
+        if (!h->profiling && h->cycle_graph[h->flip]) {
+            CUDA_TRY(cudaGraphLaunch(h->cycle_graph[h->flip], h->stream));
+            h->launches += h->cycle_graph_launches[h->flip];
+            if (h->alt_pool) {
+                for (int f : donor_fields(h)) std::swap(field_ptr(h, f), alt_ptr(h, f));
+                h->flip ^= 1;
+                h->volumes_only = true;
+            }
         } else {
             int rc = salec_gpu_phases(h, 0, 15);
             if (rc) return rc;
@@ -1238,7 +1341,7 @@ int salec_gpu_set_block_shapes(salec_gpu *h, const int *shapes, int n)
         while (kTunedPhase[t] != shapes[3 * k]) ++t;
         h->blk[kTunedKernel[t]] = dim3(shapes[3 * k + 1], shapes[3 * k + 2]);
     }
-    if (h->cycle_graph) { cudaGraphExecDestroy(h->cycle_graph); h->cycle_graph = nullptr; }
+    destroy_cycle_graphs(h);
     return SALEC_OK;
 }
 
@@ -1251,6 +1354,7 @@ int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
     const int *tuned_phase = kTunedPhase;
     const StepKernel *tuned_kernel = kTunedKernel;
     constexpr int ntuned = kNumTuned;
+    if (int rc = settle(h)) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     // snapshot of everything the cycles change: the field pool, the scalars and the tracers
     void *snap = nullptr, *snap_tr = nullptr;
@@ -1300,7 +1404,7 @@ int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
     const int rc2 = restore();
     cudaFree(snap);
     if (snap_tr) cudaFree(snap_tr);
-    if (h->cycle_graph) { cudaGraphExecDestroy(h->cycle_graph); h->cycle_graph = nullptr; }
+    destroy_cycle_graphs(h);
     if (rc) return rc;
     if (rc2) return rc2;
     if (shapes)
@@ -1896,6 +2000,7 @@ int adjoint_graphs(salec_gpu *h, size_t ub, const std::vector<size_t> &uoff)
 
 int adjoint_check(salec_gpu *h)
 {
+    if (int rc = settle(h)) return rc;
     DevMat m1;
     if (cudaMemcpy(&m1, h->mat + 1, sizeof(DevMat), cudaMemcpyDeviceToHost) != cudaSuccess)
         return fail(SALEC_ERR_CUDA, "material read-back");
@@ -1952,6 +2057,7 @@ int salec_gpu_adjoint_phase(salec_gpu *h, int phase)
 {
     if (!h || !h->adj || !h->adj->pool) return fail(SALEC_ERR_STATE, "call salec_gpu_adjoint_reset first");
     if (phase < 0 || phase > 15) return fail(SALEC_ERR_ARG, "phase out of range");
+    if (int rc = settle(h)) return rc;
     if (int rc = adjoint_phase(h, phase)) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return SALEC_OK;
@@ -2012,6 +2118,7 @@ int salec_gpu_adjoint_window(salec_gpu *h, int nsteps, int every, const double *
         const int n = std::min(every, nsteps - sgm * every);
         if (sgm < nseg - 1) {
             if (int rc = salec_gpu_step(h, n)) return rc;
+            if (int rc = settle(h)) return rc;
         } else {
             launch_slot_set(st->slot, 0, s);
             for (int k = 0; k < n; ++k) CUDA_TRY(cudaGraphLaunch(st->replay, s));

@@ -46,6 +46,13 @@ __device__ __forceinline__ void grid_dependency()
 #ifndef SALEC_REGS_REMAP
 #define SALEC_REGS_REMAP 96
 #endif
+// the remap that reads its donors from the neighbours: 96 for up to three materials and the mixed
+// form, 112 for more in FP64 (2048x2048, three materials: 1243, 1214 and 1254 us a cycle at 80, 96
+// and 112; layered 1024x1024, four porous materials: 558, 507 and 493; layered 600x450 mixed: 210,
+// 192 and 202)
+#ifndef SALEC_REGS_REMAP_DUAL
+#define SALEC_REGS_REMAP_DUAL (NM == 2 || NM == 3 || sizeof(R) == 4 ? 96 : 112)
+#endif
 #ifndef SALEC_REGS_ACCEL
 #define SALEC_REGS_ACCEL 40
 #endif
@@ -104,7 +111,8 @@ __device__ __forceinline__ void grid_dependency()
 #define SALEC_BOUNDS_FLUX __launch_bounds__(256)
 #endif
 #if SALEC_REGS_REMAP > 0
-#define SALEC_BOUNDS_REMAP __maxnreg__((sizeof(R) == 4 ? SALEC_REGS_REMAP_F : SALEC_REGS_REMAP))
+#define SALEC_BOUNDS_REMAP                                                                               \
+    __maxnreg__((DUAL ? SALEC_REGS_REMAP_DUAL : sizeof(R) == 4 ? SALEC_REGS_REMAP_F : SALEC_REGS_REMAP))
 #else
 #define SALEC_BOUNDS_REMAP __launch_bounds__(256)
 #endif
@@ -1017,40 +1025,68 @@ __global__ void k_strength_condition(const CtxT<R> c)
 // A face with zero swept volume gets zero material volumes, which stands in for the
 // reference's clean_flux (src/advect.c:597-626): the other members of such a record are only
 // ever multiplied by those zero volumes.
-// Upwind record of one face of cell p (_calculate_flux_set_bphi, src/advect.c:1138-1223): the
-// face is written by the cell it flows out of; a face with zero swept volume gets zero material
-// volumes (see k_flux).
-template <class R, int NM, bool POR, int MM>
-__device__ __forceinline__ void store_face(const CtxT<R> &c, double *f, double vol, const double (&flux)[MM][4], int k,
-                                           long long p, int nmat)
+// The donor members of a face record, from the state `d` of cell p.
+template <class R, int NM, bool POR, class State>
+__device__ __forceinline__ void store_donor(const CtxT<R> &c, const State &d, double *f, long long p, int nmat)
 {
-    if (vol > 0.) return;
     const long long PL = c.d.PL;
-    if (vol == 0.) {
-#pragma unroll
-        for (int m = 0; m < nmat; ++m) f[m * PL] = 0.0;
-        return;
-    }
 #pragma unroll
     for (int m = 0; m < nmat; ++m) {
-        f[m * PL] = flux[m][k];
-        f[(m + nmat) * PL] = PLN(c.f.m_den, m)[p];
-        f[(m + 2 * nmat) * PL] = PLN(c.f.m_eng, m)[p];
+        f[(m + nmat) * PL] = PLN(d.m_den, m)[p];
+        f[(m + 2 * nmat) * PL] = PLN(d.m_eng, m)[p];
     }
     const int b = 3 * nmat;
     f[(b + 0) * PL] = c.f.e_vel[p];
     f[(b + 1) * PL] = PLN(c.f.e_vel, 1)[p];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) f[(b + 2 + q) * PL] = 1.0 * PLN(c.f.e_ste, q)[p];
-    f[(b + 6) * PL] = 1.0 * c.f.e_dam[p];
-    f[(b + 7) * PL] = 1.0 * c.f.e_tps[p];
-    f[(b + 8) * PL] = 1.0 * c.f.e_vib[p];
-    f[(b + 9) * PL] = 1.0 * c.f.e_ejt[p];
+    for (int q = 0; q < 4; ++q) f[(b + 2 + q) * PL] = 1.0 * PLN(d.e_ste, q)[p];
+    f[(b + 6) * PL] = 1.0 * d.e_dam[p];
+    f[(b + 7) * PL] = 1.0 * d.e_tps[p];
+    f[(b + 8) * PL] = 1.0 * d.e_vib[p];
+    f[(b + 9) * PL] = 1.0 * d.e_ejt[p];
     if (POR) {
-        f[(b + 10) * PL] = 1.0 * c.f.e_cvs[p];
+        f[(b + 10) * PL] = 1.0 * d.e_cvs[p];
 #pragma unroll
-        for (int m = 0; m < nmat; ++m) f[(b + 11 + m) * PL] = PLN(c.f.m_pty, m)[p];
+        for (int m = 0; m < nmat; ++m) f[(b + 11 + m) * PL] = PLN(d.m_pty, m)[p];
     }
+}
+
+// Upwind record of one face of cell p (_calculate_flux_set_bphi, src/advect.c:1138-1223): the
+// face is written by the cell it flows out of; a face with zero swept volume gets zero material
+// volumes (see k_flux).
+// REC = false stores the material volumes only: the cycle graph's remap reads the donor cell itself.
+template <class R, int NM, bool POR, bool REC, int MM>
+__device__ __forceinline__ void store_face(const CtxT<R> &c, double *f, double vol, const double (&flux)[MM][4], int k,
+                                           long long p, int nmat)
+{
+    if (vol > 0.) return;
+    const long long PL = c.d.PL;
+    if (vol == 0. || !REC) {
+#pragma unroll
+        for (int m = 0; m < nmat; ++m) f[m * PL] = vol == 0. ? 0.0 : flux[m][k];
+        return;
+    }
+#pragma unroll
+    for (int m = 0; m < nmat; ++m) f[m * PL] = flux[m][k];
+    store_donor<R, NM, POR>(c, c.f, f, p, nmat);
+}
+
+// Corner positions and displacements of cell (i, j) and the swept volumes of its faces (negative:
+// the flow leaves the cell).
+template <class C>
+__device__ __forceinline__ void cell_swept_volumes(const C &c, int i, int j, double (&px)[4], double (&py)[4], double (&dx)[4],
+                                                   double (&dy)[4], double &lv, double &bv, double &rv, double &uv)
+{
+    const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        px[k] = c.f.v_pos[vl[k]]; py[k] = PLN(c.f.v_pos, 1)[vl[k]];
+        dx[k] = c.f.v_dis[vl[k]]; dy[k] = PLN(c.f.v_dis, 1)[vl[k]];
+    }
+    lv = swept_volume(px[0], py[0], px[3], py[3], dx[0], dy[0], dx[3], dy[3]);
+    rv = swept_volume(px[2], py[2], px[1], py[1], dx[2], dy[2], dx[1], dy[1]);
+    bv = swept_volume(px[1], py[1], px[0], py[0], dx[1], dy[1], dx[0], dy[0]);
+    uv = swept_volume(px[3], py[3], px[2], py[2], dx[3], dy[3], dx[2], dy[2]);
 }
 
 // Cell t of the two-cell pad ring, t < 4 enx + 4 (eny - 4): the two bottom rows, the two top
@@ -1076,7 +1112,7 @@ __device__ __forceinline__ void pad_ring_cell(int t, int enx, int eny, int &i, i
 // waves. The first `tracer_rows` rows of blocks move the tracers instead (they read nothing the
 // fluxes write and write only tracer arrays), so that their chain of dependent loads runs beside
 // the fluxes: as a launch of their own they cost 41 us of the 2048x2048 impact's cycle.
-template <class R, int NM, bool POR>
+template <class R, int NM, bool POR, bool REC = true>
 __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass, int tracer_rows)
 {
     grid_dependency();
@@ -1100,16 +1136,8 @@ __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass, int tracer_r
     const int nmat = NM > 0 ? NM : c.d.nmat;
     const long long p = KIDX(i, j);
     const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
-    double px[4], py[4], dx[4], dy[4];
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        px[k] = c.f.v_pos[vl[k]]; py[k] = PLN(c.f.v_pos, 1)[vl[k]];
-        dx[k] = c.f.v_dis[vl[k]]; dy[k] = PLN(c.f.v_dis, 1)[vl[k]];
-    }
-    const double lv = swept_volume(px[0], py[0], px[3], py[3], dx[0], dy[0], dx[3], dy[3]);
-    const double rv = swept_volume(px[2], py[2], px[1], py[1], dx[2], dy[2], dx[1], dy[1]);
-    const double bv = swept_volume(px[1], py[1], px[0], py[0], dx[1], dy[1], dx[0], dy[0]);
-    const double uv = swept_volume(px[3], py[3], px[2], py[2], dx[3], dy[3], dx[2], dy[2]);
+    double px[4], py[4], dx[4], dy[4], lv, bv, rv, uv;
+    cell_swept_volumes(c, i, j, px, py, dx, dy, lv, bv, rv, uv);
     double vof[MM];
     #pragma unroll
     for (int m = 0; m < nmat; ++m) vof[m] = PLN(c.f.m_vof, m)[p];
@@ -1256,10 +1284,29 @@ __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass, int tracer_r
     }
 
     // faces l, b, r, u
-    store_face<R, NM, POR>(c, c.f.bx_phi + KIDX(i, j), lv, flux, 0, p, nmat);
-    store_face<R, NM, POR>(c, c.f.by_phi + KIDX(i, j), bv, flux, 1, p, nmat);
-    store_face<R, NM, POR>(c, c.f.bx_phi + KIDX(i + 1, j), rv, flux, 2, p, nmat);
-    store_face<R, NM, POR>(c, c.f.by_phi + KIDX(i, j + 1), uv, flux, 3, p, nmat);
+    store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i, j), lv, flux, 0, p, nmat);
+    store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j), bv, flux, 1, p, nmat);
+    store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i + 1, j), rv, flux, 2, p, nmat);
+    store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j + 1), uv, flux, 3, p, nmat);
+}
+
+// Donor members of the face records of a cycle whose fluxes stored volumes only, for readers of
+// bx_phi and by_phi: the donor state before the remap is the copy the remap did not write (c.o),
+// and v_dis and e_vel are still that cycle's.
+template <class R, int NM, bool POR>
+__global__ void k_face_records(const CtxT<R> c)
+{
+    grid_dependency();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= c.d.enx || j >= c.d.eny) return;
+    const int nmat = NM > 0 ? NM : c.d.nmat;
+    const long long p = KIDX(i, j);
+    double px[4], py[4], dx[4], dy[4], lv, bv, rv, uv;
+    cell_swept_volumes(c, i, j, px, py, dx, dy, lv, bv, rv, uv);
+    if (lv < 0.) store_donor<R, NM, POR>(c, c.o, c.f.bx_phi + p, p, nmat);
+    if (bv < 0.) store_donor<R, NM, POR>(c, c.o, c.f.by_phi + p, p, nmat);
+    if (rv < 0.) store_donor<R, NM, POR>(c, c.o, c.f.bx_phi + KIDX(i + 1, j), p, nmat);
+    if (uv < 0.) store_donor<R, NM, POR>(c, c.o, c.f.by_phi + KIDX(i, j + 1), p, nmat);
 }
 
 // ============================================================ phase 14: remap + damping + EOS
@@ -1305,26 +1352,30 @@ __device__ __forceinline__ void store_cell(const CtxT<R> &c, long long p, const 
     #pragma unroll
     for (int m = 0; m < nmat; ++m) {
         PLN(c.f.m_vof, m)[p] = s.vof[m];
-        PLN(c.f.m_den, m)[p] = s.rho[m];
-        PLN(c.f.m_eng, m)[p] = s.eng[m];
-        if (POR) PLN(c.f.m_pty, m)[p] = s.pty[m];
+        PLN(c.o.m_den, m)[p] = s.rho[m];
+        PLN(c.o.m_eng, m)[p] = s.eng[m];
+        if (POR) PLN(c.o.m_pty, m)[p] = s.pty[m];
     }
     c.f.e_dvel[p] = s.dvx;
     PLN(c.f.e_dvel, 1)[p] = s.dvy;
     #pragma unroll
-    for (int q = 0; q < 4; ++q) PLN(c.f.e_ste, q)[p] = s.st[q];
-    c.f.e_dam[p] = s.dam;
-    c.f.e_tps[p] = s.tps;
-    c.f.e_vib[p] = s.vib;
-    c.f.e_ejt[p] = s.ejt;
-    if (POR) c.f.e_cvs[p] = s.cvs;
+    for (int q = 0; q < 4; ++q) PLN(c.o.e_ste, q)[p] = s.st[q];
+    c.o.e_dam[p] = s.dam;
+    c.o.e_tps[p] = s.tps;
+    c.o.e_vib[p] = s.vib;
+    c.o.e_ejt[p] = s.ejt;
+    if (POR) c.o.e_cvs[p] = s.cvs;
     if (den) c.f.e_den[p] = s.eden;
 }
 
 // advect_flux_default (src/advect.c:26-302) for one interior cell, into registers. The loads
 // that do not depend on the flow (the cell's own state and the material volumes of its four
-// faces) are all issued before the first dependent one.
-template <class R, int NM, bool POR, bool P3>
+// faces) are all issued before the first dependent one, the own state only where that leaves
+// registers for it.
+// DUAL: the donor members of a face's flow are read from the cell it leaves instead of the face
+// record; the net volume of the face says which cell that is (all of its material volumes have its
+// sign, but for roundings of a vanishing one).
+template <class R, int NM, bool POR, bool P3, bool DUAL>
 __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long long p, CellState<NM, POR> &s)
 {
     constexpr int MM = CellState<NM, POR>::MM;
@@ -1340,21 +1391,25 @@ __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long 
     for (int k = 0; k < 4; ++k)
         #pragma unroll
         for (int m = 0; m < nmat; ++m) fv[k][m] = face[k][m * PL];
-    double vof[MM], rho[MM], eng[MM], pty[MM];
-    #pragma unroll
-    for (int m = 0; m < nmat; ++m) {
-        vof[m] = PLN(c.f.m_vof, m)[p];
-        rho[m] = PLN(c.f.m_den, m)[p];
-        eng[m] = PLN(c.f.m_eng, m)[p];
-        pty[m] = por ? PLN(c.f.m_pty, m)[p] : 1.0;
-    }
-    const double evol = c.f.e_vol[p];
-    const double eden0 = c.f.e_den[p];
-    double st0[4];
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) st0[q] = PLN(c.f.e_ste, q)[p];
-    const double dam0 = c.f.e_dam[p], tps0 = c.f.e_tps[p], vib0 = c.f.e_vib[p], ejt0 = c.f.e_ejt[p];
-    const double cvs0 = por ? c.f.e_cvs[p] : 0.0;
+    double vof[MM], rho[MM], eng[MM], pty[MM], evol, eden0, st0[4], dam0, tps0, vib0, ejt0, cvs0;
+    auto load_own = [&]() {
+        #pragma unroll
+        for (int m = 0; m < nmat; ++m) {
+            vof[m] = PLN(c.f.m_vof, m)[p];
+            rho[m] = PLN(c.f.m_den, m)[p];
+            eng[m] = PLN(c.f.m_eng, m)[p];
+            pty[m] = por ? PLN(c.f.m_pty, m)[p] : 1.0;
+        }
+        evol = c.f.e_vol[p];
+        eden0 = c.f.e_den[p];
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) st0[q] = PLN(c.f.e_ste, q)[p];
+        dam0 = c.f.e_dam[p]; tps0 = c.f.e_tps[p]; vib0 = c.f.e_vib[p]; ejt0 = c.f.e_ejt[p];
+        cvs0 = por ? c.f.e_cvs[p] : 0.0;
+    };
+    // from face records the own state is loaded ahead of the faces; with the donors of DUAL beside
+    // it, that spills (2048x2048: 1265 us a cycle against 1214 with the own state after the faces)
+    if (!DUAL) load_own();
 
     // advect_flux_pml3 (src/advect.c:304-594) differs from the default remap in the PML
     // auxiliaries e_beta (fluxes of mass, energy and momentum weighted by the layer's sigma,
@@ -1377,32 +1432,78 @@ __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long 
     #pragma unroll
     for (int q = 0; q < phi; ++q) dphi[q] = 0.;
     const int b = 3 * nmat;
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const double *f = face[k];
+    if constexpr (DUAL) {
+        const long long nb[4] = {p - 1, p - c.d.P, p + 1, p + c.d.P};
         #pragma unroll
-        for (int m = 0; m < nmat; ++m) {
-            const double mv = dir[k] * fv[k][m];
-            if (mv == 0.0) continue;   // adds only signed zeros to dphi and e_beta (see k_flux)
-            const double rho_f = f[(m + nmat) * PL];
-            dphi[m] += mv;
-            dphi[m + nmat] += mv * rho_f;
-            dphi[m + 2 * nmat] += mv * f[(m + 2 * nmat) * PL];
-            const double fm = mv * rho_f;
+        for (int k = 0; k < 4; ++k) {
+            double in = 0.;
+            bool flow = false;
             #pragma unroll
-            for (int q = 0; q < 10; ++q) dphi[b + q] += fm * f[(b + q) * PL];
-            if (por && !p3) {
-                dphi[b + 10] += (f[(b + 10) * PL]) * (mv * rho_f);
-                dphi[m + b + 11] += (f[(m + b + 11) * PL]) * (mv * rho_f);
+            for (int m = 0; m < nmat; ++m) { in += dir[k] * fv[k][m]; flow = flow || fv[k][m] != 0.0; }
+            if (!flow) continue;
+            const long long q = in > 0. ? nb[k] : p;
+            // the donor's members in one batch, then every material's share
+            double rf[MM], ef[MM], pf[MM], g[11];
+            #pragma unroll
+            for (int m = 0; m < nmat; ++m) {
+                rf[m] = PLN(c.f.m_den, m)[q];
+                ef[m] = PLN(c.f.m_eng, m)[q];
+                pf[m] = por ? PLN(c.f.m_pty, m)[q] : 0.0;
             }
-            if (p3_layer) {
-                eb0 += mv * rho_f * para[k];
-                eb1 += mv * f[(m + 2 * nmat) * PL] * para[k];
-                eb2 += mv * rho_f * para[k] * f[b * PL];
-                eb3 += mv * rho_f * para[k] * f[(b + 1) * PL];
+            g[0] = c.f.e_vel[q];
+            g[1] = PLN(c.f.e_vel, 1)[q];
+            #pragma unroll
+            for (int r = 0; r < 4; ++r) g[2 + r] = PLN(c.f.e_ste, r)[q];
+            g[6] = c.f.e_dam[q];
+            g[7] = c.f.e_tps[q];
+            g[8] = c.f.e_vib[q];
+            g[9] = c.f.e_ejt[q];
+            g[10] = por ? c.f.e_cvs[q] : 0.0;
+            #pragma unroll
+            for (int m = 0; m < nmat; ++m) {
+                const double mv = dir[k] * fv[k][m];
+                if (mv == 0.0) continue;   // adds only signed zeros to dphi (see k_flux)
+                dphi[m] += mv;
+                const double fm = mv * rf[m];
+                dphi[m + nmat] += fm;
+                dphi[m + 2 * nmat] += mv * ef[m];
+                #pragma unroll
+                for (int r = 0; r < 10; ++r) dphi[b + r] += fm * g[r];
+                if (por) {
+                    dphi[b + 10] += g[10] * fm;
+                    dphi[m + b + 11] += pf[m] * fm;
+                }
+            }
+        }
+    } else {
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double *f = face[k];
+            #pragma unroll
+            for (int m = 0; m < nmat; ++m) {
+                const double mv = dir[k] * fv[k][m];
+                if (mv == 0.0) continue;   // adds only signed zeros to dphi and e_beta (see k_flux)
+                const double rho_f = f[(m + nmat) * PL];
+                dphi[m] += mv;
+                dphi[m + nmat] += mv * rho_f;
+                dphi[m + 2 * nmat] += mv * f[(m + 2 * nmat) * PL];
+                const double fm = mv * rho_f;
+                #pragma unroll
+                for (int q = 0; q < 10; ++q) dphi[b + q] += fm * f[(b + q) * PL];
+                if (por && !p3) {
+                    dphi[b + 10] += (f[(b + 10) * PL]) * (mv * rho_f);
+                    dphi[m + b + 11] += (f[(m + b + 11) * PL]) * (mv * rho_f);
+                }
+                if (p3_layer) {
+                    eb0 += mv * rho_f * para[k];
+                    eb1 += mv * f[(m + 2 * nmat) * PL] * para[k];
+                    eb2 += mv * rho_f * para[k] * f[b * PL];
+                    eb3 += mv * rho_f * para[k] * f[(b + 1) * PL];
+                }
             }
         }
     }
+    if (DUAL) load_own();
     // sphi = cell content + face fluxes, accumulated in place in dphi (the content of each
     // member is formed as 0 + term, then the flux sum is added, as in the reference)
     double emass = evol * eden0;
@@ -1740,7 +1841,9 @@ __device__ __forceinline__ void state_cell(const CtxT<R> &c, long long p, const 
 
 // One thread per cell: remap (interior), damping (every cell, while t < damp_time), ejecta
 // drag and EOS (interior). The cell's state is stored once, after damping and drag.
-template <class R, int NM, bool POR, bool P3>
+// DUAL (the cycle graph): donors are read from the neighbouring cells and every cell, pads
+// included, is stored into the other copy of the donor state.
+template <class R, int NM, bool POR, bool P3, bool DUAL = false>
 __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_remap, int do_damp, int do_ejecta, int do_state)
 {
     grid_dependency();
@@ -1753,11 +1856,11 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
     const bool damp = do_damp && c.rp.damp_time > c.scal->time && c.rp.damp_type != 4 && c.rp.damp_type != 5;
     const bool ejecta = do_ejecta && interior;
     const bool state = do_state && interior;
-    if (!(remap || damp || ejecta || state)) return;
+    if (!DUAL && !(remap || damp || ejecta || state)) return;
     CellState<NM, POR> s;
-    if (remap) remap_cell<R, NM, POR, P3>(c, i, j, p, s);
+    if (remap) remap_cell<R, NM, POR, P3, DUAL>(c, i, j, p, s);
     else load_cell<R, NM, POR>(c, p, s);
-    bool dirty = remap;
+    bool dirty = remap || DUAL;
     if (damp) dirty |= damp_cell<R, NM, POR>(c, p, dt, s);
     if (ejecta) {
         ejecta_drag_cell<R, NM, POR>(c, i, j, p, dt, s);
@@ -2015,15 +2118,16 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
         }                                                                                                      \
     } while (0)
 
+#define SALEC_LIST(...) __VA_ARGS__
 #define SALEC_NM_DISPATCH_P3(KERNEL, X, ...)                                                                   \
     do {                                                                                                       \
         const bool por_ = c.rp.porosity_model != 0;                                                            \
         switch (c.d.nmat) {                                                                                    \
-        case 2: if (por_) launch_dependent(KERNEL<R, 2, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false, X>, g, b, s, __VA_ARGS__); break; \
-        case 3: if (por_) launch_dependent(KERNEL<R, 3, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false, X>, g, b, s, __VA_ARGS__); break; \
-        case 4: if (por_) launch_dependent(KERNEL<R, 4, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false, X>, g, b, s, __VA_ARGS__); break; \
-        case 5: if (por_) launch_dependent(KERNEL<R, 5, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false, X>, g, b, s, __VA_ARGS__); break; \
-        default: if (por_) launch_dependent(KERNEL<R, 0, true, X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false, X>, g, b, s, __VA_ARGS__); break; \
+        case 2: if (por_) launch_dependent(KERNEL<R, 2, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
+        case 3: if (por_) launch_dependent(KERNEL<R, 3, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
+        case 4: if (por_) launch_dependent(KERNEL<R, 4, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
+        case 5: if (por_) launch_dependent(KERNEL<R, 5, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
+        default: if (por_) launch_dependent(KERNEL<R, 0, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
         }                                                                                                      \
     } while (0)
 
@@ -2044,7 +2148,7 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, 
     case SK_GRADIENT: launch_dependent(k_gradient_viscosity_cfl<R>, g, b, s, c); break;
     case SK_FINALIZE_DT: launch_dependent(k_finalize_dt<R>, 148, SALEC_FINALIZE_THREADS, s, c); break;
     case SK_STRESS: SALEC_NM_DISPATCH(k_stress, c); break;
-    case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, true, c); break;
+    case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, (true), c); break;
     case SK_ACCELERATION: launch_dependent(k_vertex_acceleration<R>, gv, b, s, c); break;
     case SK_DISPLACEMENT: launch_dependent(k_vertex_displacement<R>, gv, b, s, c); break;
     case SK_ENERGY: SALEC_NM_DISPATCH(k_energy, c); break;
@@ -2061,14 +2165,19 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, 
             const int per_row = (int)(g.x * b.x * b.y), rows = a1 && c.tr.n > 0 ? (c.tr.n + per_row - 1) / per_row : 0;
             gt.y += rows;
             const dim3 g = gt;
-            SALEC_NM_DISPATCH(k_flux, c, a0, rows);
+            if (a2) SALEC_NM_DISPATCH_P3(k_flux, (false), c, a0, rows);   // a2: volumes only
+            else SALEC_NM_DISPATCH(k_flux, c, a0, rows);
         }
         break;
     case SK_REMAP_DAMP_STATE:
         // the pml3 remap is its own instance so that its extra state costs the others no registers
-        if (c.rp.damp_type == 2) SALEC_NM_DISPATCH_P3(k_remap_damp_state, true, c, a0, a1, a2, a3);
-        else SALEC_NM_DISPATCH_P3(k_remap_damp_state, false, c, a0, a1, a2, a3);
+        if (c.rp.damp_type == 2) SALEC_NM_DISPATCH_P3(k_remap_damp_state, (true), c, a0, a1, a2, a3);
+        else SALEC_NM_DISPATCH_P3(k_remap_damp_state, (false), c, a0, a1, a2, a3);
         break;
+    case SK_REMAP_DUAL:
+        SALEC_NM_DISPATCH_P3(k_remap_damp_state, (false, true), c, a0, a1, a2, a3);
+        break;
+    case SK_FACE_RECORDS: SALEC_NM_DISPATCH(k_face_records, c); break;
     case SK_LAPLACE_MASK:
         launch_dependent(k_laplace_mask<R>, dim3(c.d.P / 32, (c.d.vny + 7) / 8), b8, s, c, const_cast<unsigned *>(c.lap_mask));
         break;
