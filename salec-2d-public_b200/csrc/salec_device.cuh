@@ -24,6 +24,7 @@
 #define SALEC_TOLQPRE 1e-4
 #define SALEC_DTF 0.2
 #define SALEC_CISSAMK1 1.0
+#define SALEC_TILE_ROWS 8
 
 namespace salec {
 
@@ -166,6 +167,17 @@ struct CtxT {
     const double *dt_sched;
     long long dt_sched_i0;
     int dt_sched_n;
+    // The sweeps run over tiles of 32 x SALEC_TILE_ROWS points, tx by ty of them. In the cycle graph of
+    // a handle with a quiet map the tiles to visit are listed (packed x | y << 16), *tile_count of them;
+    // else tile_list is null and all are visited.
+    int tx, ty;
+    const int *tile_list, *tile_count;
+    // Quiet map (null outside the graph): vacuum[] says of every row segment of a tile whether the
+    // last remap left pure vacuum in all of its cells, all of them interior; quiet[] counts, up to
+    // 255, the cycles that began with the tile and its surroundings all vacuum; next_list and
+    // next_count are the list under construction for the next cycle. See count_quiet().
+    unsigned char *vacuum, *quiet;
+    int *next_list, *next_count;
 };
 using Ctx = CtxT<double>;
 

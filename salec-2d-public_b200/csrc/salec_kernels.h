@@ -82,13 +82,15 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// flux: a0 = pass (see k_flux), a1 = the tracers move in the same launch,
-// a2 = face volumes only; remap: a0..a3 = remap, damping, ejecta drag, EOS switches
-// blk is the block shape of the 2-D sweeps (cells, faces, vertices); the surface profile, the
-// Laplacian mask, the tracer and the single-thread kernels use their own fixed shapes.
+// flux: a0 = the tracers move in the same launch, a1 = face volumes only; remap: a0..a3 = remap,
+// damping, ejecta drag, EOS switches. blk is the block shape of the 2-D sweeps (cells, faces,
+// vertices), of which the thread count matters; the surface profile, the Laplacian mask, the tracer and
+// the single-thread kernels use their own fixed shapes.
 template <class R>
 void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 blk, int a0 = 0, int a1 = 0,
                         int a2 = 0, int a3 = 0);
+void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
+                         cudaStream_t s);
 __global__ void k_gather(GatherBatch g, int mode, double *scratch);
 void launch_aos_to_planes(const double *aos, void *base, bool f32, long long plane, int P, int nx, int ny, int nc,
                           cudaStream_t s);

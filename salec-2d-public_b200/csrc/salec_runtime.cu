@@ -169,6 +169,11 @@ struct salec_gpu {
     Fields alt{};
     char *alt_pool = nullptr;
     int flip = 0;
+    // quiet map (CtxT): vacuum[], quiet[], and per flip a tile list with its count. Null where the
+    // map is not used.
+    unsigned char *quiet_map = nullptr;
+    bool quiet_known = true;     // the map may hold quiet tiles: a graph cycle has run since it was forgotten
+    bool in_graph = false;       // the cycle graph is being captured: its kernels take the quiet map
     bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
     // its completion event and whether it is in flight
@@ -182,6 +187,19 @@ struct salec_gpu {
     long long dt_sched_i0 = 0;
     int dt_sched_n = 0;
     struct AdjointState *adj = nullptr;   // adjoint buffers (salec_gpu_adjoint_*)
+
+    int tiles_x() const { return d.P / 32; }
+    int tiles_y() const { return (d.R + SALEC_TILE_ROWS - 1) / SALEC_TILE_ROWS; }
+    int tiles() const { return tiles_x() * tiles_y(); }
+    // layout of quiet_map: vacuum[], quiet[], two lists, two counts, each 128-byte aligned
+    static size_t rounded(size_t n) { return (n + 127) / 128 * 128; }
+    size_t segment_bytes() const { return rounded((size_t)tiles() * SALEC_TILE_ROWS); }
+    int *tile_list(int k) const
+    {
+        return reinterpret_cast<int *>(quiet_map + segment_bytes() + rounded(tiles()) + k * rounded(sizeof(int) * tiles()));
+    }
+    int *tile_count(int k) const { return tile_list(2) + 32 * k; }
+    size_t quiet_bytes() const { return segment_bytes() + rounded(tiles()) + 2 * rounded(sizeof(int) * tiles()) + 256; }
 
     // other: the remap's output (c.o) is the other copy of the donor state
     template <class R>
@@ -206,6 +224,19 @@ struct salec_gpu {
         c.dt_sched = dt_sched;
         c.dt_sched_i0 = dt_sched_i0;
         c.dt_sched_n = dt_sched_n;
+        c.tx = tiles_x();
+        c.ty = tiles_y();
+        c.tile_list = c.tile_count = nullptr;
+        c.next_list = c.next_count = nullptr;
+        c.vacuum = c.quiet = nullptr;
+        if (in_graph && quiet_map) {
+            c.vacuum = quiet_map;
+            c.quiet = quiet_map + segment_bytes();
+            c.tile_list = tile_list(flip);
+            c.tile_count = tile_count(flip);
+            c.next_list = tile_list(flip ^ 1);
+            c.next_count = tile_count(flip ^ 1);
+        }
         return c;
     }
     Ctx ctx() const { return ctx_t<double>(); }
@@ -387,7 +418,7 @@ int run_phase_t(salec_gpu *h, int ph, bool fused)
         break;
     case 12:   // ghost fills of the donor state, then the fluxes of every cell in one launch
         rc = run_gather(h, h->g_flux_state);
-        launch_step_kernel(SK_FLUX, c, s, h->blk[SK_FLUX], 3);
+        launch_step_kernel(SK_FLUX, c, s, h->blk[SK_FLUX]);
         break;
     case 13:   // strength condition: count the lubricating tracers of every cell in e_cnd
         if (h->rp.tracer_lubrication > 0) {
@@ -430,6 +461,21 @@ double *&alt_ptr(salec_gpu *h, int k)
     return *reinterpret_cast<double **>(reinterpret_cast<char *>(&h->alt) + kFields[k].off);
 }
 
+// Something other than a graph cycle changes the fields: nothing is known to be quiet.
+int forget_quiet(salec_gpu *h)
+{
+    if (!h->quiet_map || !h->quiet_known) return SALEC_OK;
+    h->quiet_known = false;
+    launch_forget_quiet(h->quiet_map, h->tiles() * SALEC_TILE_ROWS, h->quiet_map + h->segment_bytes(), h->tiles_x(),
+                        h->tiles_y(), h->tile_list(h->flip), h->tile_count(h->flip), h->stream);
+    CUDA_TRY(cudaGetLastError());
+    return SALEC_OK;
+}
+
+#ifndef SALEC_QUIET_MIN_CELLS
+#define SALEC_QUIET_MIN_CELLS 200000
+#endif
+
 // The second copy of the donor state. The pml3 remap works in place, and so does a handle whose
 // second copy does not fit on the device.
 void allocate_donor_copy(salec_gpu *h)
@@ -450,6 +496,16 @@ void allocate_donor_copy(salec_gpu *h)
     }
     // points outside the cells (the plane padding) are never stored by the remap
     cudaMemsetAsync(h->alt_pool, 0, bytes, h->stream);
+    // The quiet map needs a cycle whose vacuum is the same whatever the time step (count_quiet). Small
+    // meshes fill the device for a moment only, whatever they visit, and looking the tile up costs
+    // them more than it saves (64x80: 81 us a cycle without, 86 with; 517x771: 194 and 184).
+    if (h->rp.damp_type == SALEC_DAMP_PML2 || (long long)h->d.enx * h->d.eny < SALEC_QUIET_MIN_CELLS) return;
+    if (cudaMalloc(reinterpret_cast<void **>(&h->quiet_map), h->quiet_bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        h->quiet_map = nullptr;
+        return;
+    }
+    forget_quiet(h);
 }
 
 // The donor members of the face records, where the last cycle stored only their volumes. They come
@@ -464,18 +520,20 @@ int complete_records(salec_gpu *h)
     return SALEC_OK;
 }
 
-// Full face records, and the donor state in the pool's own planes.
+// Full face records, the donor state in the pool's own planes and no segment taken for quiet.
 int settle(salec_gpu *h)
 {
     if (int rc = complete_records(h)) return rc;
-    if (!h->flip) return SALEC_OK;
-    for (int k : donor_fields(h)) {
-        CUDA_TRY(cudaMemcpyAsync(alt_ptr(h, k), field_ptr(h, k), (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k),
-                                 cudaMemcpyDeviceToDevice, h->stream));
-        std::swap(field_ptr(h, k), alt_ptr(h, k));
+    if (h->flip) {
+        for (int k : donor_fields(h)) {
+            CUDA_TRY(cudaMemcpyAsync(alt_ptr(h, k), field_ptr(h, k),
+                                     (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k), cudaMemcpyDeviceToDevice,
+                                     h->stream));
+            std::swap(field_ptr(h, k), alt_ptr(h, k));
+        }
+        h->flip = 0;
     }
-    h->flip = 0;
-    return SALEC_OK;
+    return forget_quiet(h);
 }
 
 void destroy_cycle_graphs(salec_gpu *h)
@@ -497,7 +555,7 @@ int run_cycle_t(salec_gpu *h)
     // phases 11 and 12: the tracers move in the flux launch
     if (int rc = run_gather(h, h->g_flux_state)) return rc;
     const bool dual = h->alt_pool != nullptr;
-    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 3, 1, dual ? 1 : 0);
+    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 1, dual ? 1 : 0);
     CUDA_TRY(cudaGetLastError());
     if (int rc = run_phase(h, 13, true)) return rc;
     if (!dual) {
@@ -791,6 +849,7 @@ int transfer(salec_gpu *h, int fid, double *host, long long n, bool to_device)
     if (to_device || kFields[fid].nck == NC_PHI)
         if (int rc = complete_records(h)) return rc;
     if (to_device) {
+        if (int rc = forget_quiet(h)) return rc;
         CUDA_TRY(cudaMemcpyAsync(h->staging, host, need * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         launch_aos_to_planes(h->staging, base, f32, plane, h->d.P, nx, ny, nc, h->stream);
         CUDA_TRY(cudaGetLastError());
@@ -837,6 +896,7 @@ void release(salec_gpu *h)
     if (h->row_identity) cudaFree(h->row_identity);
     destroy_cycle_graphs(h);
     if (h->alt_pool) cudaFree(h->alt_pool);
+    if (h->quiet_map) cudaFree(h->quiet_map);
     for (auto e : h->ev_a) cudaEventDestroy(e);
     for (auto e : h->ev_b) cudaEventDestroy(e);
     for (int k = 0; k < 2; ++k) {
@@ -1142,7 +1202,9 @@ void capture_cycle_graph(salec_gpu *h)
         cudaGetLastError();
         return;
     }
+    h->in_graph = true;
     const int rc = run_cycle(h);
+    h->in_graph = false;
     const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     h->launches = before;
     if (rc != SALEC_OK || e != cudaSuccess || !g) {
@@ -1183,6 +1245,7 @@ int salec_gpu_step(salec_gpu *h, int nsteps)
                 for (int f : donor_fields(h)) std::swap(field_ptr(h, f), alt_ptr(h, f));
                 h->flip ^= 1;
                 h->volumes_only = true;
+                h->quiet_known = true;
             }
         } else {
             int rc = salec_gpu_phases(h, 0, 15);

@@ -171,6 +171,83 @@ __device__ __forceinline__ double cfl_candidate(const C &c, long long p, double 
     return SALEC_DTF * dmin(dt_r, dt_z);
 }
 
+// The point of this thread of block (bx, by). Blocks are 32 x rows threads, rows a power of two up to
+// SALEC_TILE_ROWS. Without a tile list the grid is two-dimensional; with one it is a row of blocks,
+// several a tile when rows is smaller than a tile's. False, for the whole block, behind the last
+// listed tile.
+template <class C>
+__device__ __forceinline__ bool tile_point(const C &c, int bx, int by, int &i, int &j)
+{
+    if (c.tile_list) {
+        const int sh = __clz(blockDim.y) - __clz(SALEC_TILE_ROWS);   // log2 of the blocks per tile
+        const int t = bx >> sh, sub = bx & ((1 << sh) - 1);
+        if (t >= *c.tile_count) return false;
+        const int e = c.tile_list[t];
+        bx = e & 0xffff;
+        by = ((e >> 16) << sh) + sub;
+    }
+    i = 32 * bx + threadIdx.x;
+    j = by * blockDim.y + threadIdx.y;
+    return true;
+}
+
+// Quiet vacuum: nothing can change in a tile whose cells, and those of the tiles beside it and of two
+// rows above and below, have been pure vacuum at the start of each of the last SALEC_QUIET_CYCLES
+// cycles, the coming one included. Every output of a cycle at such a point is a constant that depends
+// neither on dt nor on the time: vertices have no mass, no velocity and no acceleration, faces sweep
+// no volume, cells keep m_vof = (1, 0, ...) and zeros. The earlier of these cycles stored the
+// constants, in both copies of the donor state, so the sweeps are not run there: the cycle graph
+// visits the listed tiles only. PML2 and PML3 accelerate vacuum vertices by gravity and take no part.
+// The map is forgotten whenever a field is written from outside or the phases run one by one. About
+// half of an impact's mesh lies above its target. Leaving quiet tiles out took
+// the 2048x2048 impact from 1214 to 963 us a cycle and the 1024x1024 one from 399 to 338 (returning
+// early from quiet row segments inside full grids: 1000 and 340).
+#define SALEC_QUIET_CYCLES 4
+
+// The map and the list of the next cycle, one thread per tile, after the remap has set vacuum[].
+template <class C>
+__device__ __forceinline__ void count_quiet(const C &c, int t)
+{
+    const int S = c.tx, tj = t / S, ti = t - tj * S, j0 = SALEC_TILE_ROWS * tj;
+    const bool tile = t < S * c.ty;
+    bool active = false;
+    if (tile) {
+        bool all = tj >= 1 && tj < c.ty - 1 && ti >= 1 && ti < S - 1 && j0 + SALEC_TILE_ROWS + 2 <= c.d.R;
+        if (all) {
+            const unsigned char *v = c.vacuum + (long long)S * (j0 - 2) + ti;
+#pragma unroll
+            for (int r = 0; r < SALEC_TILE_ROWS + 4; ++r, v += S) all = all && v[-1] && v[0] && v[1];
+        }
+        const int n = all ? min(c.quiet[t] + 1, 255) : 0;
+        c.quiet[t] = (unsigned char)n;
+        active = n < SALEC_QUIET_CYCLES;
+    }
+    // the order of the warps in the list is free: no result depends on it
+    const unsigned who = __ballot_sync(0xffffffffu, active);
+    int base = 0;
+    if ((threadIdx.x & 31) == 0 && who) base = atomicAdd(c.next_count, __popc(who));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (active) c.next_list[base + __popc(who & ((1u << (threadIdx.x & 31)) - 1u))] = ti | tj << 16;
+}
+
+// Nothing is known to be quiet: every tile is listed.
+__global__ void k_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < segments) vacuum[t] = 0;
+    if (t < tx * ty) {
+        quiet[t] = 0;
+        list[t] = (t % tx) | (t / tx) << 16;
+    }
+    if (t == 0) *count = tx * ty;
+}
+
+void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
+                         cudaStream_t s)
+{
+    k_forget_quiet<<<(segments + 255) / 256, 256, 0, s>>>(vacuum, segments, quiet, tx, ty, list, count);
+}
+
 // ============================================================ phase 0: surface profile
 // trace_profile (src/ejecta.c:8-63): per column, MIN of cell-centre y over cells whose vacuum
 // fraction exceeds 0.1; cells above the ejecta threshold with no vacuum get e_ejt = 1.
@@ -301,7 +378,8 @@ template <class R>
 __global__ void SALEC_BOUNDS_VOFMOM k_vertex_vof_momentum(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
     vertex_vof(c, i, j);
     vertex_momentum(c, i, j);
@@ -313,7 +391,8 @@ template <class R>
 __global__ void k_cell_velocity(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
@@ -355,7 +434,8 @@ template <class R>
 __global__ void k_void_vertices(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
     const int corner[4] = {2, 3, 0, 1};
@@ -387,7 +467,8 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
 {
     grid_dependency();
     using A = R;   // arithmetic of the gradient and the viscosity: FP64, or FP32 in the mixed form
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     unsigned long long cand = ~0ULL;
     if (cell_interior(c, i, j)) {
         const long long p = KIDX(i, j);
@@ -459,6 +540,7 @@ template <class R>
 __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const CtxT<R> c)
 {
     grid_dependency();
+    if (c.quiet && threadIdx.x == 0 && blockIdx.x == 0) *c.next_count = 0;   // filled by k_cycle
     if (c.dt_sched) {
         const long long k = c.scal->i_step - c.dt_sched_i0;
         if (k >= 0 && k < c.dt_sched_n) {
@@ -516,7 +598,8 @@ __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
     grid_dependency();
     using A = R;   // arithmetic of stress, strength and damage: FP64, or FP32 in the mixed form
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     const int nmat = NM > 0 ? NM : c.d.nmat;
@@ -726,7 +809,8 @@ __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
 {
     grid_dependency();
     using A = R;   // arithmetic of the stress divergence: FP64, or FP32 in the mixed form
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
@@ -833,7 +917,8 @@ template <class R>
 __global__ void k_vertex_displacement(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const double dt = c.scal->dt;
@@ -909,7 +994,8 @@ template <class R, int NM, bool POR>
 __global__ void SALEC_BOUNDS_ENERGY k_energy(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     if (c.f.m_vof[p] > SALEC_TOLVOF || c.f.e_den[p] < SALEC_TOLRHO) return;
@@ -1089,49 +1175,27 @@ __device__ __forceinline__ void cell_swept_volumes(const C &c, int i, int j, dou
     uv = swept_volume(px[3], py[3], px[2], py[2], dx[3], dy[3], dx[2], dy[2]);
 }
 
-// Cell t of the two-cell pad ring, t < 4 enx + 4 (eny - 4): the two bottom rows, the two top
-// rows, then the four pad cells of each row between them (needs enx, eny >= 5).
-__device__ __forceinline__ void pad_ring_cell(int t, int enx, int eny, int &i, int &j)
-{
-    if (t < 2 * enx) {
-        j = t / enx; i = t - j * enx;
-    } else if (t < 4 * enx) {
-        const int u = t - 2 * enx, r = u / enx;
-        j = eny - 2 + r; i = u - r * enx;
-    } else {
-        const int u = t - 4 * enx, r = u >> 2, k = u & 3;
-        j = 2 + r; i = k < 2 ? k : enx - 4 + k;
-    }
-}
-
-// pass 0: interior cells; pass 1: pad cells (after the ghost fills of m_den, m_eng, ...), over
-// the whole grid; pass 2: the same pad cells, one thread each (1-D grid over the pad ring);
-// pass 3: every cell, after the ghost fills. No cell's flux reads a ghost member the fills write
-// except the pad cells' own, and no flux writes what the fills read, so pass 3 computes what
-// passes 0 and 2 around the fills compute, in one launch whose pad cells hide in the interior's
-// waves. The first `tracer_rows` rows of blocks move the tracers instead (they read nothing the
-// fluxes write and write only tracer arrays), so that their chain of dependent loads runs beside
-// the fluxes: as a launch of their own they cost 41 us of the 2048x2048 impact's cycle.
+// Every cell in one launch, after the ghost fills: no interior cell's flux reads a ghost member that
+// the fills write, and no flux writes what the fills read, so this computes what the reference's
+// interior pass, ghost update and pad pass compute, and the pad cells hide in the interior's waves.
+// The first `tracer_blocks` blocks (rows of blocks, on a two-dimensional grid) move the tracers instead (they read nothing the fluxes write and
+// write only tracer arrays), so that their chain of dependent loads runs beside the fluxes: as a
+// launch of their own they cost 41 us of the 2048x2048 impact's cycle.
 template <class R, int NM, bool POR, bool REC = true>
-__global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int pass, int tracer_rows)
+__global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int tracer_blocks)
 {
     grid_dependency();
-    int i, j;
-    if ((int)blockIdx.y < tracer_rows) {
-        const int block = blockIdx.y * gridDim.x + blockIdx.x;
+    int bx = blockIdx.x, by = blockIdx.y;
+    if ((c.tile_list ? bx : by) < tracer_blocks) {
+        const int block = by * gridDim.x + bx;
         move_tracer(c, (block * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x);
         return;
     }
-    if (pass == 2) {
-        const int t = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
-        if (t >= 4 * c.d.enx + 4 * (c.d.eny - 4)) return;
-        pad_ring_cell(t, c.d.enx, c.d.eny, i, j);
-    } else {
-        i = blockIdx.x * blockDim.x + threadIdx.x;
-        j = (blockIdx.y - tracer_rows) * blockDim.y + threadIdx.y;
-        if (i >= c.d.enx || j >= c.d.eny) return;
-        if (pass != 3 && (pass == 0) != cell_interior(c, i, j)) return;
-    }
+    if (c.tile_list) bx -= tracer_blocks;
+    else by -= tracer_blocks;
+    int i, j;
+    if (!tile_point(c, bx, by, i, j)) return;
+    if (i >= c.d.enx || j >= c.d.eny) return;
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
     const int nmat = NM > 0 ? NM : c.d.nmat;
     const long long p = KIDX(i, j);
@@ -1297,7 +1361,8 @@ template <class R, int NM, bool POR>
 __global__ void k_face_records(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (i >= c.d.enx || j >= c.d.eny) return;
     const int nmat = NM > 0 ? NM : c.d.nmat;
     const long long p = KIDX(i, j);
@@ -1847,7 +1912,8 @@ template <class R, int NM, bool POR, bool P3, bool DUAL = false>
 __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_remap, int do_damp, int do_ejecta, int do_state)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (i >= c.d.enx || j >= c.d.eny) return;
     const long long p = KIDX(i, j);
     const bool interior = cell_interior(c, i, j);
@@ -1868,6 +1934,17 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
     }
     if (dirty) store_cell<R, NM, POR>(c, p, s, !state);   // the EOS pass writes e_den itself
     if (state) state_cell<R, NM, POR>(c, p, s);
+    if (DUAL && c.vacuum) {
+        // a warp covers one segment; only whole interior ones count
+        const int i0 = i & ~31;
+        if (i0 < 2 || i0 + 31 > c.d.enx - 3 || j < 2 || j > c.d.eny - 3) return;
+        bool empty = s.vof[0] == 1.0 && s.eden == 0.0;
+        #pragma unroll
+        for (int m = 1; m < (NM > 0 ? NM : c.d.nmat); ++m)
+            empty = empty && s.vof[m] == 0.0 && s.rho[m] == 0.0 && s.eng[m] == 0.0;
+        empty = __all_sync(0xffffffffu, empty);
+        if (i == i0) c.vacuum[c.tx * j + (i >> 5)] = empty;
+    }
 }
 
 // ============================================================ phase 15: cycle control
@@ -1877,6 +1954,7 @@ template <class R>
 __global__ void k_cycle(const CtxT<R> c)
 {
     grid_dependency();
+    if (c.quiet) count_quiet(c, blockIdx.x * blockDim.x + threadIdx.x);
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         Scal *s = c.scal;
         s->time += s->dt;
@@ -1893,7 +1971,8 @@ template <class R>
 __global__ void k_record_reference_state(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     unsigned long long cand = 0ULL;
     if (i < c.d.enx && j < c.d.eny) {
         const long long p = KIDX(i, j);
@@ -1919,7 +1998,8 @@ template <class R>
 __global__ void k_init_vertex_velocity(const CtxT<R> c)
 {
     grid_dependency();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    int i, j;
+    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
@@ -2132,43 +2212,41 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
     } while (0)
 
 template <class R>
-void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, int a0, int a1, int a2, int a3)
+void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 shape, int a0, int a1, int a2, int a3)
 {
     const dim3 b8(32, 8);
-    const dim3 g((c.d.enx + b.x - 1) / b.x, (c.d.eny + b.y - 1) / b.y);   // cells (and faces)
-    const dim3 gv((c.d.vnx + b.x - 1) / b.x, (c.d.vny + b.y - 1) / b.y);  // vertices
+    // a block shape stands for its thread count: rows of 32 points, a power of two of them (tile_point)
+    int rows = 1;
+    while (2 * rows <= SALEC_TILE_ROWS && 64 * rows <= (int)(shape.x * shape.y)) rows *= 2;
+    const dim3 b(32, rows), g = c.tile_list ? dim3(c.tx * c.ty * (SALEC_TILE_ROWS / rows))
+                                            : dim3(c.tx, c.ty * (SALEC_TILE_ROWS / rows));
     const int ncol = (c.d.enx + 255) / 256;
     switch (k) {
     case SK_PROFILE_RESET: launch_dependent(k_profile_reset<R>, ncol, 256, s, c); break;
     case SK_TRACE_PROFILE: launch_dependent(k_trace_profile<R>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
     case SK_PROFILE_DECODE: launch_dependent(k_profile_decode<R>, ncol, 256, s, c); break;
-    case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, gv, b, s, c); break;
+    case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, g, b, s, c); break;
     case SK_CELL_VELOCITY: launch_dependent(k_cell_velocity<R>, g, b, s, c); break;
-    case SK_VOID_VERTICES: launch_dependent(k_void_vertices<R>, gv, b, s, c); break;
+    case SK_VOID_VERTICES: launch_dependent(k_void_vertices<R>, g, b, s, c); break;
     case SK_GRADIENT: launch_dependent(k_gradient_viscosity_cfl<R>, g, b, s, c); break;
     case SK_FINALIZE_DT: launch_dependent(k_finalize_dt<R>, 148, SALEC_FINALIZE_THREADS, s, c); break;
     case SK_STRESS: SALEC_NM_DISPATCH(k_stress, c); break;
     case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, (true), c); break;
-    case SK_ACCELERATION: launch_dependent(k_vertex_acceleration<R>, gv, b, s, c); break;
-    case SK_DISPLACEMENT: launch_dependent(k_vertex_displacement<R>, gv, b, s, c); break;
+    case SK_ACCELERATION: launch_dependent(k_vertex_acceleration<R>, g, b, s, c); break;
+    case SK_DISPLACEMENT: launch_dependent(k_vertex_displacement<R>, g, b, s, c); break;
     case SK_ENERGY: SALEC_NM_DISPATCH(k_energy, c); break;
     case SK_TRACERS:
         if (c.tr.n > 0) launch_dependent(k_tracers<R>, (c.tr.n + 127) / 128, 128, s, c);
         break;
-    case SK_FLUX:
-        if (a0 == 2) {   // pad ring, 1-D
-            const long long ring = 4LL * c.d.enx + 4LL * (c.d.eny - 4);
-            const dim3 g((unsigned)((ring + b.x * b.y - 1) / (b.x * b.y)));
-            SALEC_NM_DISPATCH(k_flux, c, a0, 0);
-        } else {
-            dim3 gt = g;   // a1: the tracers' blocks come first
-            const int per_row = (int)(g.x * b.x * b.y), rows = a1 && c.tr.n > 0 ? (c.tr.n + per_row - 1) / per_row : 0;
-            gt.y += rows;
-            const dim3 g = gt;
-            if (a2) SALEC_NM_DISPATCH_P3(k_flux, (false), c, a0, rows);   // a2: volumes only
-            else SALEC_NM_DISPATCH(k_flux, c, a0, rows);
-        }
+    case SK_FLUX: {
+        const dim3 cells = g;
+        const int per = 32 * rows * (c.tile_list ? 1 : (int)cells.x);   // tracers of a leading block, or row of blocks
+        const int tb = a0 && c.tr.n > 0 ? (c.tr.n + per - 1) / per : 0;
+        const dim3 g = c.tile_list ? dim3(cells.x + tb) : dim3(cells.x, cells.y + tb);
+        if (a1) SALEC_NM_DISPATCH_P3(k_flux, (false), c, tb);
+        else SALEC_NM_DISPATCH(k_flux, c, tb);
         break;
+    }
     case SK_REMAP_DAMP_STATE:
         // the pml3 remap is its own instance so that its extra state costs the others no registers
         if (c.rp.damp_type == 2) SALEC_NM_DISPATCH_P3(k_remap_damp_state, (true), c, a0, a1, a2, a3);
@@ -2184,9 +2262,12 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 b, 
     case SK_STRENGTH_CONDITION:
         if (c.tr.n > 0) launch_dependent(k_strength_condition<R>, (c.tr.n + 127) / 128, 128, s, c);
         break;
-    case SK_CYCLE: launch_dependent(k_cycle<R>, 1, 32, s, c); break;
+    case SK_CYCLE:
+        if (c.quiet) launch_dependent(k_cycle<R>, (c.tx * c.ty + 255) / 256, 256, s, c);
+        else launch_dependent(k_cycle<R>, 1, 32, s, c);
+        break;
     case SK_RECORD_REFERENCE: launch_dependent(k_record_reference_state<R>, g, b, s, c); break;
-    case SK_INIT_VERTEX_VELOCITY: launch_dependent(k_init_vertex_velocity<R>, gv, b, s, c); break;
+    case SK_INIT_VERTEX_VELOCITY: launch_dependent(k_init_vertex_velocity<R>, g, b, s, c); break;
     }
 }
 
