@@ -178,6 +178,9 @@ struct CtxT {
     // next_count are the list under construction for the next cycle. See count_quiet().
     unsigned char *vacuum, *quiet;
     int *next_list, *next_count;
+    // ordered-bits MIN per column of the surface profile (cycle graph: reset by the last kernel of a
+    // cycle, decoded into y_profile beside the time step; null elsewhere)
+    unsigned long long *profile;
 };
 using Ctx = CtxT<double>;
 

@@ -33,6 +33,25 @@ struct GatherBatch {
     int nfield, total;
 };
 
+// The same as a list of entries, one per lane: the entries of a component follow one another inside
+// one warp, so that a warp barrier between the loads and the stores gives every source its original
+// value; lists are padded to whole warps, one field to a warp (dst < 0: no entry).
+struct EdgeEntry {
+    int dst, src;
+    unsigned ops;
+    int field;
+};
+struct EdgeField {
+    void *base;
+    long long plane;
+    int ncomp, f32;
+};
+struct EdgeBatch {
+    EdgeField field[SALEC_MAX_GATHER_FIELDS];
+    const EdgeEntry *entries;
+    int total;
+};
+
 // Host-side gather map of one field: entries in increasing destination order.
 struct GatherMap {
     std::vector<int> dst, src;
@@ -56,7 +75,7 @@ bool group_gather_components(const GatherMap &m, GatherMap &out, std::vector<int
 // Step kernels of salec_step.cu, launched over their own grids by launch_step_kernel; R is
 // the storage type of the relaxed fields (double: plain FP64 form, float: mixed form).
 enum StepKernel {
-    SK_PROFILE_RESET, SK_TRACE_PROFILE, SK_PROFILE_DECODE, SK_VERTEX_VOF_MOMENTUM, SK_CELL_VELOCITY,
+    SK_PROFILE_RESET, SK_TRACE_PROFILE, SK_PROFILE_DECODE, SK_TRACE_ACCUMULATED, SK_VERTEX_VOF_MOMENTUM, SK_CELL_VELOCITY,
     SK_VOID_VERTICES, SK_GRADIENT, SK_FINALIZE_DT, SK_STRESS, SK_ACCELERATION, SK_DISPLACEMENT, SK_ENERGY,
     SK_TRACERS, SK_FLUX, SK_REMAP_DAMP_STATE, SK_CYCLE, SK_RECORD_REFERENCE, SK_INIT_VERTEX_VELOCITY,
     SK_STRENGTH_CONDITION, SK_LAPLACE_MASK, SK_STRESS_ENERGY, SK_REMAP_DUAL, SK_FACE_RECORDS, SK_COUNT
@@ -92,6 +111,7 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 blk
 void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
                          cudaStream_t s);
 __global__ void k_gather(GatherBatch g, int mode, double *scratch);
+__global__ void k_edges(const __grid_constant__ EdgeBatch g);
 void launch_aos_to_planes(const double *aos, void *base, bool f32, long long plane, int P, int nx, int ny, int nc,
                           cudaStream_t s);
 void launch_planes_to_aos(const void *base, bool f32, double *aos, long long plane, int P, int nx, int ny, int nc,

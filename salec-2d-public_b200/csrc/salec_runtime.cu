@@ -102,11 +102,20 @@ const char *kFuncNames[] = {"SimpleRock", "SimpleShear", "JohnsonCook1", "Johnso
                             "IceStrength", "Collins", "Ivanov", "SimpleTensile", "None", "Wunnemann",
                             "VonMises1", "VonMises2"};
 
+// One-launch form of one or more gather maps (k_edges); not ok: some component is too large for it.
+struct Edges {
+    EdgeBatch batch{};
+    int nfield = 0;
+    int fid[SALEC_MAX_GATHER_FIELDS] = {0};   // the fields: their planes can move (salec_gpu::flip)
+    bool ok = false;
+};
+
 struct Gather {
+    Edges edges;
     GatherBatch batch{};
     bool two_pass = false;
     int ncomp_max = 0;
-    int fid[SALEC_MAX_GATHER_FIELDS] = {0};       // the fields: their planes can move (salec_gpu::flip)
+    int fid[SALEC_MAX_GATHER_FIELDS] = {0};
     int entries[SALEC_MAX_GATHER_FIELDS] = {0};   // map entries per field (the adjoint walks entries)
 };
 
@@ -136,6 +145,9 @@ struct salec_gpu {
     size_t scratch_doubles = 0;
     double *staging = nullptr;   // AoS staging for field transfer
     size_t staging_doubles = 0;
+    // batches that the cycle graph joins: g_mvof with g_dvel_den, and r_dis with g_flux_state
+    Edges e_head, e_tail;
+    unsigned long long *profile_acc = nullptr;   // CtxT::profile
     Gather g_mvof, g_dvel_den, g_evel, g_pre_ste_q, g_flux_state, r_vel, r_acc, r_dis, g_init;
     Tracers tr{};
     void *tr_block = nullptr;   // one allocation holding every tracer array
@@ -229,6 +241,7 @@ struct salec_gpu {
         c.tile_list = c.tile_count = nullptr;
         c.next_list = c.next_count = nullptr;
         c.vacuum = c.quiet = nullptr;
+        c.profile = in_graph ? profile_acc : nullptr;
         if (in_graph && quiet_map) {
             c.vacuum = quiet_map;
             c.quiet = quiet_map + segment_bytes();
@@ -310,6 +323,40 @@ int upload_axis(salec_gpu *h, const double *xs, int n, const int **bkt, int *nb,
     return upload_vec(h, v, bkt);
 }
 
+int make_edges(salec_gpu *h, Edges &g, const std::vector<std::pair<int, GatherMap>> &maps)
+{
+    g = Edges();
+    std::vector<EdgeEntry> list;
+    g.nfield = (int)maps.size();
+    for (int k = 0; k < g.nfield; ++k) {
+        const int fid = maps[k].first;
+        g.fid[k] = fid;
+        EdgeField &f = g.batch.field[k];
+        f.base = field_ptr(h, fid);
+        f.f32 = field_f32(h, fid) ? 1 : 0;
+        f.plane = h->d.PL;
+        f.ncomp = field_ncomp(h, fid);
+        const GatherMap &m = maps[k].second;
+        GatherMap grouped;
+        std::vector<int> cstart;
+        if (m.needs_scratch) {
+            if (!group_gather_components(m, grouped, cstart)) return SALEC_OK;
+        } else {
+            for (int e = 0; e <= (int)m.dst.size(); ++e) cstart.push_back(e);
+        }
+        const GatherMap &src = m.needs_scratch ? grouped : m;
+        auto pad = [&](size_t to) { while (list.size() % 32 && list.size() % 32 + to > 32) list.push_back({-1, 0, 0, k}); };
+        for (size_t c = 0; c + 1 < cstart.size(); ++c) {
+            pad(cstart[c + 1] - cstart[c]);
+            for (int e = cstart[c]; e < cstart[c + 1]; ++e) list.push_back({src.dst[e], src.src[e], src.ops[e], k});
+        }
+        pad(33);   // the next field starts a warp
+    }
+    g.batch.total = (int)list.size();
+    g.ok = true;
+    return upload_vec(h, list, &g.batch.entries);
+}
+
 int make_gather(salec_gpu *h, Gather &g, const std::vector<std::pair<int, GatherMap>> &maps)
 {
     g = Gather();
@@ -348,23 +395,32 @@ int make_gather(salec_gpu *h, Gather &g, const std::vector<std::pair<int, Gather
     }
     g.batch.start[maps.size()] = total;
     g.batch.total = total;
+    if (int rc = make_edges(h, g.edges, maps)) return rc;
     if (g.two_pass) h->scratch_doubles = std::max(h->scratch_doubles, (size_t)total * g.ncomp_max);
+    return SALEC_OK;
+}
+
+int run_edges(salec_gpu *h, const Edges &g)
+{
+    if (g.batch.total == 0) return SALEC_OK;
+    EdgeBatch b = g.batch;
+    for (int k = 0; k < g.nfield; ++k) b.field[k].base = field_ptr(h, g.fid[k]);
+    h->launches += 1;
+    launch_dependent(k_edges, (b.total + 255) / 256, 256, h->stream, b);
+    CUDA_TRY(cudaGetLastError());
     return SALEC_OK;
 }
 
 int run_gather(salec_gpu *h, const Gather &g)
 {
+    if (g.edges.ok) return run_edges(h, g.edges);
     if (g.batch.total == 0) return SALEC_OK;
     const int tb = 256, nb = (g.batch.total + tb - 1) / tb;
-    h->launches += g.two_pass ? 2 : 1;
+    h->launches += 2;
     GatherBatch b = g.batch;
     for (int k = 0; k < b.nfield; ++k) b.field[k].base = field_ptr(h, g.fid[k]);
-    if (!g.two_pass) {
-        launch_dependent(k_gather, nb, tb, h->stream, b, 0, nullptr);
-    } else {
-        launch_dependent(k_gather, nb, tb, h->stream, b, 1, h->scratch);
-        launch_dependent(k_gather, nb, tb, h->stream, b, 2, h->scratch);
-    }
+    launch_dependent(k_gather, nb, tb, h->stream, b, 1, h->scratch);
+    launch_dependent(k_gather, nb, tb, h->stream, b, 2, h->scratch);
     CUDA_TRY(cudaGetLastError());
     return SALEC_OK;
 }
@@ -550,12 +606,30 @@ void destroy_cycle_graphs(salec_gpu *h)
 template <class R>
 int run_cycle_t(salec_gpu *h)
 {
-    for (int p = 0; p <= 10; ++p)
+    const CtxT<R> c = h->ctx_t<R>();
+    cudaStream_t s = h->stream;
+    const bool joined = h->e_head.ok && h->e_tail.ok;
+    launch_step_kernel(SK_TRACE_ACCUMULATED, c, s, h->blk[SK_TRACE_PROFILE]);
+    if (joined) {
+        if (int rc = run_edges(h, h->e_head)) return rc;
+        launch_step_kernel(SK_VERTEX_VOF_MOMENTUM, c, s, h->blk[SK_VERTEX_VOF_MOMENTUM]);
+        if (int rc = run_gather(h, h->r_vel)) return rc;
+    } else {
+        if (int rc = run_phase(h, 1, true)) return rc;
+    }
+    for (int p = 3; p <= 8; ++p)
         if (int rc = run_phase(h, p, true)) return rc;
-    // phases 11 and 12: the tracers move in the flux launch
-    if (int rc = run_gather(h, h->g_flux_state)) return rc;
+    // phases 9 to 12: restricted displacements and donor-state ghosts in one batch, then the fluxes,
+    // in whose launch the tracers move
+    if (joined) {
+        launch_step_kernel(SK_DISPLACEMENT, c, s, h->blk[SK_DISPLACEMENT]);
+        if (int rc = run_edges(h, h->e_tail)) return rc;
+    } else {
+        if (int rc = run_phase(h, 9, true)) return rc;
+        if (int rc = run_gather(h, h->g_flux_state)) return rc;
+    }
     const bool dual = h->alt_pool != nullptr;
-    launch_step_kernel(SK_FLUX, h->ctx_t<R>(), h->stream, h->blk[SK_FLUX], 1, dual ? 1 : 0);
+    launch_step_kernel(SK_FLUX, c, s, h->blk[SK_FLUX], 1, dual ? 1 : 0);
     CUDA_TRY(cudaGetLastError());
     if (int rc = run_phase(h, 13, true)) return rc;
     if (!dual) {
@@ -588,6 +662,8 @@ int build_gathers(salec_gpu *h)
     if ((rc = make_gather(h, h->g_pre_ste_q,
                           {gm("e_pre", GP_ALWAYS_COPY), gm("e_ste", GP_STRESS), gm("e_q", GP_ALWAYS_COPY)})))
         return rc;
+    if ((rc = make_edges(h, h->e_head, {gm("m_vof", GP_ALWAYS_COPY), gm("e_dvel", GP_VELOCITY_INC), gm("e_den", GP_DENSITY)})))
+        return rc;
     std::vector<std::pair<int, GatherMap>> fs = {gm("m_den", GP_DENSITY), gm("e_vib", GP_ALWAYS_COPY),
                                                  gm("m_eng", GP_DENSITY)};
     if (h->rp.porosity_model) {
@@ -595,6 +671,8 @@ int build_gathers(salec_gpu *h)
         fs.push_back(gm("e_cvs", GP_ALWAYS_COPY));
     }
     if ((rc = make_gather(h, h->g_flux_state, fs))) return rc;
+    fs.insert(fs.begin(), rm("v_dis"));
+    if ((rc = make_edges(h, h->e_tail, fs))) return rc;
     if ((rc = make_gather(h, h->g_init,
                           {gm("e_den", GP_DENSITY), gm("e_pre", GP_ALWAYS_COPY), gm("e_ste", GP_STRESS),
                            gm("m_eng", GP_DENSITY), gm("m_pty", GP_ALWAYS_COPY), gm("e_cvs", GP_ALWAYS_COPY)})))
@@ -1071,6 +1149,14 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
         off += kFields[k].loc == L_COL ? col * sizeof(double) : (size_t)field_ncomp(h, k) * d.PL * field_elem(h, k);
     }
 
+    {
+        // the cycle graph's surface-profile minima, as the last kernel of a cycle leaves them
+        std::vector<unsigned long long> acc(d.enx, ord_encode(rp.threshold_z * 2.0));
+        const unsigned long long *dev = nullptr;
+        if (int rc = upload_vec(h, acc, &dev)) return bail(rc);
+        if (int rc = flush_uploads(h)) return bail(rc);
+        h->profile_acc = const_cast<unsigned long long *>(dev);
+    }
     allocate_donor_copy(h);
     {
         const size_t words = (size_t)(d.P / 32) * d.R;

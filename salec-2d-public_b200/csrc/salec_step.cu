@@ -259,7 +259,8 @@ __global__ void k_profile_reset(const CtxT<R> c)
     if (i < c.d.enx) c.f.y_profile[i] = __longlong_as_double((long long)ord_encode(c.rp.threshold_z * 2.0));
 }
 
-template <class R>
+// The columns' minima accumulate in y_profile itself between reset and decode, or, ACC, in c.profile.
+template <class R, bool ACC>
 __global__ void k_trace_profile(const CtxT<R> c)
 {
     grid_dependency();
@@ -294,7 +295,7 @@ __global__ void k_trace_profile(const CtxT<R> c)
     __syncthreads();
     if (threadIdx.y == 0 && i < c.d.enx) {
         for (int k = 1; k < 8; ++k) best = min(best, smin[k][threadIdx.x]);
-        if (best != ~0ULL) atomicMin((unsigned long long *)&c.f.y_profile[i], best);
+        if (best != ~0ULL) atomicMin(ACC ? &c.profile[i] : (unsigned long long *)&c.f.y_profile[i], best);
     }
 }
 
@@ -541,6 +542,9 @@ __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const Ct
 {
     grid_dependency();
     if (c.quiet && threadIdx.x == 0 && blockIdx.x == 0) *c.next_count = 0;   // filled by k_cycle
+    if (c.profile)
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c.d.enx; i += gridDim.x * blockDim.x)
+            c.f.y_profile[i] = ord_decode(c.profile[i]);
     if (c.dt_sched) {
         const long long k = c.scal->i_step - c.dt_sched_i0;
         if (k >= 0 && k < c.dt_sched_n) {
@@ -1954,7 +1958,10 @@ template <class R>
 __global__ void k_cycle(const CtxT<R> c)
 {
     grid_dependency();
-    if (c.quiet) count_quiet(c, blockIdx.x * blockDim.x + threadIdx.x);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c.quiet) count_quiet(c, t);
+    if (c.profile)
+        for (int i = t; i < c.d.enx; i += gridDim.x * blockDim.x) c.profile[i] = ord_encode(c.rp.threshold_z * 2.0);
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         Scal *s = c.scal;
         s->time += s->dt;
@@ -2043,9 +2050,8 @@ __global__ void k_laplace_mask(const CtxT<R> c, unsigned *mask)
 }
 
 // ============================================================ boundary gathers
-// Apply a precomputed gather map (built on the host from the reference's ghost and
-// restriction tables): dst[k] = op_c(src[k]) per component c. In-place when no source is also
-// a destination; otherwise gathered through scratch in two passes.
+// Apply a precomputed gather map (built on the host from the reference's ghost and restriction
+// tables): dst[k] = op_c(src[k]) per component c.
 __device__ __forceinline__ double apply_op(unsigned op, double v)
 {
     switch (op) {
@@ -2057,6 +2063,41 @@ __device__ __forceinline__ double apply_op(unsigned op, double v)
     }
 }
 
+// Four planes at a time: every source of the warp's entries is read before any destination is
+// written (the points of a component are touched by no other warp, and planes are disjoint).
+template <class T>
+__device__ __forceinline__ void edge_copy(const EdgeField &f, const EdgeEntry &e)
+{
+    T *base = static_cast<T *>(f.base);
+    for (int c0 = 0; c0 < f.ncomp; c0 += 4) {
+        double v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (c0 + k < f.ncomp && e.dst >= 0)
+                v[k] = apply_op((e.ops >> (3 * (c0 + k))) & 7u, (double)base[(c0 + k) * f.plane + e.src]);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (c0 + k < f.ncomp && e.dst >= 0) base[(c0 + k) * f.plane + e.dst] = (T)v[k];
+    }
+}
+
+// One lane per entry. A batch takes a few microseconds whatever its size: a launch, the entry, its
+// sources. One thread per component, walking up to 16 entries through index arrays, took 2-3 us
+// more (64x80: 35 us a cycle in eight batches, 12 in the five that are left).
+__global__ void __launch_bounds__(256) k_edges(const __grid_constant__ EdgeBatch g)
+{
+    grid_dependency();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.total) return;   // whole warps
+    const EdgeEntry e = g.entries[t];
+    const EdgeField &f = g.field[e.field];
+    if (f.f32) edge_copy<float>(f, e);
+    else edge_copy<double>(f, e);
+}
+
+// The two passes through scratch of a map with a component too large for a warp's list.
+// mode 1: gather into scratch; 2: scatter from scratch
 template <class T>
 __device__ __forceinline__ void gather_one(const GatherField &gf, int mode, long long d, long long s, unsigned ops,
                                            double *scratch, long long row)
@@ -2065,65 +2106,22 @@ __device__ __forceinline__ void gather_one(const GatherField &gf, int mode, long
     for (int comp = 0; comp < gf.ncomp; ++comp) {
         T *plane = base + (long long)comp * gf.plane;
         const unsigned op = (ops >> (3 * comp)) & 7u;
-        if (mode == 0) {
-            plane[d] = (T)apply_op(op, (double)plane[s]);
-        } else if (mode == 1) {
-            scratch[row * gf.ncomp_max + comp] = apply_op(op, (double)plane[s]);
-        } else {
-            plane[d] = (T)scratch[row * gf.ncomp_max + comp];
-        }
+        if (mode == 1) scratch[row * gf.ncomp_max + comp] = apply_op(op, (double)plane[s]);
+        else plane[d] = (T)scratch[row * gf.ncomp_max + comp];
     }
-}
-
-// One component of a map whose sources include destinations: per plane, every source of the
-// component is read before any destination is written, which is what the two passes through
-// scratch do for the whole map (the component's points are touched by no other thread, and
-// planes are disjoint).
-template <class T>
-__device__ __forceinline__ void gather_component(const GatherField &gf, int a, int b)
-{
-    T *base = static_cast<T *>(gf.base);
-    // fixed-length predicated loops: every load of the component is issued before the first
-    // one is needed
-    int src[SALEC_GATHER_MAX_COMPONENT], dst[SALEC_GATHER_MAX_COMPONENT];
-    unsigned ops[SALEC_GATHER_MAX_COMPONENT];
-#pragma unroll
-    for (int e = 0; e < SALEC_GATHER_MAX_COMPONENT; ++e)
-        if (a + e < b) { src[e] = gf.src[a + e]; dst[e] = gf.dst[a + e]; ops[e] = gf.ops[a + e]; }
-    for (int comp = 0; comp < gf.ncomp; ++comp) {
-        T *plane = base + (long long)comp * gf.plane;
-        double v[SALEC_GATHER_MAX_COMPONENT];
-#pragma unroll
-        for (int e = 0; e < SALEC_GATHER_MAX_COMPONENT; ++e)
-            if (a + e < b) v[e] = apply_op((ops[e] >> (3 * comp)) & 7u, (double)plane[src[e]]);
-#pragma unroll
-        for (int e = 0; e < SALEC_GATHER_MAX_COMPONENT; ++e)
-            if (a + e < b) plane[dst[e]] = (T)v[e];
-    }
-}
-
-// mode 0: in place, one entry (or one component, where the field has them) per thread;
-// 1: gather into scratch; 2: scatter from scratch
-__device__ __forceinline__ void gather_item(const GatherBatch &g, int t, int mode, double *scratch)
-{
-    if (t >= g.total) return;
-    int f = 0;
-    while (f + 1 < g.nfield && t >= g.start[f + 1]) ++f;
-    const GatherField &gf = g.field[f];
-    const int k = t - g.start[f];
-    if (mode == 0 && gf.cstart) {
-        if (gf.f32) gather_component<float>(gf, gf.cstart[k], gf.cstart[k + 1]);
-        else gather_component<double>(gf, gf.cstart[k], gf.cstart[k + 1]);
-        return;
-    }
-    if (gf.f32) gather_one<float>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
-    else gather_one<double>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
 }
 
 __global__ void k_gather(GatherBatch g, int mode, double *scratch)
 {
     grid_dependency();
-    gather_item(g, blockIdx.x * blockDim.x + threadIdx.x, mode, scratch);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.total) return;
+    int f = 0;
+    while (f + 1 < g.nfield && t >= g.start[f + 1]) ++f;
+    const GatherField &gf = g.field[f];
+    const int k = t - g.start[f];
+    if (gf.f32) gather_one<float>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
+    else gather_one<double>(gf, mode, gf.dst[k], gf.src[k], gf.ops[k], scratch, t);
 }
 
 // ============================================================ layout conversion
@@ -2223,7 +2221,8 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 sha
     const int ncol = (c.d.enx + 255) / 256;
     switch (k) {
     case SK_PROFILE_RESET: launch_dependent(k_profile_reset<R>, ncol, 256, s, c); break;
-    case SK_TRACE_PROFILE: launch_dependent(k_trace_profile<R>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
+    case SK_TRACE_PROFILE: launch_dependent(k_trace_profile<R, false>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
+    case SK_TRACE_ACCUMULATED: launch_dependent(k_trace_profile<R, true>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
     case SK_PROFILE_DECODE: launch_dependent(k_profile_decode<R>, ncol, 256, s, c); break;
     case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, g, b, s, c); break;
     case SK_CELL_VELOCITY: launch_dependent(k_cell_velocity<R>, g, b, s, c); break;
@@ -2264,6 +2263,7 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 sha
         break;
     case SK_CYCLE:
         if (c.quiet) launch_dependent(k_cycle<R>, (c.tx * c.ty + 255) / 256, 256, s, c);
+        else if (c.profile) launch_dependent(k_cycle<R>, ncol, 256, s, c);
         else launch_dependent(k_cycle<R>, 1, 32, s, c);
         break;
     case SK_RECORD_REFERENCE: launch_dependent(k_record_reference_state<R>, g, b, s, c); break;
