@@ -101,7 +101,7 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// flux: a0 = the tracers move in the same launch, a1 = face volumes only; remap: a0..a3 = remap,
+// gradient: a0 = with the void vertices of phase 4; flux: a0 = the tracers move in the same launch, a1 = face volumes only; remap: a0..a3 = remap,
 // damping, ejecta drag, EOS switches. blk is the block shape of the 2-D sweeps (cells, faces,
 // vertices), of which the thread count matters; the surface profile, the Laplacian mask, the tracer and
 // the single-thread kernels use their own fixed shapes.

@@ -617,7 +617,9 @@ int run_cycle_t(salec_gpu *h)
     } else {
         if (int rc = run_phase(h, 1, true)) return rc;
     }
-    for (int p = 3; p <= 8; ++p)
+    if (int rc = run_phase(h, 3, true)) return rc;
+    launch_step_kernel(SK_GRADIENT, c, s, h->blk[SK_GRADIENT], 1);   // phases 4 and 5
+    for (int p = 6; p <= 8; ++p)
         if (int rc = run_phase(h, p, true)) return rc;
     // phases 9 to 12: restricted displacements and donor-state ghosts in one batch, then the fluxes,
     // in whose launch the tracers move

@@ -431,6 +431,29 @@ __global__ void k_cell_velocity(const CtxT<R> c)
 // ============================================================ phase 4: void vertices
 // check_v_vel (src/sale2d.c:1051-1142): a vertex whose four corners are all void takes the
 // density-weighted velocity of its non-empty cells.
+// corners: the vertex's count of void corners (v_mass[1], set by the momentum sweep from the same
+// e_wpt). True where the vertex takes the velocity (vx, vy).
+template <class C>
+__device__ __forceinline__ bool void_velocity(const C &c, int i, int j, double corners, double &vx, double &vy)
+{
+    if (corners < 4.) return false;
+    const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
+    double ax = 0., ay = 0., ad = 0.;
+    int void_cell = 0;
+    for (int k = 0; k < 4; ++k) {
+        const double rho = c.f.e_den[cl[k]];
+        if (rho < SALEC_TOLRHO) { void_cell++; continue; }
+        ad += rho;
+        ax += rho * c.f.e_vel[cl[k]];
+        ay += rho * PLN(c.f.e_vel, 1)[cl[k]];
+    }
+    if (void_cell >= 4) return false;
+    const double s = 1.0 / ad;
+    vx = s * ax;
+    vy = s * ay;
+    return true;
+}
+
 template <class R>
 __global__ void k_void_vertices(const CtxT<R> c)
 {
@@ -438,32 +461,21 @@ __global__ void k_void_vertices(const CtxT<R> c)
     int i, j;
     if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     if (!vert_active(c, i, j)) return;
-    const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
-    const int corner[4] = {2, 3, 0, 1};
-    int void_cell = 0, void_corner = 0;
-    for (int k = 0; k < 4; ++k) {
-        if (c.f.e_den[cl[k]] < SALEC_TOLRHO) void_cell++;
-        if (PLN(c.f.e_wpt, corner[k])[cl[k]] > 0.) void_corner++;
-    }
-    if (void_cell >= 4 || void_corner < 4) return;
-    double ax = 0., ay = 0., ad = 0.;
-    for (int k = 0; k < 4; ++k) {
-        const double rho = c.f.e_den[cl[k]];
-        if (rho < SALEC_TOLRHO) continue;
-        ad += rho;
-        ax += rho * c.f.e_vel[cl[k]];
-        ay += rho * PLN(c.f.e_vel, 1)[cl[k]];
-    }
-    const double s = 1.0 / ad;
     const long long p = KIDX(i, j);
-    c.f.v_vel[p] = s * ax;
-    PLN(c.f.v_vel, 1)[p] = s * ay;
+    double vx, vy;
+    if (!void_velocity(c, i, j, PLN(c.f.v_mass, 1)[p], vx, vy)) return;
+    c.f.v_vel[p] = vx;
+    PLN(c.f.v_vel, 1)[p] = vy;
 }
 
 // ============================================================ phase 5 (+6): velocity gradient,
 // artificial viscosity and the CFL candidate of every interior cell.
 // update_e_gradvel (src/sale2d.c:1144-1236) and calculate_dt (src/sale2d.c:1959-2016).
-template <class R>
+// VOID (the cycle graph): phase 4 runs here too. A thread corrects the vertex of its own index and
+// every cell takes a corrected corner from void_velocity itself, so that no thread depends on when
+// another one stores; the sweep of its own read the five fields that the corner count replaces
+// (2048x2048: 28 us).
+template <class R, bool VOID>
 __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
 {
     grid_dependency();
@@ -471,11 +483,28 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
     int i, j;
     if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     unsigned long long cand = ~0ULL;
+    if (VOID && vert_active(c, i, j)) {
+        const long long p = KIDX(i, j);
+        double x, y;
+        if (void_velocity(c, i, j, PLN(c.f.v_mass, 1)[p], x, y)) {
+            c.f.v_vel[p] = x;
+            PLN(c.f.v_vel, 1)[p] = y;
+        }
+    }
     if (cell_interior(c, i, j)) {
         const long long p = KIDX(i, j);
         const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
         A vx[4], vy[4];
         for (int k = 0; k < 4; ++k) { vx[k] = c.f.v_vel[vl[k]]; vy[k] = PLN(c.f.v_vel, 1)[vl[k]]; }
+        if (VOID) {
+            R corners[4];
+            for (int k = 0; k < 4; ++k) corners[k] = PLN(c.f.v_mass, 1)[vl[k]];
+            for (int k = 0; k < 4; ++k) {
+                double x, y;
+                const int di = k == 1 || k == 2, dj = k >= 2;
+                if (void_velocity(c, i + di, j + dj, corners[k], x, y)) { vx[k] = R(x); vy[k] = R(y); }
+            }
+        }
         A g[12];
         for (int k = 0; k < 12; ++k) g[k] = GEO(c.g_e_grad, k);
         A d0 = A(0.), d1 = A(0.), d2 = A(0.), d3 = A(0.), d4 = A(0.);
@@ -2227,7 +2256,10 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 sha
     case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, g, b, s, c); break;
     case SK_CELL_VELOCITY: launch_dependent(k_cell_velocity<R>, g, b, s, c); break;
     case SK_VOID_VERTICES: launch_dependent(k_void_vertices<R>, g, b, s, c); break;
-    case SK_GRADIENT: launch_dependent(k_gradient_viscosity_cfl<R>, g, b, s, c); break;
+    case SK_GRADIENT:
+        if (a0) launch_dependent(k_gradient_viscosity_cfl<R, true>, g, b, s, c);   // a0: with the void vertices
+        else launch_dependent(k_gradient_viscosity_cfl<R, false>, g, b, s, c);
+        break;
     case SK_FINALIZE_DT: launch_dependent(k_finalize_dt<R>, 148, SALEC_FINALIZE_THREADS, s, c); break;
     case SK_STRESS: SALEC_NM_DISPATCH(k_stress, c); break;
     case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, (true), c); break;
