@@ -1499,8 +1499,10 @@ int salec_gpu_set_block_shapes(salec_gpu *h, const int *shapes, int n)
 int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
 {
     if (!h || cycles < 1) return fail(SALEC_ERR_ARG, "bad argument");
-    static const dim3 cand[] = {dim3(32, 4), dim3(32, 8), dim3(64, 2), dim3(32, 2), dim3(64, 4), dim3(128, 1),
-                                dim3(32, 1), dim3(64, 1)};
+    // a shape stands for its thread count (launch_step_kernel). 32x1 is not offered: timed sweep by sweep
+    // it ties with the others, but one block per row segment of a listed tile costs the cycle graph
+    // up to 30 us a sweep (2048x2048: 956-996 us a cycle with one sweep at 32x1, 920-930 without)
+    static const dim3 cand[] = {dim3(32, 4), dim3(32, 8), dim3(32, 2)};
     constexpr int ncand = sizeof(cand) / sizeof(cand[0]);
     const int *tuned_phase = kTunedPhase;
     const StepKernel *tuned_kernel = kTunedKernel;
