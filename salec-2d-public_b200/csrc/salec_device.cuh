@@ -90,6 +90,14 @@ struct Scal {
     unsigned int dt_tail_blocks, pad_;
 };
 
+// Page-locked record that k_report fills: the scalars, the ticket of the report they belong to, and
+// the surface profile behind them.
+struct Report {
+    double dt, time;
+    unsigned ticket, pad_[3];
+    __host__ __device__ double *profile() { return reinterpret_cast<double *>(this + 1); }
+};
+
 // Device planes of every field. R is the storage type of the "relaxed" fields: double in the
 // plain FP64 form, float in the mixed form. The fields that carry volume-fraction advection,
 // mass and energy conservation and the mesh positions stay FP64 in both forms (m_vof, m_den,

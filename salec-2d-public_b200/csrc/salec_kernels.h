@@ -7,6 +7,8 @@ namespace salec {
 
 template <class R>
 struct CtxT;   // salec_device.cuh
+struct Scal;
+struct Report;
 
 #define SALEC_MAX_GATHER_FIELDS 8
 
@@ -110,6 +112,7 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 blk
                         int a2 = 0, int a3 = 0);
 void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
                          cudaStream_t s);
+void launch_report(const Scal *scal, const double *profile, int n, Report *out, unsigned ticket, cudaStream_t s);
 __global__ void k_gather(GatherBatch g, int mode, double *scratch);
 __global__ void k_edges(const __grid_constant__ EdgeBatch g);
 void launch_aos_to_planes(const double *aos, void *base, bool f32, long long plane, int P, int nx, int ny, int nc,

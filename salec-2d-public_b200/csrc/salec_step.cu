@@ -2000,6 +2000,29 @@ __global__ void k_cycle(const CtxT<R> c)
     }
 }
 
+// Read-back of a cycle's report: dt, time and (n > 0) the surface profile, written to page-locked host
+// memory, then `ticket`, which the host waits for. One block: a few kilobytes and a flag.
+__global__ void __launch_bounds__(512) k_report(const Scal *scal, const double *profile, int n, Report *out, unsigned ticket)
+{
+    grid_dependency();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) out->profile()[i] = profile[i];
+    if (threadIdx.x == 0) {
+        out->dt = scal->dt;
+        out->time = scal->time;
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence_system();
+        *const_cast<volatile unsigned *>(&out->ticket) = ticket;
+    }
+}
+
+void launch_report(const Scal *scal, const double *profile, int n, Report *out, unsigned ticket, cudaStream_t s)
+{
+    launch_dependent(k_report, 1, 512, s, scal, profile, n, out, ticket);
+}
+
 // ============================================================ initialisation sweeps
 // record_avg_value (src/sale2d.c:1562-1627): reference state of the damping layers and the
 // latest arrival time of the impact wave at a damped cell (MAX over cells).
