@@ -43,6 +43,11 @@ __device__ __forceinline__ void grid_dependency()
 #ifndef SALEC_REGS_FLUX
 #define SALEC_REGS_FLUX 80
 #endif
+// the flux that stores volumes only (the cycle graph's): us at 2048x2048 FP64 with three materials,
+// layered 1024x1024 and 1536x1536 mixed: 104/54/58 at 64, 102/57/59 at 72, 110/57/62 at 80
+#ifndef SALEC_REGS_FLUX_VOLUMES
+#define SALEC_REGS_FLUX_VOLUMES (NM == 0 || NM >= 4 || sizeof(R) == 4 ? 64 : 72)
+#endif
 #ifndef SALEC_REGS_REMAP
 #define SALEC_REGS_REMAP 96
 #endif
@@ -106,7 +111,8 @@ __device__ __forceinline__ void grid_dependency()
 #define SALEC_BOUNDS_STRESS __launch_bounds__(256)
 #endif
 #if SALEC_REGS_FLUX > 0
-#define SALEC_BOUNDS_FLUX __maxnreg__((sizeof(R) == 4 ? SALEC_REGS_FLUX_F : SALEC_REGS_FLUX))
+#define SALEC_BOUNDS_FLUX                                                                                \
+    __maxnreg__((!REC ? SALEC_REGS_FLUX_VOLUMES : sizeof(R) == 4 ? SALEC_REGS_FLUX_F : SALEC_REGS_FLUX))
 #else
 #define SALEC_BOUNDS_FLUX __launch_bounds__(256)
 #endif
@@ -171,24 +177,46 @@ __device__ __forceinline__ double cfl_candidate(const C &c, long long p, double 
     return SALEC_DTF * dmin(dt_r, dt_z);
 }
 
-// The point of this thread of block (bx, by). Blocks are 32 x rows threads, rows a power of two up to
-// SALEC_TILE_ROWS. Without a tile list the grid is two-dimensional; with one it is a row of blocks,
-// several a tile when rows is smaller than a tile's. False, for the whole block, behind the last
-// listed tile.
-template <class C>
-__device__ __forceinline__ bool tile_point(const C &c, int bx, int by, int &i, int &j)
+// The point of this thread on a two-dimensional grid of 32 x rows blocks.
+#define GRID_POINT(i, j) const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y
+
+// f(i, j) for the points of this thread. Blocks are 32 x rows threads, rows a power of two up to
+// SALEC_TILE_ROWS. Without a tile list each thread of a two-dimensional grid has one point (`lead` rows
+// of blocks do something else first). With one there are `lead` other blocks and then, WALK, as many
+// blocks as the device holds at once, walking the list, each on its next tile's entry while it works on
+// this one, or else a block or more per tile. Looking up the count and the entry takes a block per tile
+// a third of its life where the sweep is short: the four light sweeps walk (2048x2048: displacement 40
+// -> 26 us, gradient 102 -> 88, cell velocity 50 -> 42, vertex momentum 85 -> 82). The heavy ones do not:
+// their tiles differ too much in cost for equal shares (layered 1024x1024: flux 48 -> 57, remap 123 ->
+// 131), and the acceleration spills around the loop (88 -> 180).
+template <bool WALK, class C, class F>
+__device__ __forceinline__ void for_points(const C &c, int lead, F f)
 {
-    if (c.tile_list) {
-        const int sh = __clz(blockDim.y) - __clz(SALEC_TILE_ROWS);   // log2 of the blocks per tile
-        const int t = bx >> sh, sub = bx & ((1 << sh) - 1);
-        if (t >= *c.tile_count) return false;
-        const int e = c.tile_list[t];
-        bx = e & 0xffff;
-        by = ((e >> 16) << sh) + sub;
+    const int sh = __clz(blockDim.y) - __clz(SALEC_TILE_ROWS);   // log2 of the blocks per tile
+    const bool listed = c.tile_list != nullptr;
+    int b = blockIdx.x, n = 0, e = 0;
+    if (listed) {
+        b -= lead;
+        n = *c.tile_count << sh;
+        if (b >= n) return;
+        e = c.tile_list[b >> sh];
     }
-    i = 32 * bx + threadIdx.x;
-    j = by * blockDim.y + threadIdx.y;
-    return true;
+    for (;;) {
+        const int next = b + (int)gridDim.x - lead;
+        int e_next = 0, i, j;
+        if (listed) {
+            if (WALK && next < n) e_next = c.tile_list[next >> sh];
+            i = 32 * (e & 0xffff) + threadIdx.x;
+            j = (((e >> 16) << sh) + (b & ((1 << sh) - 1))) * blockDim.y + threadIdx.y;
+        } else {
+            i = 32 * b + threadIdx.x;
+            j = (blockIdx.y - lead) * blockDim.y + threadIdx.y;
+        }
+        f(i, j);
+        if (!WALK || !listed || next >= n) return;
+        b = next;
+        e = e_next;
+    }
 }
 
 // Quiet vacuum: nothing can change in a tile whose cells, and those of the tiles beside it and of two
@@ -379,11 +407,11 @@ template <class R>
 __global__ void SALEC_BOUNDS_VOFMOM k_vertex_vof_momentum(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<true>(c, 0, [&](int i, int j) {
     if (!vert_active(c, i, j)) return;
     vertex_vof(c, i, j);
     vertex_momentum(c, i, j);
+    });
 }
 
 // ============================================================ phase 3: cell velocity
@@ -392,8 +420,7 @@ template <class R>
 __global__ void k_cell_velocity(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<true>(c, 0, [&](int i, int j) {
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
@@ -426,6 +453,7 @@ __global__ void k_cell_velocity(const CtxT<R> c)
     }
     c.f.e_vel[p] = ex;
     PLN(c.f.e_vel, 1)[p] = ey;
+    });
 }
 
 // ============================================================ phase 4: void vertices
@@ -458,8 +486,7 @@ template <class R>
 __global__ void k_void_vertices(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    GRID_POINT(i, j);
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     double vx, vy;
@@ -480,9 +507,8 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
 {
     grid_dependency();
     using A = R;   // arithmetic of the gradient and the viscosity: FP64, or FP32 in the mixed form
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
     unsigned long long cand = ~0ULL;
+    for_points<true>(c, 0, [&](int i, int j) {
     if (VOID && vert_active(c, i, j)) {
         const long long p = KIDX(i, j);
         double x, y;
@@ -538,10 +564,11 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
         // by its position in the reference's traversal order instead (see k_finalize_dt)
         if (!(vof0 > 1.0 - SALEC_TOLVOF)) {
             const double dt_rz = cfl_candidate(c, p, (double)csd);
-            if (dt_rz == dt_rz) cand = ord_encode(dt_rz);
+            if (dt_rz == dt_rz) cand = min(cand, ord_encode(dt_rz));
             else atomicMax(&c.scal->dt_nan_last, (long long)j * c.d.enx + i);
         }
     }
+    });
     // block MIN, one atomic per block
     for (int o = 16; o > 0; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
     __shared__ unsigned long long wmin[32];
@@ -631,8 +658,7 @@ __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
     grid_dependency();
     using A = R;   // arithmetic of stress, strength and damage: FP64, or FP32 in the mixed form
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<false>(c, 0, [&](int i, int j) {
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     const int nmat = NM > 0 ? NM : c.d.nmat;
@@ -831,6 +857,7 @@ __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
     c.f.e_strength[p] = strength;
     if (EN && !(rho < SALEC_TOLRHO))
         energy_cell<R, NM, POR>(c, p, R(s0), R(s1), R(s2), R(s3), g0, g1, g2, g3, g4, pre);
+    });
 }
 
 // ============================================================ phase 8: vertex acceleration
@@ -842,8 +869,7 @@ __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
 {
     grid_dependency();
     using A = R;   // arithmetic of the stress divergence: FP64, or FP32 in the mixed form
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<false>(c, 0, [&](int i, int j) {
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
@@ -942,6 +968,7 @@ __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
     if (fabs(ay) < A(c.rp.acceleration_min * 1)) ay = A(0.);
     c.f.v_acc[p] = ax;
     PLN(c.f.v_acc, 1)[p] = ay;
+    });
 }
 
 // ============================================================ phase 9: vertex displacement
@@ -950,8 +977,7 @@ template <class R>
 __global__ void k_vertex_displacement(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<true>(c, 0, [&](int i, int j) {
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const double dt = c.scal->dt;
@@ -961,6 +987,7 @@ __global__ void k_vertex_displacement(const CtxT<R> c)
         PLN(c.f.v_dis, k)[p] = dt * v + hdt2 * a;
         PLN(c.f.v_vel, k)[p] = v + dt * a;
     }
+    });
 }
 
 // ============================================================ phase 10: internal energy
@@ -1027,8 +1054,7 @@ template <class R, int NM, bool POR>
 __global__ void SALEC_BOUNDS_ENERGY k_energy(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    GRID_POINT(i, j);
     if (!cell_interior(c, i, j)) return;
     const long long p = KIDX(i, j);
     if (c.f.m_vof[p] > SALEC_TOLVOF || c.f.e_den[p] < SALEC_TOLRHO) return;
@@ -1218,16 +1244,12 @@ template <class R, int NM, bool POR, bool REC = true>
 __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int tracer_blocks)
 {
     grid_dependency();
-    int bx = blockIdx.x, by = blockIdx.y;
-    if ((c.tile_list ? bx : by) < tracer_blocks) {
-        const int block = by * gridDim.x + bx;
+    if ((int)(c.tile_list ? blockIdx.x : blockIdx.y) < tracer_blocks) {
+        const int block = blockIdx.y * gridDim.x + blockIdx.x;
         move_tracer(c, (block * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x);
         return;
     }
-    if (c.tile_list) bx -= tracer_blocks;
-    else by -= tracer_blocks;
-    int i, j;
-    if (!tile_point(c, bx, by, i, j)) return;
+    for_points<false>(c, tracer_blocks, [&](int i, int j) {
     if (i >= c.d.enx || j >= c.d.eny) return;
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
     const int nmat = NM > 0 ? NM : c.d.nmat;
@@ -1385,6 +1407,7 @@ __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int tracer_blocks)
     store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j), bv, flux, 1, p, nmat);
     store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i + 1, j), rv, flux, 2, p, nmat);
     store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j + 1), uv, flux, 3, p, nmat);
+    });
 }
 
 // Donor members of the face records of a cycle whose fluxes stored volumes only, for readers of
@@ -1394,8 +1417,7 @@ template <class R, int NM, bool POR>
 __global__ void k_face_records(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    GRID_POINT(i, j);
     if (i >= c.d.enx || j >= c.d.eny) return;
     const int nmat = NM > 0 ? NM : c.d.nmat;
     const long long p = KIDX(i, j);
@@ -1945,8 +1967,7 @@ template <class R, int NM, bool POR, bool P3, bool DUAL = false>
 __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_remap, int do_damp, int do_ejecta, int do_state)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    for_points<false>(c, 0, [&](int i, int j) {
     if (i >= c.d.enx || j >= c.d.eny) return;
     const long long p = KIDX(i, j);
     const bool interior = cell_interior(c, i, j);
@@ -1978,6 +1999,7 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
         empty = __all_sync(0xffffffffu, empty);
         if (i == i0) c.vacuum[c.tx * j + (i >> 5)] = empty;
     }
+    });
 }
 
 // ============================================================ phase 15: cycle control
@@ -2030,8 +2052,7 @@ template <class R>
 __global__ void k_record_reference_state(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    GRID_POINT(i, j);
     unsigned long long cand = 0ULL;
     if (i < c.d.enx && j < c.d.eny) {
         const long long p = KIDX(i, j);
@@ -2057,8 +2078,7 @@ template <class R>
 __global__ void k_init_vertex_velocity(const CtxT<R> c)
 {
     grid_dependency();
-    int i, j;
-    if (!tile_point(c, blockIdx.x, blockIdx.y, i, j)) return;
+    GRID_POINT(i, j);
     if (!vert_active(c, i, j)) return;
     const long long p = KIDX(i, j);
     const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
@@ -2240,11 +2260,11 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
     do {                                                                                                       \
         const bool por_ = c.rp.porosity_model != 0;                                                            \
         switch (c.d.nmat) {                                                                                    \
-        case 2: if (por_) launch_dependent(KERNEL<R, 2, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false>, g, b, s, __VA_ARGS__); break; \
-        case 3: if (por_) launch_dependent(KERNEL<R, 3, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false>, g, b, s, __VA_ARGS__); break; \
-        case 4: if (por_) launch_dependent(KERNEL<R, 4, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false>, g, b, s, __VA_ARGS__); break; \
-        case 5: if (por_) launch_dependent(KERNEL<R, 5, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false>, g, b, s, __VA_ARGS__); break; \
-        default: if (por_) launch_dependent(KERNEL<R, 0, true>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false>, g, b, s, __VA_ARGS__); break; \
+        case 2: if (por_) points(KERNEL<R, 2, true>, __VA_ARGS__); else points(KERNEL<R, 2, false>, __VA_ARGS__); break; \
+        case 3: if (por_) points(KERNEL<R, 3, true>, __VA_ARGS__); else points(KERNEL<R, 3, false>, __VA_ARGS__); break; \
+        case 4: if (por_) points(KERNEL<R, 4, true>, __VA_ARGS__); else points(KERNEL<R, 4, false>, __VA_ARGS__); break; \
+        case 5: if (por_) points(KERNEL<R, 5, true>, __VA_ARGS__); else points(KERNEL<R, 5, false>, __VA_ARGS__); break; \
+        default: if (por_) points(KERNEL<R, 0, true>, __VA_ARGS__); else points(KERNEL<R, 0, false>, __VA_ARGS__); break; \
         }                                                                                                      \
     } while (0)
 
@@ -2253,11 +2273,11 @@ void launch_count_nonfinite(const void *base, bool f32, long long n, unsigned lo
     do {                                                                                                       \
         const bool por_ = c.rp.porosity_model != 0;                                                            \
         switch (c.d.nmat) {                                                                                    \
-        case 2: if (por_) launch_dependent(KERNEL<R, 2, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 2, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
-        case 3: if (por_) launch_dependent(KERNEL<R, 3, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 3, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
-        case 4: if (por_) launch_dependent(KERNEL<R, 4, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 4, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
-        case 5: if (por_) launch_dependent(KERNEL<R, 5, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 5, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
-        default: if (por_) launch_dependent(KERNEL<R, 0, true, SALEC_LIST X>, g, b, s, __VA_ARGS__); else launch_dependent(KERNEL<R, 0, false, SALEC_LIST X>, g, b, s, __VA_ARGS__); break; \
+        case 2: if (por_) points(KERNEL<R, 2, true, SALEC_LIST X>, __VA_ARGS__); else points(KERNEL<R, 2, false, SALEC_LIST X>, __VA_ARGS__); break; \
+        case 3: if (por_) points(KERNEL<R, 3, true, SALEC_LIST X>, __VA_ARGS__); else points(KERNEL<R, 3, false, SALEC_LIST X>, __VA_ARGS__); break; \
+        case 4: if (por_) points(KERNEL<R, 4, true, SALEC_LIST X>, __VA_ARGS__); else points(KERNEL<R, 4, false, SALEC_LIST X>, __VA_ARGS__); break; \
+        case 5: if (por_) points(KERNEL<R, 5, true, SALEC_LIST X>, __VA_ARGS__); else points(KERNEL<R, 5, false, SALEC_LIST X>, __VA_ARGS__); break; \
+        default: if (por_) points(KERNEL<R, 0, true, SALEC_LIST X>, __VA_ARGS__); else points(KERNEL<R, 0, false, SALEC_LIST X>, __VA_ARGS__); break; \
         }                                                                                                      \
     } while (0)
 
@@ -2265,40 +2285,52 @@ template <class R>
 void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 shape, int a0, int a1, int a2, int a3)
 {
     const dim3 b8(32, 8);
-    // a block shape stands for its thread count: rows of 32 points, a power of two of them (tile_point)
+    // a block shape stands for its thread count: rows of 32 points, a power of two of them (for_points)
     int rows = 1;
     while (2 * rows <= SALEC_TILE_ROWS && 64 * rows <= (int)(shape.x * shape.y)) rows *= 2;
-    const dim3 b(32, rows), g = c.tile_list ? dim3(c.tx * c.ty * (SALEC_TILE_ROWS / rows))
-                                            : dim3(c.tx, c.ty * (SALEC_TILE_ROWS / rows));
+    const dim3 b(32, rows), g(c.tx, c.ty * (SALEC_TILE_ROWS / rows));
     const int ncol = (c.d.enx + 255) / 256;
+    // a sweep over points: the whole two-dimensional grid, or the walkers of a tile list (for_points)
+    int lead = 0;
+    bool walk = false;
+    auto points = [&](auto kernel, auto... args) {
+        dim3 grid(g.x, g.y + lead);
+        if (c.tile_list && !walk) grid = dim3(lead + g.x * g.y);
+        if (c.tile_list && walk) {
+            int dev = 0, sms = 0, per_sm = 0;
+            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)(b.x * b.y), 0);
+            grid = dim3(lead + max(1, min((int)(g.x * g.y), sms * per_sm)));
+        }
+        launch_dependent(kernel, grid, b, s, args...);
+    };
     switch (k) {
     case SK_PROFILE_RESET: launch_dependent(k_profile_reset<R>, ncol, 256, s, c); break;
     case SK_TRACE_PROFILE: launch_dependent(k_trace_profile<R, false>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
     case SK_TRACE_ACCUMULATED: launch_dependent(k_trace_profile<R, true>, dim3((c.d.enx + 31) / 32, (c.d.eny + 63) / 64), b8, s, c); break;
     case SK_PROFILE_DECODE: launch_dependent(k_profile_decode<R>, ncol, 256, s, c); break;
-    case SK_VERTEX_VOF_MOMENTUM: launch_dependent(k_vertex_vof_momentum<R>, g, b, s, c); break;
-    case SK_CELL_VELOCITY: launch_dependent(k_cell_velocity<R>, g, b, s, c); break;
+    case SK_VERTEX_VOF_MOMENTUM: walk = true; points(k_vertex_vof_momentum<R>, c); break;
+    case SK_CELL_VELOCITY: walk = true; points(k_cell_velocity<R>, c); break;
     case SK_VOID_VERTICES: launch_dependent(k_void_vertices<R>, g, b, s, c); break;
     case SK_GRADIENT:
-        if (a0) launch_dependent(k_gradient_viscosity_cfl<R, true>, g, b, s, c);   // a0: with the void vertices
-        else launch_dependent(k_gradient_viscosity_cfl<R, false>, g, b, s, c);
+        walk = true;
+        if (a0) points(k_gradient_viscosity_cfl<R, true>, c);   // a0: with the void vertices
+        else points(k_gradient_viscosity_cfl<R, false>, c);
         break;
     case SK_FINALIZE_DT: launch_dependent(k_finalize_dt<R>, 148, SALEC_FINALIZE_THREADS, s, c); break;
     case SK_STRESS: SALEC_NM_DISPATCH(k_stress, c); break;
     case SK_STRESS_ENERGY: SALEC_NM_DISPATCH_P3(k_stress, (true), c); break;
-    case SK_ACCELERATION: launch_dependent(k_vertex_acceleration<R>, g, b, s, c); break;
-    case SK_DISPLACEMENT: launch_dependent(k_vertex_displacement<R>, g, b, s, c); break;
+    case SK_ACCELERATION: points(k_vertex_acceleration<R>, c); break;
+    case SK_DISPLACEMENT: walk = true; points(k_vertex_displacement<R>, c); break;
     case SK_ENERGY: SALEC_NM_DISPATCH(k_energy, c); break;
     case SK_TRACERS:
         if (c.tr.n > 0) launch_dependent(k_tracers<R>, (c.tr.n + 127) / 128, 128, s, c);
         break;
     case SK_FLUX: {
-        const dim3 cells = g;
-        const int per = 32 * rows * (c.tile_list ? 1 : (int)cells.x);   // tracers of a leading block, or row of blocks
-        const int tb = a0 && c.tr.n > 0 ? (c.tr.n + per - 1) / per : 0;
-        const dim3 g = c.tile_list ? dim3(cells.x + tb) : dim3(cells.x, cells.y + tb);
-        if (a1) SALEC_NM_DISPATCH_P3(k_flux, (false), c, tb);
-        else SALEC_NM_DISPATCH(k_flux, c, tb);
+        const int per = 32 * rows * (c.tile_list ? 1 : (int)g.x);   // tracers of a leading block, or row of blocks
+        lead = a0 && c.tr.n > 0 ? (c.tr.n + per - 1) / per : 0;
+        if (a1) SALEC_NM_DISPATCH_P3(k_flux, (false), c, lead);
+        else SALEC_NM_DISPATCH(k_flux, c, lead);
         break;
     }
     case SK_REMAP_DAMP_STATE:
