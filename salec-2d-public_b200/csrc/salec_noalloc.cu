@@ -10,7 +10,7 @@
 // Facts a caller must know:
 //  - the scratch arrays hold SALEC_CFL_MAX_PARTIALS partial minima (64 KiB) and as many one-byte
 //    NaN flags (8 KiB) on every device that loads the library, for the life of the process;
-//  - one partial covers SALEC_CFL_CELLS_PER_BLOCK interior cells, so a call accepts at most
+//  - one partial covers at most SALEC_CFL_CELLS_PER_BLOCK interior cells, so a call accepts at most
 //    SALEC_CFL_MAX_PARTIALS * SALEC_CFL_CELLS_PER_BLOCK cells and rejects larger meshes;
 //  - every call looks up the array's device address (cudaGetSymbolAddress) with the caller's
 //    device current, so the address always belongs to the context the kernels run in (also
@@ -72,6 +72,13 @@ __device__ __forceinline__ long long block_max(long long v)
     return v;
 }
 
+__device__ __forceinline__ double cfl_value(double vr, double vz, double c, double sr, double sz)
+{
+    const double dt_r = 1.0 * sr / (fabs(vr) + c);
+    const double dt_z = 1.0 * sz / (fabs(vz) + c);
+    return SALEC_DTF * salec::dmin(dt_r, dt_z);
+}
+
 // CFL candidate of interior cell t (row-major over the interior, the reference's traversal
 // order), or false for a pure-vacuum cell: calculate_dt (src/sale2d.c:1999-2002)
 __device__ __forceinline__ bool cfl_cell(long long t, int nx, const double *vr, const double *vz, const double *csd,
@@ -81,30 +88,50 @@ __device__ __forceinline__ bool cfl_cell(long long t, int nx, const double *vr, 
     const int i = (int)(t % nx) + 2, j = (int)(t / nx) + 2;
     const long long p = i + (long long)pitch * j;
     if (vof0[p] > 1.0 - SALEC_TOLVOF) return false;
-    const double c = csd[p];
-    const double dt_r = 1.0 * sr[p] / (fabs(vr[p]) + c);
-    const double dt_z = 1.0 * sz[p] / (fabs(vz[p]) + c);
-    cand = SALEC_DTF * salec::dmin(dt_r, dt_z);
+    cand = cfl_value(vr[p], vz[p], csd[p], sr[p], sz[p]);
     return true;
 }
 
 // stage 1: per block, whether it saw a NaN candidate, and the MIN of its candidates after its
-// last NaN (all of them when it saw none)
+// last NaN (all of them when it saw none). CPT cells a thread, four at a time with their 24 loads in
+// flight together; the cell's column and row come from one division and are carried on. What bounds it
+// is the six planes' bandwidth, and the two launches where the mesh is small: 1021x1533 cells took
+// 38 us with one cell at a time behind two 64-bit divisions and the vacuum test, 27 now.
+template <int CPT>
 __global__ void __launch_bounds__(SALEC_CFL_THREADS)
 k_cfl_partials(int nx, int ny, const double *vr, const double *vz, const double *csd, const double *sr,
                const double *sz, const double *vof0, unsigned long long *partials, unsigned char *nanflag)
 {
-    const long long ncell = (long long)nx * ny;
-    const long long t0 = (long long)blockIdx.x * SALEC_CFL_CELLS_PER_BLOCK;
+    const int ncell = nx * ny, pitch = nx + 4;   // at most 2^25 cells (checked by the caller)
+    const int t0 = blockIdx.x * (SALEC_CFL_THREADS * CPT);
     unsigned long long best = ~0ULL;
     long long last_nan = -1;
-    for (int k = 0; k < SALEC_CFL_CELLS_PER_THREAD; ++k) {
-        const long long t = t0 + (long long)k * SALEC_CFL_THREADS + threadIdx.x;
-        if (t >= ncell) break;
-        double cand;
-        if (!cfl_cell(t, nx, vr, vz, csd, sr, sz, vof0, cand)) continue;
-        if (cand == cand) best = min(best, salec::ord_encode(cand));
-        else last_nan = t;
+    int t = t0 + threadIdx.x, j = t / nx, i = t - j * nx;
+    for (int k = 0; k < CPT; k += 4) {
+        double c[4], sr_[4], sz_[4], vr_[4], vz_[4], v0[4];
+        int tt[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            tt[u] = t;
+            if (t < ncell) {
+                const long long p = (i + 2) + (long long)pitch * (j + 2);
+                v0[u] = vof0[p]; c[u] = csd[p]; sr_[u] = sr[p]; sz_[u] = sz[p]; vr_[u] = vr[p]; vz_[u] = vz[p];
+            }
+            t += SALEC_CFL_THREADS;
+            i += SALEC_CFL_THREADS;
+            if (i >= nx) {
+                const int rows = i / nx;
+                i -= rows * nx;
+                j += rows;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (tt[u] >= ncell || v0[u] > 1.0 - SALEC_TOLVOF) continue;
+            const double cand = cfl_value(vr_[u], vz_[u], c[u], sr_[u], sz_[u]);
+            if (cand == cand) best = min(best, salec::ord_encode(cand));
+            else last_nan = tt[u];
+        }
     }
     last_nan = block_max(last_nan);
     __shared__ long long s_last;
@@ -113,8 +140,8 @@ k_cfl_partials(int nx, int ny, const double *vr, const double *vz, const double 
     last_nan = s_last;
     if (last_nan >= 0) {   // rare: recount the candidates after the block's last NaN
         best = ~0ULL;
-        for (int k = 0; k < SALEC_CFL_CELLS_PER_THREAD; ++k) {
-            const long long t = t0 + (long long)k * SALEC_CFL_THREADS + threadIdx.x;
+        for (int k = 0; k < CPT; ++k) {
+            const int t = t0 + k * SALEC_CFL_THREADS + threadIdx.x;
             if (t >= ncell) break;
             double cand;
             if (t > last_nan && cfl_cell(t, nx, vr, vz, csd, sr, sz, vof0, cand)) best = min(best, salec::ord_encode(cand));
@@ -177,10 +204,17 @@ extern "C" int salec_cfl_dt_noalloc(int nx, int ny, const double *vel_r, const d
                                                     cudaGetErrorString(le)).c_str());
     unsigned long long *partials = static_cast<unsigned long long *>(addr);
     unsigned char *nanflag = static_cast<unsigned char *>(flag_addr);
-    const int nblocks = (int)((ncell + SALEC_CFL_CELLS_PER_BLOCK - 1) / SALEC_CFL_CELLS_PER_BLOCK);
+    // four cells a thread while the partials suffice for it (8.4 million cells), sixteen beyond
+    const bool fine = ncell <= (long long)SALEC_CFL_MAX_PARTIALS * SALEC_CFL_THREADS * 4;
+    const int per_block = SALEC_CFL_THREADS * (fine ? 4 : SALEC_CFL_CELLS_PER_THREAD);
+    const int nblocks = (int)((ncell + per_block - 1) / per_block);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_cfl_partials<<<nblocks, SALEC_CFL_THREADS, 0, s>>>(nx, ny, vel_r, vel_z, csd, scale_r, scale_z, vof_vacuum,
-                                                       partials, nanflag);
+    if (fine)
+        k_cfl_partials<4><<<nblocks, SALEC_CFL_THREADS, 0, s>>>(nx, ny, vel_r, vel_z, csd, scale_r, scale_z, vof_vacuum,
+                                                               partials, nanflag);
+    else
+        k_cfl_partials<SALEC_CFL_CELLS_PER_THREAD><<<nblocks, SALEC_CFL_THREADS, 0, s>>>(
+            nx, ny, vel_r, vel_z, csd, scale_r, scale_z, vof_vacuum, partials, nanflag);
     k_cfl_final<<<1, SALEC_CFL_THREADS, 0, s>>>(nblocks, dt_prev, max_dt, partials, nanflag, dt_out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
