@@ -140,7 +140,9 @@ int salec_gpu_get_run(const salec_gpu *h, salec_run_desc *out);
 int salec_gpu_field_index(const char *name);
 /* Points in x and y and doubles per point of a field in the reference's layout. */
 int salec_gpu_field_shape(const salec_gpu *h, int field, int *nx, int *ny, int *ncomp);
-/* Copy a whole field from / to a host buffer of n doubles in the reference's layout. */
+/* Copy a whole field from / to a host buffer of n doubles in the reference's layout. Of the face
+ * records bx_phi and by_phi, a face without flow has its material volumes (zeros) only: its other
+ * members are unspecified, and nothing reads them. */
 int salec_gpu_set_field(salec_gpu *h, int field, const double *host, long long n);
 int salec_gpu_get_field(salec_gpu *h, int field, double *host, long long n);
 

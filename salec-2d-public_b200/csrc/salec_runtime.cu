@@ -327,32 +327,42 @@ int upload_axis(salec_gpu *h, const double *xs, int n, const int **bkt, int *nb,
     return upload_vec(h, v, bkt);
 }
 
-int make_edges(salec_gpu *h, Edges &g, const std::vector<std::pair<int, GatherMap>> &maps)
+// One field's gather map with its components: built once, used by every batch the field is in.
+struct FieldMap {
+    int fid;
+    GatherMap map, grouped;    // grouped and cstart: where the map's sources include destinations
+    std::vector<int> cstart;
+    bool fits = true;          // no component is too large
+    FieldMap(int f, GatherMap m) : fid(f), map(std::move(m))
+    {
+        if (map.needs_scratch) fits = group_gather_components(map, grouped, cstart);
+    }
+};
+using FieldMaps = std::vector<const FieldMap *>;
+
+int make_edges(salec_gpu *h, Edges &g, const FieldMaps &maps)
 {
     g = Edges();
     std::vector<EdgeEntry> list;
     g.nfield = (int)maps.size();
     for (int k = 0; k < g.nfield; ++k) {
-        const int fid = maps[k].first;
+        const FieldMap &fm = *maps[k];
+        const int fid = fm.fid;
         g.fid[k] = fid;
         EdgeField &f = g.batch.field[k];
         f.base = field_ptr(h, fid);
         f.f32 = field_f32(h, fid) ? 1 : 0;
         f.plane = h->d.PL;
         f.ncomp = field_ncomp(h, fid);
-        const GatherMap &m = maps[k].second;
-        GatherMap grouped;
-        std::vector<int> cstart;
-        if (m.needs_scratch) {
-            if (!group_gather_components(m, grouped, cstart)) return SALEC_OK;
-        } else {
-            for (int e = 0; e <= (int)m.dst.size(); ++e) cstart.push_back(e);
-        }
-        const GatherMap &src = m.needs_scratch ? grouped : m;
+        if (!fm.fits) return SALEC_OK;
+        const bool comp = fm.map.needs_scratch;
+        const GatherMap &src = comp ? fm.grouped : fm.map;
+        const size_t items = comp ? fm.cstart.size() - 1 : src.dst.size();
         auto pad = [&](size_t to) { while (list.size() % 32 && list.size() % 32 + to > 32) list.push_back({-1, 0, 0, k}); };
-        for (size_t c = 0; c + 1 < cstart.size(); ++c) {
-            pad(cstart[c + 1] - cstart[c]);
-            for (int e = cstart[c]; e < cstart[c + 1]; ++e) list.push_back({src.dst[e], src.src[e], src.ops[e], k});
+        for (size_t c = 0; c < items; ++c) {
+            const int e0 = comp ? fm.cstart[c] : (int)c, e1 = comp ? fm.cstart[c + 1] : (int)c + 1;
+            pad(e1 - e0);
+            for (int e = e0; e < e1; ++e) list.push_back({src.dst[e], src.src[e], src.ops[e], k});
         }
         pad(33);   // the next field starts a warp
     }
@@ -361,23 +371,20 @@ int make_edges(salec_gpu *h, Edges &g, const std::vector<std::pair<int, GatherMa
     return upload_vec(h, list, &g.batch.entries);
 }
 
-int make_gather(salec_gpu *h, Gather &g, const std::vector<std::pair<int, GatherMap>> &maps)
+int make_gather(salec_gpu *h, Gather &g, const FieldMaps &maps)
 {
     g = Gather();
     g.batch.nfield = (int)maps.size();
     int total = 0;
-    for (size_t k = 0; k < maps.size(); ++k) g.ncomp_max = std::max(g.ncomp_max, field_ncomp(h, maps[k].first));
+    for (size_t k = 0; k < maps.size(); ++k) g.ncomp_max = std::max(g.ncomp_max, field_ncomp(h, maps[k]->fid));
     // maps whose sources include destinations run as components in the same single launch;
     // only when a component is too large does the batch fall back to two passes through scratch
-    std::vector<GatherMap> grouped(maps.size());
-    std::vector<std::vector<int>> cstart(maps.size());
-    for (size_t k = 0; k < maps.size() && !g.two_pass; ++k)
-        if (maps[k].second.needs_scratch && !group_gather_components(maps[k].second, grouped[k], cstart[k]))
-            g.two_pass = true;
+    for (const FieldMap *m : maps) g.two_pass = g.two_pass || !m->fits;
     for (size_t k = 0; k < maps.size(); ++k) {
-        const int fid = maps[k].first;
-        const bool comp = !g.two_pass && maps[k].second.needs_scratch;
-        const GatherMap &m = comp ? grouped[k] : maps[k].second;
+        const int fid = maps[k]->fid;
+        const bool comp = !g.two_pass && maps[k]->map.needs_scratch;
+        const GatherMap &m = comp ? maps[k]->grouped : maps[k]->map;
+        const std::vector<int> &cstart = maps[k]->cstart;
         GatherField &gf = g.batch.field[k];
         gf.base = field_ptr(h, fid);
         gf.f32 = field_f32(h, fid) ? 1 : 0;
@@ -391,11 +398,11 @@ int make_gather(salec_gpu *h, Gather &g, const std::vector<std::pair<int, Gather
         if (rc) return rc;
         rc = upload_vec(h, m.ops, &gf.ops);
         if (rc) return rc;
-        if (comp && (rc = upload_vec(h, cstart[k], &gf.cstart))) return rc;
+        if (comp && (rc = upload_vec(h, cstart, &gf.cstart))) return rc;
         g.batch.start[k] = total;
         g.entries[k] = (int)m.dst.size();
         g.fid[k] = fid;
-        total += comp ? (int)cstart[k].size() - 1 : (int)m.dst.size();
+        total += comp ? (int)cstart.size() - 1 : (int)m.dst.size();
     }
     g.batch.start[maps.size()] = total;
     g.batch.total = total;
@@ -542,8 +549,12 @@ void allocate_donor_copy(salec_gpu *h)
 {
     h->alt = h->f;
     if (h->rp.damp_type == SALEC_DAMP_PML3) return;
-    size_t bytes = 0;
+    size_t bytes = 0, free_bytes = 0, total_bytes = 0;
     for (int k : donor_fields(h)) bytes += (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k);
+    // large meshes leave room for what comes after (staging, geometry tables, tracers)
+    if (bytes > ((size_t)64 << 20) && (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess ||
+                                       free_bytes < bytes + h->pool_bytes / 4 + ((size_t)512 << 20)))
+        return;
     if (cudaMalloc(&h->alt_pool, bytes) != cudaSuccess) {
         cudaGetLastError();
         h->alt_pool = nullptr;
@@ -604,6 +615,27 @@ void destroy_cycle_graphs(salec_gpu *h)
     }
 }
 
+// The second copy of the donor state only makes cycles faster: it is given up where the device runs out
+// of memory for something a caller asked for. False when there is nothing to give up.
+bool release_donor_copy(salec_gpu *h)
+{
+    cudaGetLastError();
+    if (!h->alt_pool || settle(h) != SALEC_OK || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+    destroy_cycle_graphs(h);
+    cudaFree(h->alt_pool);
+    if (h->quiet_map) cudaFree(h->quiet_map);
+    h->alt_pool = nullptr;
+    h->quiet_map = nullptr;
+    h->alt = h->f;
+    return true;
+}
+
+cudaError_t device_malloc(salec_gpu *h, void **p, size_t n)
+{
+    const cudaError_t e = cudaMalloc(p, n);
+    return e == cudaErrorMemoryAllocation && release_donor_copy(h) ? cudaMalloc(p, n) : e;
+}
+
 // The whole cycle as the cycle graph holds it: the phases in order, with the energy update inside
 // the stress sweep, the tracers in the flux launch and, with a second copy of the donor state, face
 // volumes instead of records and the remap from one copy into the other.
@@ -653,39 +685,43 @@ int run_cycle(salec_gpu *h) { return h->mixed ? run_cycle_t<float>(h) : run_cycl
 int build_gathers(salec_gpu *h)
 {
     const Dims &d = h->d;
+    std::map<std::string, FieldMap> built;   // each field has one ghost pattern, the vertex fields one restriction
+    auto add = [&](const char *name, auto make) -> const FieldMap * {
+        auto it = built.find(name);
+        if (it == built.end()) {
+            const int fid = field_by_name(name);
+            it = built.emplace(name, FieldMap(fid, make(field_ncomp(h, fid)))).first;
+        }
+        return &it->second;
+    };
     auto gm = [&](const char *name, GhostPattern pat) {
-        int fid = field_by_name(name);
-        return std::make_pair(fid, build_ghost_map(d.enx, d.eny, d.P, field_ncomp(h, fid), h->go, pat));
+        return add(name, [&](int nc) { return build_ghost_map(d.enx, d.eny, d.P, nc, h->go, pat); });
     };
     auto rm = [&](const char *name) {
-        int fid = field_by_name(name);
-        return std::make_pair(fid, build_restrict_map(d.vnx, d.vny, d.P, field_ncomp(h, fid), h->go));
+        return add(name, [&](int nc) { return build_restrict_map(d.vnx, d.vny, d.P, nc, h->go); });
     };
+    const FieldMap *mvof = gm("m_vof", GP_ALWAYS_COPY), *dvel = gm("e_dvel", GP_VELOCITY_INC), *den = gm("e_den", GP_DENSITY),
+                   *pre = gm("e_pre", GP_ALWAYS_COPY), *ste = gm("e_ste", GP_STRESS), *mden = gm("m_den", GP_DENSITY),
+                   *vib = gm("e_vib", GP_ALWAYS_COPY), *meng = gm("m_eng", GP_DENSITY), *pty = gm("m_pty", GP_ALWAYS_COPY),
+                   *cvs = gm("e_cvs", GP_ALWAYS_COPY), *dis = rm("v_dis");
     int rc;
-    if ((rc = make_gather(h, h->g_mvof, {gm("m_vof", GP_ALWAYS_COPY)}))) return rc;
-    if ((rc = make_gather(h, h->g_dvel_den, {gm("e_dvel", GP_VELOCITY_INC), gm("e_den", GP_DENSITY)}))) return rc;
+    if ((rc = make_gather(h, h->g_mvof, {mvof}))) return rc;
+    if ((rc = make_gather(h, h->g_dvel_den, {dvel, den}))) return rc;
+    if ((rc = make_edges(h, h->e_head, {mvof, dvel, den}))) return rc;
     if ((rc = make_gather(h, h->g_evel, {gm("e_vel", GP_VELOCITY)}))) return rc;
-    if ((rc = make_gather(h, h->g_pre_ste_q,
-                          {gm("e_pre", GP_ALWAYS_COPY), gm("e_ste", GP_STRESS), gm("e_q", GP_ALWAYS_COPY)})))
-        return rc;
-    if ((rc = make_edges(h, h->e_head, {gm("m_vof", GP_ALWAYS_COPY), gm("e_dvel", GP_VELOCITY_INC), gm("e_den", GP_DENSITY)})))
-        return rc;
-    std::vector<std::pair<int, GatherMap>> fs = {gm("m_den", GP_DENSITY), gm("e_vib", GP_ALWAYS_COPY),
-                                                 gm("m_eng", GP_DENSITY)};
+    if ((rc = make_gather(h, h->g_pre_ste_q, {pre, ste, gm("e_q", GP_ALWAYS_COPY)}))) return rc;
+    FieldMaps fs = {mden, vib, meng};
     if (h->rp.porosity_model) {
-        fs.push_back(gm("m_pty", GP_ALWAYS_COPY));
-        fs.push_back(gm("e_cvs", GP_ALWAYS_COPY));
+        fs.push_back(pty);
+        fs.push_back(cvs);
     }
     if ((rc = make_gather(h, h->g_flux_state, fs))) return rc;
-    fs.insert(fs.begin(), rm("v_dis"));
+    fs.insert(fs.begin(), dis);
     if ((rc = make_edges(h, h->e_tail, fs))) return rc;
-    if ((rc = make_gather(h, h->g_init,
-                          {gm("e_den", GP_DENSITY), gm("e_pre", GP_ALWAYS_COPY), gm("e_ste", GP_STRESS),
-                           gm("m_eng", GP_DENSITY), gm("m_pty", GP_ALWAYS_COPY), gm("e_cvs", GP_ALWAYS_COPY)})))
-        return rc;
+    if ((rc = make_gather(h, h->g_init, {den, pre, ste, meng, pty, cvs}))) return rc;
     if ((rc = make_gather(h, h->r_vel, {rm("v_vel")}))) return rc;
     if ((rc = make_gather(h, h->r_acc, {rm("v_acc")}))) return rc;
-    if ((rc = make_gather(h, h->r_dis, {rm("v_dis")}))) return rc;
+    if ((rc = make_gather(h, h->r_dis, {dis}))) return rc;
     if (h->scratch_doubles) {
         void *p = nullptr;
         CUDA_TRY(cudaMalloc(&p, h->scratch_doubles * sizeof(double)));
@@ -912,7 +948,10 @@ int ensure_staging(salec_gpu *h, size_t need)
     if (h->staging) CUDA_TRY(cudaFreeAsync(h->staging, h->stream));
     h->staging = nullptr;
     h->staging_doubles = 0;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&h->staging), need * sizeof(double), h->stream));
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&h->staging), need * sizeof(double), h->stream);
+    if (e == cudaErrorMemoryAllocation && release_donor_copy(h))
+        e = cudaMallocAsync(reinterpret_cast<void **>(&h->staging), need * sizeof(double), h->stream);
+    CUDA_TRY(e);
     h->staging_doubles = need;
     return SALEC_OK;
 }
@@ -1156,15 +1195,6 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     }
 
     {
-        // the cycle graph's surface-profile minima, as the last kernel of a cycle leaves them
-        std::vector<unsigned long long> acc(d.enx, ord_encode(rp.threshold_z * 2.0));
-        const unsigned long long *dev = nullptr;
-        if (int rc = upload_vec(h, acc, &dev)) return bail(rc);
-        if (int rc = flush_uploads(h)) return bail(rc);
-        h->profile_acc = const_cast<unsigned long long *>(dev);
-    }
-    allocate_donor_copy(h);
-    {
         const size_t words = (size_t)(d.P / 32) * d.R;
         if (cudaMalloc(&h->lap_mask, words * sizeof(unsigned)) != cudaSuccess)
             return bail(fail(SALEC_ERR_ALLOC, "Laplacian mask"));
@@ -1212,7 +1242,13 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
 
     int rc = build_gathers(h);
     if (rc) return bail(rc);
+    // the cycle graph's surface-profile minima, as the last kernel of a cycle leaves them
+    const std::vector<unsigned long long> acc(d.enx, ord_encode(rp.threshold_z * 2.0));
+    const unsigned long long *acc_dev = nullptr;
+    if ((rc = upload_vec(h, acc, &acc_dev))) return bail(rc);
     if ((rc = flush_uploads(h))) return bail(rc);
+    h->profile_acc = const_cast<unsigned long long *>(acc_dev);
+    allocate_donor_copy(h);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(SALEC_ERR_CUDA, "create sync"));
     *out = h;
     return SALEC_OK;
@@ -1519,7 +1555,7 @@ int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
     void *snap = nullptr, *snap_tr = nullptr;
     Scal scal_host{};
     CUDA_TRY(cudaMemcpy(&scal_host, h->scal, sizeof(Scal), cudaMemcpyDeviceToHost));
-    if (cudaMalloc(&snap, h->pool_bytes) != cudaSuccess) return fail(SALEC_ERR_ALLOC, "autotune snapshot");
+    if (device_malloc(h, &snap, h->pool_bytes) != cudaSuccess) return fail(SALEC_ERR_ALLOC, "autotune snapshot");
     if (h->tr_bytes && cudaMalloc(&snap_tr, h->tr_bytes) != cudaSuccess) {
         cudaFree(snap);
         return fail(SALEC_ERR_ALLOC, "autotune snapshot");
@@ -1919,7 +1955,7 @@ int adjoint_ensure(salec_gpu *h)
     if (!h->adj) h->adj = new AdjointState();
     AdjointState *st = h->adj;
     if (!st->pool) {
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->pool), h->pool_bytes));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->pool), h->pool_bytes));
         CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->theta), 4 * sizeof(double)));
         for (int k = 0; k < kNumFields; ++k) {
             const size_t off = reinterpret_cast<char *>(field_ptr(h, k)) - h->pool;
@@ -1939,9 +1975,9 @@ int adjoint_ensure(salec_gpu *h)
         for (int p = 0; p < 16; ++p) tb = std::max(tb, list_bytes(h, kAdjWrites[p]));
         for (const auto *l : {&kKeep12, &kKeep8, &kKeep1}) tb = std::max(tb, list_bytes(h, *l));
         st->tmp_bytes = tb;
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->tmp), tb));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->tmp), tb));
         CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->slot), sizeof(long long)));
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->cscr), 16 * (size_t)h->d.PL * sizeof(double)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->cscr), 16 * (size_t)h->d.PL * sizeof(double)));
         // every list table, so that the graphs can be captured
         const std::vector<const char *> snap(std::begin(kAdjSnapshot), std::end(kAdjSnapshot));
         std::vector<const std::vector<const char *> *> all = {&snap, &kKeep12, &kKeep8, &kKeep1};
@@ -2035,6 +2071,7 @@ int adjoint_phase(salec_gpu *h, int p)
 
 int adjoint_transfer(salec_gpu *h, int fid, double *host, long long n, bool to_device)
 {
+    if (int rc = settle(h)) return rc;   // the adjoint planes are addressed by the pool's own layout
     double *&slot = field_ptr(h, fid);
     double *saved = slot;
     slot = reinterpret_cast<double *>(h->adj->pool + (reinterpret_cast<char *>(saved) - h->pool));
@@ -2252,14 +2289,14 @@ int salec_gpu_adjoint_window(salec_gpu *h, int nsteps, int every, const double *
         cudaFree(st->ckpt);
         st->ckpt = nullptr;
         st->ckpt_bytes = 0;
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->ckpt), need_ck));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->ckpt), need_ck));
         st->ckpt_bytes = need_ck;
     }
     if (st->undo_bytes < need_ud) {
         cudaFree(st->undo);
         st->undo = nullptr;
         st->undo_bytes = 0;
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->undo), need_ud));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->undo), need_ud));
         st->undo_bytes = need_ud;
     }
     const size_t md = 1 + 3 * (size_t)ncols;

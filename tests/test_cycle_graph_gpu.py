@@ -82,3 +82,19 @@ def test_cycle_graph_equals_the_phases(cuda_device, tmp_path, kind, precision):
     _same(_state(graph), _state(phases), "after the body")
     graph.close()
     phases.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cycles", [1, 2])
+def test_adjoint_fields_after_graph_cycles(cuda_device, tmp_path, cycles):
+    """An adjoint field read after forward cycles is the one that was set: the forward donor state may
+    then live in its second copy, the adjoint planes have one place."""
+    deck = decks.config5_deck(64, velocity=1000.0, cppr=8.0)
+    sim = capi.Simulation.from_deck(decks.write_deck(deck, str(tmp_path)), str(tmp_path))
+    sim.adjoint_reset()
+    bar = np.random.default_rng(3).standard_normal(sim.shape("m_den"))
+    sim.step(cycles)
+    sim.adjoint_set("m_den", bar)
+    sim.step(cycles)
+    assert np.array_equal(sim.adjoint_get("m_den"), bar)
+    sim.close()
