@@ -508,7 +508,7 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
     grid_dependency();
     using A = R;   // arithmetic of the gradient and the viscosity: FP64, or FP32 in the mixed form
     unsigned long long cand = ~0ULL;
-    for_points<true>(c, 0, [&](int i, int j) {
+    for_points<VOID>(c, 0, [&](int i, int j) {
     if (VOID && vert_active(c, i, j)) {
         const long long p = KIDX(i, j);
         double x, y;
