@@ -110,8 +110,8 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
 template <class R>
 void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 blk, int a0 = 0, int a1 = 0,
                         int a2 = 0, int a3 = 0);
-void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
-                         cudaStream_t s);
+void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list0, int *count0,
+                         int *list1, int *count1, cudaStream_t s);
 void launch_report(const Scal *scal, const double *profile, int n, Report *out, unsigned ticket, cudaStream_t s);
 __global__ void k_gather(GatherBatch g, int mode, double *scratch);
 __global__ void k_edges(const __grid_constant__ EdgeBatch g);

@@ -188,7 +188,8 @@ struct salec_gpu {
     // quiet map (CtxT): vacuum[], quiet[], and per flip a tile list with its count. Null where the
     // map is not used.
     unsigned char *quiet_map = nullptr;
-    bool quiet_known = true;     // the map may hold quiet tiles: a graph cycle has run since it was forgotten
+    bool quiet_known = true;     // a graph cycle has run since the map was forgotten: false means that
+                                 // both lists hold every tile
     bool in_graph = false;       // the cycle graph is being captured: its kernels take the quiet map
     bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
@@ -534,7 +535,7 @@ int forget_quiet(salec_gpu *h)
     if (!h->quiet_map || !h->quiet_known) return SALEC_OK;
     h->quiet_known = false;
     launch_forget_quiet(h->quiet_map, h->tiles() * SALEC_TILE_ROWS, h->quiet_map + h->segment_bytes(), h->tiles_x(),
-                        h->tiles_y(), h->tile_list(h->flip), h->tile_count(h->flip), h->stream);
+                        h->tiles_y(), h->tile_list(0), h->tile_count(0), h->tile_list(1), h->tile_count(1), h->stream);
     CUDA_TRY(cudaGetLastError());
     return SALEC_OK;
 }
@@ -1091,6 +1092,18 @@ Dims salec_internal_dims(salec_gpu *h) { return h->d; }
 void salec_internal_add_launches(salec_gpu *h, int n) { h->launches += n; }
 void *&salec_internal_output_slot(salec_gpu *h) { return h->output; }
 void *&salec_internal_conserve_slot(salec_gpu *h) { return h->conserve; }
+
+// The tiles that the next graph cycle visits and the mesh's tiles, for tests of the quiet map: 0 and 0
+// where the handle has none.
+extern "C" int salec_internal_listed_tiles(salec_gpu *h, int *listed, int *total)
+{
+    *listed = *total = 0;
+    if (!h->quiet_map) return SALEC_OK;
+    *total = h->tiles();
+    CUDA_TRY(cudaMemcpyAsync(listed, h->tile_count(h->flip), sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return SALEC_OK;
+}
 
 // ================================================================== C ABI
 extern "C" {

@@ -258,22 +258,24 @@ __device__ __forceinline__ void count_quiet(const C &c, int t)
     if (active) c.next_list[base + __popc(who & ((1u << (threadIdx.x & 31)) - 1u))] = ti | tj << 16;
 }
 
-// Nothing is known to be quiet: every tile is listed.
-__global__ void k_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count)
+// Nothing is known to be quiet: every tile is listed, in both lists, as the handle may still turn to the
+// other copy of the donor state (and with it to the other list) before its next cycle.
+__global__ void k_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list0, int *count0,
+                               int *list1, int *count1)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < segments) vacuum[t] = 0;
     if (t < tx * ty) {
         quiet[t] = 0;
-        list[t] = (t % tx) | (t / tx) << 16;
+        list0[t] = list1[t] = (t % tx) | (t / tx) << 16;
     }
-    if (t == 0) *count = tx * ty;
+    if (t == 0) *count0 = *count1 = tx * ty;
 }
 
-void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list, int *count,
-                         cudaStream_t s)
+void launch_forget_quiet(unsigned char *vacuum, int segments, unsigned char *quiet, int tx, int ty, int *list0, int *count0,
+                         int *list1, int *count1, cudaStream_t s)
 {
-    k_forget_quiet<<<(segments + 255) / 256, 256, 0, s>>>(vacuum, segments, quiet, tx, ty, list, count);
+    k_forget_quiet<<<(segments + 255) / 256, 256, 0, s>>>(vacuum, segments, quiet, tx, ty, list0, count0, list1, count1);
 }
 
 // ============================================================ phase 0: surface profile
