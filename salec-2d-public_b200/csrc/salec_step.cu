@@ -226,11 +226,24 @@ __device__ __forceinline__ void for_points(const C &c, int lead, F f)
 // no volume, cells keep m_vof = (1, 0, ...) and zeros. The earlier of these cycles stored the
 // constants, in both copies of the donor state, so the sweeps are not run there: the cycle graph
 // visits the listed tiles only. PML2 and PML3 accelerate vacuum vertices by gravity and take no part.
+// The one dt that matters is one whose square is not finite, as 0 * dt is NaN then: it lists every tile for
+// the rest of its own cycle (list_all_tiles) and the count starts again after it.
 // The map is forgotten whenever a field is written from outside or the phases run one by one. About
 // half of an impact's mesh lies above its target. Leaving quiet tiles out took
 // the 2048x2048 impact from 1214 to 963 us a cycle and the 1024x1024 one from 399 to 338 (returning
 // early from quiet row segments inside full grids: 1000 and 340).
 #define SALEC_QUIET_CYCLES 4
+
+__device__ __forceinline__ bool leaves_vacuum_alone(double dt) { return 0.0 * (0.5 * dt * dt) == 0.0; }
+
+// Every tile into the list of this cycle, by n threads of which this is number t.
+template <class C>
+__device__ __forceinline__ void list_all_tiles(const C &c, int t, int n)
+{
+    int *list = const_cast<int *>(c.tile_list);
+    for (int k = t; k < c.tx * c.ty; k += n) list[k] = (k % c.tx) | (k / c.tx) << 16;
+    if (t == 0) *const_cast<int *>(c.tile_count) = c.tx * c.ty;
+}
 
 // The map and the list of the next cycle, one thread per tile, after the remap has set vacuum[].
 template <class C>
@@ -240,7 +253,8 @@ __device__ __forceinline__ void count_quiet(const C &c, int t)
     const bool tile = t < S * c.ty;
     bool active = false;
     if (tile) {
-        bool all = tj >= 1 && tj < c.ty - 1 && ti >= 1 && ti < S - 1 && j0 + SALEC_TILE_ROWS + 2 <= c.d.R;
+        bool all = tj >= 1 && tj < c.ty - 1 && ti >= 1 && ti < S - 1 && j0 + SALEC_TILE_ROWS + 2 <= c.d.R &&
+                   leaves_vacuum_alone(c.scal->dt);
         if (all) {
             const unsigned char *v = c.vacuum + (long long)S * (j0 - 2) + ti;
 #pragma unroll
@@ -603,16 +617,21 @@ __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const Ct
     if (c.profile)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c.d.enx; i += gridDim.x * blockDim.x)
             c.f.y_profile[i] = ord_decode(c.profile[i]);
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+    auto take = [&](double dt) {
+        if (thread == 0) c.scal->dt = dt;
+        if (c.tile_list && !leaves_vacuum_alone(dt)) list_all_tiles(c, thread, gridDim.x * blockDim.x);
+    };
     if (c.dt_sched) {
         const long long k = c.scal->i_step - c.dt_sched_i0;
         if (k >= 0 && k < c.dt_sched_n) {
-            if (threadIdx.x == 0 && blockIdx.x == 0) c.scal->dt = c.dt_sched[k];
+            take(c.dt_sched[k]);
             return;
         }
     }
     const long long last = c.scal->dt_nan_last;
     if (last < 0) {
-        if (threadIdx.x == 0 && blockIdx.x == 0) c.scal->dt = step_dt(c);
+        take(step_dt(c));
         return;
     }
     const int nx = c.d.enx - 4;
@@ -628,8 +647,10 @@ __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const Ct
     __shared__ unsigned long long wmin[SALEC_FINALIZE_THREADS / 32];
     for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
     if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = best;
+    __shared__ bool all_tiles;
     __syncthreads();
     if (threadIdx.x == 0) {
+        all_tiles = false;
         for (int w = 1; w < SALEC_FINALIZE_THREADS / 32; ++w) best = min(best, wmin[w]);
         if (best != ~0ULL) atomicMin(&c.scal->dt_tail, best);
         __threadfence();
@@ -637,11 +658,15 @@ __global__ void __launch_bounds__(SALEC_FINALIZE_THREADS) k_finalize_dt(const Ct
             __threadfence();
             const unsigned long long tail = atomicMin(&c.scal->dt_tail, ~0ULL);
             const double r = tail == ~0ULL ? __longlong_as_double(0x7ff8000000000000LL) : ord_decode(tail);
-            c.scal->dt = dmin(c.rp.max_dt, r);
+            const double dt = dmin(c.rp.max_dt, r);
+            c.scal->dt = dt;
             c.scal->dt_tail = ~0ULL;
             c.scal->dt_tail_blocks = 0u;
+            all_tiles = !leaves_vacuum_alone(dt);
         }
     }
+    __syncthreads();
+    if (all_tiles && c.tile_list) list_all_tiles(c, threadIdx.x, blockDim.x);
 }
 
 // ============================================================ phase 7: vibration, stress, damage

@@ -74,3 +74,24 @@ def test_a_write_after_odd_cycles_reaches_every_tile(cuda_device, tmp_path, betw
         _same(_state(graph), _state(phases), "after %d more cycles" % n)
     graph.close()
     phases.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", [float("nan"), float("inf"), 1.0e200])
+def test_a_time_step_beyond_bounds_reaches_every_tile(cuda_device, tmp_path, dt):
+    """0 * dt is NaN for such a time step, in vacuum too: what it leaves behind is the phase-by-phase
+    path's, in the cycle itself and in those after it (whose CFL steps are then recounted)."""
+    path = decks.write_deck(_deck("nothing"), str(tmp_path))
+    graph, phases = (capi.Simulation.from_deck(path, str(tmp_path)) for _ in range(2))
+    graph.step(40)
+    _phases(phases, 40)
+    listed, total = _tiles(graph)
+    assert 0 < listed < total
+    for sim in (graph, phases):
+        sim.set_dt_schedule([1.0e-3, dt])
+    for n in (2, 1, 1, 5):
+        graph.step(n)
+        _phases(phases, n)
+        _same(_state(graph), _state(phases), "after %d more cycles" % n)
+    graph.close()
+    phases.close()
