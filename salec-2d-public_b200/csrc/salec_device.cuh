@@ -87,7 +87,10 @@ struct Scal {
     // candidates after it and the count of finished blocks of that recount
     long long dt_nan_last;
     unsigned long long dt_tail;
-    unsigned int dt_tail_blocks, pad_;
+    unsigned int dt_tail_blocks;
+    // cycle graph: the material fractions of this cycle, and those its remap left for the next, may hold
+    // a NaN or a negative one (see remap_cell)
+    unsigned int odd_fractions, odd_next, pad_;
 };
 
 // Page-locked record that k_report fills: the scalars, the ticket of the report they belong to, and

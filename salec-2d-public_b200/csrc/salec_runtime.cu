@@ -190,6 +190,7 @@ struct salec_gpu {
     unsigned char *quiet_map = nullptr;
     bool quiet_known = true;     // a graph cycle has run since the map was forgotten: false means that
                                  // both lists hold every tile
+    bool fractions_known = false;   // Scal::odd_fractions is what the last graph cycle left
     bool in_graph = false;       // the cycle graph is being captured: its kernels take the quiet map
     bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
@@ -529,9 +530,10 @@ double *&alt_ptr(salec_gpu *h, int k)
     return *reinterpret_cast<double **>(reinterpret_cast<char *>(&h->alt) + kFields[k].off);
 }
 
-// Something other than a graph cycle changes the fields: nothing is known to be quiet.
+// Something other than a graph cycle changes the fields: nothing is known to be quiet, or of the fractions.
 int forget_quiet(salec_gpu *h)
 {
+    h->fractions_known = false;
     if (!h->quiet_map || !h->quiet_known) return SALEC_OK;
     h->quiet_known = false;
     launch_forget_quiet(h->quiet_map, h->tiles() * SALEC_TILE_ROWS, h->quiet_map + h->segment_bytes(), h->tiles_x(),
@@ -1382,6 +1384,10 @@ int salec_gpu_step(salec_gpu *h, int nsteps)
     for (int k = 0; k < nsteps; ++k) {
         if (!h->profiling && !h->cycle_graph[h->flip]) capture_cycle_graph(h);
         if (!h->profiling && h->cycle_graph[h->flip]) {
+            if (!h->fractions_known) {
+                CUDA_TRY(cudaMemsetAsync(&h->scal->odd_fractions, 1, sizeof(unsigned), h->stream));
+                h->fractions_known = true;
+            }
             CUDA_TRY(cudaGraphLaunch(h->cycle_graph[h->flip], h->stream));
             h->launches += h->cycle_graph_launches[h->flip];
             if (h->alt_pool) {
