@@ -475,8 +475,9 @@ __global__ void k_cell_velocity(const CtxT<R> c)
 // ============================================================ phase 4: void vertices
 // check_v_vel (src/sale2d.c:1051-1142): a vertex whose four corners are all void takes the
 // density-weighted velocity of its non-empty cells.
-// corners: the vertex's count of void corners (v_mass[1], set by the momentum sweep from the same
-// e_wpt). True where the vertex takes the velocity (vx, vy).
+// corners: the vertex's count of void corners. The momentum sweep leaves it in v_mass[1], which the cycle
+// graph takes it from; a phase 4 that runs by itself counts again, as the state may be a caller's.
+// True where the vertex takes the velocity (vx, vy).
 template <class C>
 __device__ __forceinline__ bool void_velocity(const C &c, int i, int j, double corners, double &vx, double &vy)
 {
@@ -504,9 +505,13 @@ __global__ void k_void_vertices(const CtxT<R> c)
     grid_dependency();
     GRID_POINT(i, j);
     if (!vert_active(c, i, j)) return;
-    const long long p = KIDX(i, j);
+    const long long p = KIDX(i, j), cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
+    const int corner[4] = {2, 3, 0, 1};
+    int void_corner = 0;
+    for (int k = 0; k < 4; ++k)
+        if (PLN(c.f.e_wpt, corner[k])[cl[k]] > 0.) void_corner++;
     double vx, vy;
-    if (!void_velocity(c, i, j, PLN(c.f.v_mass, 1)[p], vx, vy)) return;
+    if (!void_velocity(c, i, j, void_corner, vx, vy)) return;
     c.f.v_vel[p] = vx;
     PLN(c.f.v_vel, 1)[p] = vy;
 }
