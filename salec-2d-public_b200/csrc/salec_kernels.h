@@ -54,6 +54,22 @@ struct EdgeBatch {
     int total;
 };
 
+// A tile of the cycle graph's list is its column and row in one int (tile_pack); a mesh of more columns or
+// rows of tiles than fit (2,097,120 points in x, 262,136 in y) has no list and is swept whole.
+inline bool tiles_fit_a_list(int tx, int ty) { return tx <= 0xffff && ty <= 0x7fff; }
+#ifdef __CUDACC__
+#define SALEC_HD __host__ __device__
+#else
+#define SALEC_HD
+#endif
+SALEC_HD inline int tile_pack(int ti, int tj) { return ti | tj << 16; }
+SALEC_HD inline int tile_column(int e) { return e & 0xffff; }
+SALEC_HD inline int tile_row(int e) { return e >> 16; }
+// Rows of blocks of a two-dimensional sweep over `points` rows of points, and whether `lead` more can go in
+// front of them in the same grid (a grid has at most 65535 rows).
+inline int sweep_block_rows(int points, int rows) { return (points + rows - 1) / rows; }
+inline bool lead_fits(int block_rows, int lead) { return (long long)block_rows + lead <= 65535; }
+
 // Host-side gather map of one field: entries in increasing destination order.
 struct GatherMap {
     std::vector<int> dst, src;

@@ -573,7 +573,9 @@ void allocate_donor_copy(salec_gpu *h)
     // The quiet map needs a cycle whose vacuum is the same whatever the time step (count_quiet). Small
     // meshes fill the device for a moment only, whatever they visit, and looking the tile up costs
     // them more than it saves (64x80: 81 us a cycle without, 86 with; 517x771: 194 and 184).
-    if (h->rp.damp_type == SALEC_DAMP_PML2 || (long long)h->d.enx * h->d.eny < SALEC_QUIET_MIN_CELLS) return;
+    if (h->rp.damp_type == SALEC_DAMP_PML2 || (long long)h->d.enx * h->d.eny < SALEC_QUIET_MIN_CELLS ||
+        !tiles_fit_a_list(h->tiles_x(), h->tiles_y()))
+        return;
     if (cudaMalloc(reinterpret_cast<void **>(&h->quiet_map), h->quiet_bytes()) != cudaSuccess) {
         cudaGetLastError();
         h->quiet_map = nullptr;

@@ -206,8 +206,8 @@ __device__ __forceinline__ void for_points(const C &c, int lead, F f)
         int e_next = 0, i, j;
         if (listed) {
             if (WALK && next < n) e_next = c.tile_list[next >> sh];
-            i = 32 * (e & 0xffff) + threadIdx.x;
-            j = (((e >> 16) << sh) + (b & ((1 << sh) - 1))) * blockDim.y + threadIdx.y;
+            i = 32 * tile_column(e) + threadIdx.x;
+            j = ((tile_row(e) << sh) + (b & ((1 << sh) - 1))) * blockDim.y + threadIdx.y;
         } else {
             i = 32 * b + threadIdx.x;
             j = (blockIdx.y - lead) * blockDim.y + threadIdx.y;
@@ -241,7 +241,7 @@ template <class C>
 __device__ __forceinline__ void list_all_tiles(const C &c, int t, int n)
 {
     int *list = const_cast<int *>(c.tile_list);
-    for (int k = t; k < c.tx * c.ty; k += n) list[k] = (k % c.tx) | (k / c.tx) << 16;
+    for (int k = t; k < c.tx * c.ty; k += n) list[k] = tile_pack(k % c.tx, k / c.tx);
     if (t == 0) *const_cast<int *>(c.tile_count) = c.tx * c.ty;
 }
 
@@ -269,7 +269,7 @@ __device__ __forceinline__ void count_quiet(const C &c, int t)
     int base = 0;
     if ((threadIdx.x & 31) == 0 && who) base = atomicAdd(c.next_count, __popc(who));
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (active) c.next_list[base + __popc(who & ((1u << (threadIdx.x & 31)) - 1u))] = ti | tj << 16;
+    if (active) c.next_list[base + __popc(who & ((1u << (threadIdx.x & 31)) - 1u))] = tile_pack(ti, tj);
 }
 
 // Nothing is known to be quiet: every tile is listed, in both lists, as the handle may still turn to the
@@ -281,7 +281,7 @@ __global__ void k_forget_quiet(unsigned char *vacuum, int segments, unsigned cha
     if (t < segments) vacuum[t] = 0;
     if (t < tx * ty) {
         quiet[t] = 0;
-        list0[t] = list1[t] = (t % tx) | (t / tx) << 16;
+        list0[t] = list1[t] = tile_pack(t % tx, t / tx);
     }
     if (t == 0) *count0 = *count1 = tx * ty;
 }
@@ -2347,19 +2347,20 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 sha
     // a block shape stands for its thread count: rows of 32 points, a power of two of them (for_points)
     int rows = 1;
     while (2 * rows <= SALEC_TILE_ROWS && 64 * rows <= (int)(shape.x * shape.y)) rows *= 2;
-    const dim3 b(32, rows), g(c.tx, c.ty * (SALEC_TILE_ROWS / rows));
+    const dim3 b(32, rows), g(c.tx, sweep_block_rows(c.d.R, rows));
+    const int listed = c.tx * c.ty * (SALEC_TILE_ROWS / rows);   // blocks of a whole list
     const int ncol = (c.d.enx + 255) / 256;
     // a sweep over points: the whole two-dimensional grid, or the walkers of a tile list (for_points)
     int lead = 0;
     bool walk = false;
     auto points = [&](auto kernel, auto... args) {
         dim3 grid(g.x, g.y + lead);
-        if (c.tile_list && !walk) grid = dim3(lead + g.x * g.y);
+        if (c.tile_list && !walk) grid = dim3(lead + listed);
         if (c.tile_list && walk) {
             int dev = 0, sms = 0, per_sm = 0;
             if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)(b.x * b.y), 0);
-            grid = dim3(lead + max(1, min((int)(g.x * g.y), sms * per_sm)));
+            grid = dim3(lead + max(1, min(listed, sms * per_sm)));
         }
         launch_dependent(kernel, grid, b, s, args...);
     };
@@ -2388,6 +2389,10 @@ void launch_step_kernel(StepKernel k, const CtxT<R> &c, cudaStream_t s, dim3 sha
     case SK_FLUX: {
         const int per = 32 * rows * (c.tile_list ? 1 : (int)g.x);   // tracers of a leading block, or row of blocks
         lead = a0 && c.tr.n > 0 ? (c.tr.n + per - 1) / per : 0;
+        if (lead && !c.tile_list && !lead_fits(g.y, lead)) {   // a very tall mesh: a launch of their own
+            launch_dependent(k_tracers<R>, (c.tr.n + 127) / 128, 128, s, c);
+            lead = 0;
+        }
         if (a1) SALEC_NM_DISPATCH_P3(k_flux, (false), c, lead);
         else SALEC_NM_DISPATCH(k_flux, c, lead);
         break;
