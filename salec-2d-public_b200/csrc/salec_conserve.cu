@@ -19,11 +19,14 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 
 using namespace salec;
 
 int salec_internal_fail(int code, const char *msg);
+int salec_internal_malloc(salec_gpu *h, void **p, size_t n);
+std::unique_lock<std::recursive_mutex> salec_internal_enter(salec_gpu *h);
 int salec_internal_field_view(salec_gpu *h, const char *name, const void **base, int *f32, long long *plane,
                               int *pitch, int *nx, int *ny, int *nc);
 cudaStream_t salec_internal_stream(salec_gpu *h);
@@ -141,11 +144,19 @@ __global__ void k_conserve_final(int nblocks, const double *partials, double *ou
 extern "C" int salec_gpu_conservation(salec_gpu *h, double *out, int n)
 {
     if (!h || !out) return salec_internal_fail(SALEC_ERR_ARG, "salec_gpu_conservation: null argument");
+    const auto lock = salec_internal_enter(h);
     const Dims d = salec_internal_dims(h);
     const int need = 5 + (d.nmat - 1);
     if (n < need)
         return salec_internal_fail(SALEC_ERR_ARG, ("salec_gpu_conservation: needs " + std::to_string(need) +
                                                    " doubles, got " + std::to_string(n)).c_str());
+    void *&slot = salec_internal_conserve_slot(h);
+    if (!slot) {
+        // block partials (kBlocks x kQ pairs) and the kQ results, kept for the handle's lifetime; before the
+        // fields are looked at, as an allocation may move them
+        if (salec_internal_malloc(h, &slot, sizeof(double) * (2 * kBlocks * kQ + kQ)) != 0)
+            return salec_internal_fail(SALEC_ERR_ALLOC, "salec_gpu_conservation: scratch");
+    }
     Planes q{};
     const void *base;
     int f32, pitch, nx, ny, nc;
@@ -170,12 +181,6 @@ extern "C" int salec_gpu_conservation(salec_gpu *h, double *out, int n)
     q.enx = d.enx; q.eny = d.eny; q.vnx = d.vnx; q.vny = d.vny;
     q.nmat = d.nmat;
     cudaStream_t s = salec_internal_stream(h);
-    void *&slot = salec_internal_conserve_slot(h);
-    if (!slot) {
-        // block partials (kBlocks x kQ pairs) and the kQ results, kept for the handle's lifetime
-        if (cudaMalloc(&slot, sizeof(double) * (2 * kBlocks * kQ + kQ)) != cudaSuccess)
-            return salec_internal_fail(SALEC_ERR_ALLOC, "salec_gpu_conservation: scratch");
-    }
     double *partials = static_cast<double *>(slot);
     double *res = partials + 2 * kBlocks * kQ;
     k_conserve_partial<<<kBlocks, kThreads, 0, s>>>(q, partials);

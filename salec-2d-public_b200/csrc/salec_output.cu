@@ -22,6 +22,7 @@
 #include <cerrno>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <sys/stat.h>
 #include <thread>
@@ -31,6 +32,8 @@ using namespace salec;
 
 struct salec_gpu;
 int salec_internal_fail(int code, const char *msg);
+int salec_internal_malloc(salec_gpu *h, void **p, size_t n);
+std::unique_lock<std::recursive_mutex> salec_internal_enter(salec_gpu *h);
 int salec_internal_field_view(salec_gpu *h, const char *name, const void **base, int *f32, long long *plane,
                               int *pitch, int *nx, int *ny, int *nc);
 cudaStream_t salec_internal_stream(salec_gpu *h);
@@ -363,14 +366,14 @@ int finish(Writer *W)
 }
 
 template <typename T>
-int ensure(T *&p, size_t &have, size_t need, bool pinned)
+int ensure(salec_gpu *h, T *&p, size_t &have, size_t need, bool pinned)
 {
     if (need <= have) return 0;
     if (p) { if (pinned) cudaFreeHost(p); else cudaFree(p); }
     p = nullptr;
     have = 0;
-    cudaError_t e = pinned ? cudaMallocHost((void **)&p, need * sizeof(T)) : cudaMalloc((void **)&p, need * sizeof(T));
-    if (e != cudaSuccess) return -1;
+    if (pinned ? cudaMallocHost((void **)&p, need * sizeof(T)) != cudaSuccess : salec_internal_malloc(h, (void **)&p, need * sizeof(T)) != 0)
+        return -1;
     have = need;
     return 0;
 }
@@ -388,6 +391,7 @@ extern "C" int salec_gpu_write_output(salec_gpu *h, const char *dir, const char 
 {
     if (!h || !dir || !prefix || rank < 0 || out_step < 0)
         return salec_internal_fail(SALEC_ERR_ARG, "salec_gpu_write_output: null or negative argument");
+    const auto lock = salec_internal_enter(h);
     void *&slot = salec_internal_output_slot(h);
     if (!slot) slot = new Writer();
     Writer *W = static_cast<Writer *>(slot);
@@ -443,10 +447,17 @@ extern "C" int salec_gpu_write_output(salec_gpu *h, const char *dir, const char 
     J.ntr = T.n;
     J.tracer_off = off;
     const size_t floats = (size_t)off + (size_t)T.n * kTracerCols;
-    if (ensure(W->dev, W->dev_floats, floats, false) || ensure(W->host, W->host_floats, floats, true) ||
-        ensure(W->dev_live, W->live_n, (size_t)std::max(T.n, 1), false) ||
-        ensure(W->host_live, W->host_live_n, (size_t)std::max(T.n, 1), true))
+    if (ensure(h, W->dev, W->dev_floats, floats, false) || ensure(h, W->host, W->host_floats, floats, true) ||
+        ensure(h, W->dev_live, W->live_n, (size_t)std::max(T.n, 1), false) ||
+        ensure(h, W->host_live, W->host_live_n, (size_t)std::max(T.n, 1), true))
         return salec_internal_fail(SALEC_ERR_ALLOC, "salec_gpu_write_output: staging allocation failed");
+    // an allocation may have moved the fields (the handle gives up its second donor copy)
+    for (int k = 0; k < b.nseg; ++k) {
+        PackSeg &g = b.seg[k];
+        int nx, ny, nc;
+        if ((rc = salec_internal_field_view(h, items[k].field, &g.base, &g.f32, &g.plane, &g.pitch, &nx, &ny, &nc)))
+            return rc;
+    }
     if (!W->done && cudaEventCreateWithFlags(&W->done, cudaEventDisableTiming) != cudaSuccess)
         return salec_internal_fail(SALEC_ERR_CUDA, "salec_gpu_write_output: event creation failed");
 

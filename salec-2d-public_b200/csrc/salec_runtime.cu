@@ -18,6 +18,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -190,6 +191,12 @@ struct salec_gpu {
     unsigned char *quiet_map = nullptr;
     bool quiet_known = true;     // a graph cycle has run since the map was forgotten: false means that
                                  // both lists hold every tile
+    // Other handles may take the second copy when the device is out of memory (allocate): the entry points
+    // that use the fields, the flip or the graph hold `busy`, and the copy is taken only from a handle that
+    // none of them is in. `spare`: there is one to take.
+    std::recursive_mutex busy;
+    std::atomic<bool> spare{false};
+    int device = 0;
     bool fractions_known = false;   // Scal::odd_fractions is what the last graph cycle left
     bool in_graph = false;       // the cycle graph is being captured: its kernels take the quiet map
     bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
@@ -304,12 +311,14 @@ int upload_vec(salec_gpu *h, const std::vector<T> &v, const T **out)
     return SALEC_OK;
 }
 
+cudaError_t device_malloc(salec_gpu *h, void **p, size_t n);
+
 // One device allocation for every queued array, one copy, then the addresses.
 int flush_uploads(salec_gpu *h)
 {
     if (h->up_fix.empty()) return SALEC_OK;
     void *p = nullptr;
-    CUDA_TRY(cudaMalloc(&p, h->up_host.size()));
+    CUDA_TRY(device_malloc(h, &p, h->up_host.size()));
     h->owned.push_back(p);
     CUDA_TRY(cudaMemcpyAsync(p, h->up_host.data(), h->up_host.size(), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -625,20 +634,74 @@ void destroy_cycle_graphs(salec_gpu *h)
 bool release_donor_copy(salec_gpu *h)
 {
     cudaGetLastError();
-    if (!h->alt_pool || settle(h) != SALEC_OK || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!h->alt_pool || cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+        return false;
+    if (settle(h) != SALEC_OK || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
     destroy_cycle_graphs(h);
     cudaFree(h->alt_pool);
     if (h->quiet_map) cudaFree(h->quiet_map);
     h->alt_pool = nullptr;
     h->quiet_map = nullptr;
     h->alt = h->f;
+    h->spare = false;
     return true;
+}
+
+// The handles of the process, for the copies that they can spare. Never destroyed: a handle may be closed
+// while the process ends.
+struct Handles {
+    std::mutex mutex;
+    std::vector<salec_gpu *> list;
+};
+Handles &handles()
+{
+    static Handles &all = *new Handles();
+    return all;
+}
+
+// Run `request`, a device allocation for handle h. Where it fails for lack of memory, the second donor
+// copies are given up one after another until it succeeds: h's own, then those of the other handles on the
+// device, each when no call is inside its handle. A thread that waits here offers no copy itself, so that
+// two of them do not wait for one another.
+template <class Request>
+cudaError_t allocate(salec_gpu *h, Request request)
+{
+    cudaError_t e = request();
+    if (e == cudaErrorMemoryAllocation && release_donor_copy(h)) e = request();
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    const bool was_spare = h->spare.exchange(false);
+    {
+        std::lock_guard<std::mutex> all(handles().mutex);
+        for (salec_gpu *o : handles().list) {
+            if (o == h || o->device != h->device) continue;
+            bool released = false, tried = false;
+            while (o->spare && !tried) {
+                if (!o->busy.try_lock()) {
+                    std::this_thread::sleep_for(std::chrono::microseconds(50));
+                    continue;
+                }
+                released = release_donor_copy(o);
+                o->busy.unlock();
+                tried = true;
+            }
+            if (released && (e = request()) != cudaErrorMemoryAllocation) break;
+            cudaGetLastError();
+        }
+    }
+    if (was_spare && h->alt_pool) h->spare = true;
+    return e;
 }
 
 cudaError_t device_malloc(salec_gpu *h, void **p, size_t n)
 {
-    const cudaError_t e = cudaMalloc(p, n);
-    return e == cudaErrorMemoryAllocation && release_donor_copy(h) ? cudaMalloc(p, n) : e;
+    return allocate(h, [&] { return cudaMalloc(p, n); });
+}
+
+cudaError_t stream_malloc(salec_gpu *h, void **p, size_t n)
+{
+    return allocate(h, [&] { return cudaMallocAsync(p, n, h->stream); });
 }
 
 // The whole cycle as the cycle graph holds it: the phases in order, with the energy update inside
@@ -729,7 +792,7 @@ int build_gathers(salec_gpu *h)
     if ((rc = make_gather(h, h->r_dis, {dis}))) return rc;
     if (h->scratch_doubles) {
         void *p = nullptr;
-        CUDA_TRY(cudaMalloc(&p, h->scratch_doubles * sizeof(double)));
+        CUDA_TRY(device_malloc(h, &p, h->scratch_doubles * sizeof(double)));
         h->owned.push_back(p);
         h->scratch = static_cast<double *>(p);
     }
@@ -854,7 +917,7 @@ int build_geo_table(salec_gpu *h, int slot, int fid, int nx, int ny, int nc)
     // temporaries are stream-ordered (cudaMallocAsync / cudaFreeAsync): freeing them does not
     // synchronise the device, which would stall every other handle's work
     unsigned long long *d_hash = nullptr;
-    CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&d_hash), sizeof(unsigned long long) * 2 * ny, h->stream));
+    CUDA_TRY(stream_malloc(h, reinterpret_cast<void **>(&d_hash), sizeof(unsigned long long) * 2 * ny));
     k_geo_row_hash<<<ny, 256, 0, h->stream>>>(src, row_words, d_hash);
     cudaError_t e = cudaGetLastError();
     std::vector<unsigned long long> hashes(2 * (size_t)ny);
@@ -911,13 +974,12 @@ int build_geo_table(salec_gpu *h, int slot, int fid, int nx, int ny, int nc)
         if (d_diff) cudaFreeAsync(d_diff, h->stream);
         if (d_rows) cudaFreeAsync(d_rows, h->stream);
     };
-    e = cudaMallocAsync(reinterpret_cast<void **>(&d_idx), sizeof(int) * ((size_t)ny + U), h->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&d_diff), sizeof(unsigned), h->stream);
+    e = stream_malloc(h, reinterpret_cast<void **>(&d_idx), sizeof(int) * ((size_t)ny + U));
+    if (e == cudaSuccess) e = stream_malloc(h, reinterpret_cast<void **>(&d_diff), sizeof(unsigned));
     if (e == cudaSuccess)
-        e = cudaMallocAsync(reinterpret_cast<void **>(&d_rows), sizeof(unsigned long long) * (size_t)U * row_words,
-                            h->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&g.tab, (size_t)nc * plane * field_elem(h, fid));
-    if (e == cudaSuccess) e = cudaMalloc(&g.row, sizeof(int) * h->d.R);
+        e = stream_malloc(h, reinterpret_cast<void **>(&d_rows), sizeof(unsigned long long) * (size_t)U * row_words);
+    if (e == cudaSuccess) e = device_malloc(h, &g.tab, (size_t)nc * plane * field_elem(h, fid));
+    if (e == cudaSuccess) e = device_malloc(h, reinterpret_cast<void **>(&g.row), sizeof(int) * h->d.R);
     g.compact = true;
     g.plane = plane;
     unsigned diff = 0;
@@ -953,10 +1015,7 @@ int ensure_staging(salec_gpu *h, size_t need)
     if (h->staging) CUDA_TRY(cudaFreeAsync(h->staging, h->stream));
     h->staging = nullptr;
     h->staging_doubles = 0;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&h->staging), need * sizeof(double), h->stream);
-    if (e == cudaErrorMemoryAllocation && release_donor_copy(h))
-        e = cudaMallocAsync(reinterpret_cast<void **>(&h->staging), need * sizeof(double), h->stream);
-    CUDA_TRY(e);
+    CUDA_TRY(stream_malloc(h, reinterpret_cast<void **>(&h->staging), need * sizeof(double)));
     h->staging_doubles = need;
     return SALEC_OK;
 }
@@ -1068,8 +1127,11 @@ int finish_init_t(salec_gpu *h, double damp_time_in, double *damp_time_out)
 
 // Last start-up steps on the device (src/salec2d.c:76-94): first EOS call, ghost fills,
 // damping reference state and arrival time, vertex velocities, cleared cell velocities.
+std::unique_lock<std::recursive_mutex> salec_internal_enter(salec_gpu *h);
+
 int salec_internal_finish_init(salec_gpu *h, double damp_time_in, double *damp_time_out)
 {
+    const auto lock = salec_internal_enter(h);
     return h->mixed ? finish_init_t<float>(h, damp_time_in, damp_time_out)
                     : finish_init_t<double>(h, damp_time_in, damp_time_out);
 }
@@ -1094,6 +1156,8 @@ cudaStream_t salec_internal_stream(salec_gpu *h) { return h->stream; }
 Tracers salec_internal_tracers(salec_gpu *h) { return h->tr; }
 Dims salec_internal_dims(salec_gpu *h) { return h->d; }
 void salec_internal_add_launches(salec_gpu *h, int n) { h->launches += n; }
+int salec_internal_malloc(salec_gpu *h, void **p, size_t n) { return device_malloc(h, p, n) == cudaSuccess ? 0 : -1; }
+std::unique_lock<std::recursive_mutex> salec_internal_enter(salec_gpu *h) { return std::unique_lock<std::recursive_mutex>(h->busy); }
 void *&salec_internal_output_slot(salec_gpu *h) { return h->output; }
 void *&salec_internal_conserve_slot(salec_gpu *h) { return h->conserve; }
 
@@ -1101,6 +1165,7 @@ void *&salec_internal_conserve_slot(salec_gpu *h) { return h->conserve; }
 // where the handle has none.
 extern "C" int salec_internal_listed_tiles(salec_gpu *h, int *listed, int *total)
 {
+    const auto lock = salec_internal_enter(h);
     *listed = *total = 0;
     if (!h->quiet_map) return SALEC_OK;
     *total = h->tiles();
@@ -1163,6 +1228,7 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     if (run->precision != SALEC_PRECISION_FP64 && run->precision != SALEC_PRECISION_MIXED)
         return fail(SALEC_ERR_ARG, "precision must be SALEC_PRECISION_FP64 or SALEC_PRECISION_MIXED");
     salec_gpu *h = new salec_gpu();
+    cudaGetDevice(&h->device);
     for (int k = 0; k < SK_COUNT; ++k) h->blk[k] = dim3(32, 4);
     Dims &d = h->d;
     d.nmat = run->nmat;
@@ -1201,7 +1267,7 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     for (int k = 0; k < kNumFields; ++k)
         bytes += kFields[k].loc == L_COL ? col * sizeof(double) : (size_t)field_ncomp(h, k) * d.PL * field_elem(h, k);
     h->pool_bytes = bytes;
-    if (cudaMalloc(&h->pool, h->pool_bytes) != cudaSuccess)
+    if (device_malloc(h, reinterpret_cast<void **>(&h->pool), h->pool_bytes) != cudaSuccess)
         return bail(fail(SALEC_ERR_ALLOC, "device pool of " + std::to_string(h->pool_bytes) + " bytes"));
     if (cudaMemsetAsync(h->pool, 0, h->pool_bytes, h->stream) != cudaSuccess)
         return bail(fail(SALEC_ERR_CUDA, "pool memset failed"));
@@ -1213,7 +1279,7 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
 
     {
         const size_t words = (size_t)(d.P / 32) * d.R;
-        if (cudaMalloc(&h->lap_mask, words * sizeof(unsigned)) != cudaSuccess)
+        if (device_malloc(h, reinterpret_cast<void **>(&h->lap_mask), words * sizeof(unsigned)) != cudaSuccess)
             return bail(fail(SALEC_ERR_ALLOC, "Laplacian mask"));
         if (cudaMemsetAsync(h->lap_mask, 0, words * sizeof(unsigned), h->stream) != cudaSuccess)
             return bail(fail(SALEC_ERR_CUDA, "Laplacian mask memset"));
@@ -1221,7 +1287,7 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     {
         std::vector<int> ident(d.R);
         for (int j = 0; j < d.R; ++j) ident[j] = j;
-        if (cudaMalloc(&h->row_identity, sizeof(int) * d.R) != cudaSuccess)
+        if (device_malloc(h, reinterpret_cast<void **>(&h->row_identity), sizeof(int) * d.R) != cudaSuccess)
             return bail(fail(SALEC_ERR_ALLOC, "row map"));
         if (cudaMemcpy(h->row_identity, ident.data(), sizeof(int) * d.R, cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(fail(SALEC_ERR_CUDA, "row map upload"));
@@ -1239,11 +1305,11 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
         if (rc) return bail(rc);
     }
     if (int rc = flush_uploads(h)) return bail(rc);
-    if (cudaMalloc(&h->mat, sizeof(DevMat) * d.nmat) != cudaSuccess) return bail(fail(SALEC_ERR_ALLOC, "materials"));
+    if (device_malloc(h, reinterpret_cast<void **>(&h->mat), sizeof(DevMat) * d.nmat) != cudaSuccess) return bail(fail(SALEC_ERR_ALLOC, "materials"));
     if (cudaMemcpy(h->mat, dms.data(), sizeof(DevMat) * d.nmat, cudaMemcpyHostToDevice) != cudaSuccess)
         return bail(fail(SALEC_ERR_CUDA, "material upload"));
 
-    if (cudaMalloc(&h->scal, sizeof(Scal)) != cudaSuccess) return bail(fail(SALEC_ERR_ALLOC, "scalars"));
+    if (device_malloc(h, reinterpret_cast<void **>(&h->scal), sizeof(Scal)) != cudaSuccess) return bail(fail(SALEC_ERR_ALLOC, "scalars"));
     const size_t host_bytes = salec_gpu::rounded(sizeof(Scal)) + sizeof(Report) + d.enx * sizeof(double);
     if (cudaMallocHost(&h->scal_host, host_bytes) != cudaSuccess) return bail(fail(SALEC_ERR_ALLOC, "scalars"));
     memset(h->scal_host, 0, host_bytes);
@@ -1267,6 +1333,11 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
     h->profile_acc = const_cast<unsigned long long *>(acc_dev);
     allocate_donor_copy(h);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(SALEC_ERR_CUDA, "create sync"));
+    h->spare = h->alt_pool != nullptr;
+    {
+        std::lock_guard<std::mutex> all(handles().mutex);
+        handles().list.push_back(h);
+    }
     *out = h;
     return SALEC_OK;
 }
@@ -1274,6 +1345,11 @@ int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats,
 int salec_gpu_destroy(salec_gpu *h)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    {
+        std::lock_guard<std::mutex> all(handles().mutex);
+        auto &list = handles().list;
+        list.erase(std::remove(list.begin(), list.end(), h), list.end());
+    }
     cudaStreamSynchronize(h->stream);
     release(h);
     return SALEC_OK;
@@ -1293,18 +1369,21 @@ int salec_gpu_field_shape(const salec_gpu *h, int field, int *nx, int *ny, int *
 int salec_gpu_set_field(salec_gpu *h, int field, const double *host, long long n)
 {
     if (!h || !host) return fail(SALEC_ERR_ARG, "null argument");
+    const auto lock = salec_internal_enter(h);
     return transfer(h, field, const_cast<double *>(host), n, true);
 }
 
 int salec_gpu_get_field(salec_gpu *h, int field, double *host, long long n)
 {
     if (!h || !host) return fail(SALEC_ERR_ARG, "null argument");
+    const auto lock = salec_internal_enter(h);
     return transfer(h, field, host, n, false);
 }
 
 int salec_gpu_phases(salec_gpu *h, int first, int last)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     if (first < 0 || last > 15 || first > last) return fail(SALEC_ERR_ARG, "phase range must lie in [0, 15]");
     if (int rc = settle(h)) return rc;
     for (int p = first; p <= last; ++p) {
@@ -1382,6 +1461,7 @@ void capture_cycle_graph(salec_gpu *h)
 int salec_gpu_step(salec_gpu *h, int nsteps)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     if (nsteps < 0) return fail(SALEC_ERR_ARG, "negative step count");
     for (int k = 0; k < nsteps; ++k) {
         if (!h->profiling && !h->cycle_graph[h->flip]) capture_cycle_graph(h);
@@ -1409,6 +1489,7 @@ int salec_gpu_step(salec_gpu *h, int nsteps)
 int salec_gpu_step_report(salec_gpu *h, int nsteps, double *dt, double *time, double *profile, long long profile_n)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     const int fid = field_by_name("y_profile");
     int nx = 0, ny = 0;
     field_points(h, fid, nx, ny);
@@ -1438,6 +1519,7 @@ int salec_gpu_step_report(salec_gpu *h, int nsteps, double *dt, double *time, do
 int salec_gpu_step_report_async(salec_gpu *h, int nsteps, double *profile, long long profile_n, int slot)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     if (slot < 0 || slot > 1) return fail(SALEC_ERR_ARG, "report slot must be 0 or 1");
     if (h->report_pending[slot]) return fail(SALEC_ERR_STATE, "report slot still in flight: wait for it first");
     const int fid = field_by_name("y_profile");
@@ -1541,6 +1623,7 @@ constexpr int kNumTuned = sizeof(kTunedPhase) / sizeof(kTunedPhase[0]);
 int salec_gpu_set_block_shapes(salec_gpu *h, const int *shapes, int n)
 {
     if (!h || (n > 0 && !shapes) || n < 0) return fail(SALEC_ERR_ARG, "bad argument");
+    const auto lock = salec_internal_enter(h);
     for (int k = 0; k < n; ++k) {
         const int p = shapes[3 * k], bx = shapes[3 * k + 1], by = shapes[3 * k + 2];
         int t = 0;
@@ -1562,6 +1645,7 @@ int salec_gpu_set_block_shapes(salec_gpu *h, const int *shapes, int n)
 int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
 {
     if (!h || cycles < 1) return fail(SALEC_ERR_ARG, "bad argument");
+    const auto lock = salec_internal_enter(h);
     // a shape stands for its thread count (launch_step_kernel). 32x1 is not offered: timed sweep by sweep
     // it ties with the others, but one block per row segment of a listed tile costs the cycle graph
     // up to 30 us a sweep (2048x2048: 956-996 us a cycle with one sweep at 32x1, 920-930 without)
@@ -1577,7 +1661,7 @@ int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
     Scal scal_host{};
     CUDA_TRY(cudaMemcpy(&scal_host, h->scal, sizeof(Scal), cudaMemcpyDeviceToHost));
     if (device_malloc(h, &snap, h->pool_bytes) != cudaSuccess) return fail(SALEC_ERR_ALLOC, "autotune snapshot");
-    if (h->tr_bytes && cudaMalloc(&snap_tr, h->tr_bytes) != cudaSuccess) {
+    if (h->tr_bytes && device_malloc(h, &snap_tr, h->tr_bytes) != cudaSuccess) {
         cudaFree(snap);
         return fail(SALEC_ERR_ALLOC, "autotune snapshot");
     }
@@ -1659,6 +1743,7 @@ int salec_gpu_get_scalar(salec_gpu *h, const char *name, double *value)
 int salec_gpu_set_scalar(salec_gpu *h, const char *name, double value)
 {
     if (!h || !name) return fail(SALEC_ERR_ARG, "null argument");
+    const auto lock = salec_internal_enter(h);
     if (!strcmp(name, "damp_time")) { h->rp.damp_time = value; drop_cycle_graph(h); return SALEC_OK; }
     if (!strcmp(name, "max_dt")) { h->rp.max_dt = value; drop_cycle_graph(h); return SALEC_OK; }
     CUDA_TRY(cudaMemcpyAsync(h->scal_host, h->scal, sizeof(Scal), cudaMemcpyDeviceToHost, h->stream));
@@ -1677,6 +1762,7 @@ int salec_gpu_set_scalar(salec_gpu *h, const char *name, double value)
 int salec_gpu_set_tracers(salec_gpu *h, int n, const double *rows)
 {
     if (!h || n < 0 || (n > 0 && !rows)) return fail(SALEC_ERR_ARG, "bad argument");
+    const auto lock = salec_internal_enter(h);
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     drop_cycle_graph(h);
     if (h->tr_block) cudaFree(h->tr_block);
@@ -1686,7 +1772,7 @@ int salec_gpu_set_tracers(salec_gpu *h, int n, const double *rows)
     const size_t nd = 6, nf = 2, ni = 7;
     auto rounded = [](size_t sz) { return ((sz + 255) / 256) * 256; };
     const size_t bytes = nd * rounded((size_t)n * 8) + (nf + ni) * rounded((size_t)n * 4);
-    CUDA_TRY(cudaMalloc(&h->tr_block, bytes));
+    CUDA_TRY(device_malloc(h, &h->tr_block, bytes));
     h->tr_bytes = bytes;
     char *p = static_cast<char *>(h->tr_block);
     char *const end = p + bytes;
@@ -1761,6 +1847,7 @@ int salec_gpu_get_tracers(salec_gpu *h, double *rows, int *n)
 int salec_gpu_check(salec_gpu *h, long long *n_bad)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     unsigned long long *cnt = &h->scal->nan_count;
     CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), h->stream));
     const char *names[] = {"v_vel", "v_acc", "v_dis", "e_vel", "e_ste", "e_dvel", "e_pre", "e_den", "e_csd",
@@ -1887,7 +1974,7 @@ const AdjointState::ListCopy *list_table(salec_gpu *h, const std::vector<const c
     }
     segs.push_back({reinterpret_cast<char *>(h->scal), off, sizeof(Scal)});
     AdjointState::ListCopy L;
-    if (cudaMalloc(reinterpret_cast<void **>(&L.dev), segs.size() * sizeof(CopySeg)) != cudaSuccess) return nullptr;
+    if (device_malloc(h, reinterpret_cast<void **>(&L.dev), segs.size() * sizeof(CopySeg)) != cudaSuccess) return nullptr;
     if (cudaMemcpy(L.dev, segs.data(), segs.size() * sizeof(CopySeg), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(L.dev);
         return nullptr;
@@ -1904,7 +1991,7 @@ const AdjointState::ListCopy *seg_table(salec_gpu *h, const std::string &key, co
     auto it = st->lists.find(key);
     if (it != st->lists.end()) return &it->second;
     AdjointState::ListCopy L;
-    if (cudaMalloc(reinterpret_cast<void **>(&L.dev), segs.size() * sizeof(CopySeg)) != cudaSuccess) return nullptr;
+    if (device_malloc(h, reinterpret_cast<void **>(&L.dev), segs.size() * sizeof(CopySeg)) != cudaSuccess) return nullptr;
     if (cudaMemcpy(L.dev, segs.data(), segs.size() * sizeof(CopySeg), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(L.dev);
         return nullptr;
@@ -1977,7 +2064,7 @@ int adjoint_ensure(salec_gpu *h)
     AdjointState *st = h->adj;
     if (!st->pool) {
         CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->pool), h->pool_bytes));
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->theta), 4 * sizeof(double)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->theta), 4 * sizeof(double)));
         for (int k = 0; k < kNumFields; ++k) {
             const size_t off = reinterpret_cast<char *>(field_ptr(h, k)) - h->pool;
             *reinterpret_cast<double **>(reinterpret_cast<char *>(&st->b) + kFields[k].off) =
@@ -1991,13 +2078,13 @@ int adjoint_ensure(salec_gpu *h)
             gs = std::max(gs, e * (size_t)std::max(g->ncomp_max, 1));
         }
         st->gscratch_doubles = std::max<size_t>(gs, 1);
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->gscratch), st->gscratch_doubles * sizeof(double)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->gscratch), st->gscratch_doubles * sizeof(double)));
         size_t tb = 0;
         for (int p = 0; p < 16; ++p) tb = std::max(tb, list_bytes(h, kAdjWrites[p]));
         for (const auto *l : {&kKeep12, &kKeep8, &kKeep1}) tb = std::max(tb, list_bytes(h, *l));
         st->tmp_bytes = tb;
         CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->tmp), tb));
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->slot), sizeof(long long)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->slot), sizeof(long long)));
         CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->cscr), 16 * (size_t)h->d.PL * sizeof(double)));
         // every list table, so that the graphs can be captured
         const std::vector<const char *> snap(std::begin(kAdjSnapshot), std::end(kAdjSnapshot));
@@ -2232,13 +2319,14 @@ extern "C" {
 int salec_gpu_set_dt_schedule(salec_gpu *h, const double *dts, int n)
 {
     if (!h || n < 0 || (n > 0 && !dts)) return fail(SALEC_ERR_ARG, "bad argument");
+    const auto lock = salec_internal_enter(h);
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     if (h->dt_sched) CUDA_TRY(cudaFree(h->dt_sched));
     h->dt_sched = nullptr;
     h->dt_sched_n = 0;
     if (n > 0) {
         CUDA_TRY(cudaMemcpy(&h->scal_host->i_step, &h->scal->i_step, sizeof(long long), cudaMemcpyDeviceToHost));
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&h->dt_sched), n * sizeof(double)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&h->dt_sched), n * sizeof(double)));
         CUDA_TRY(cudaMemcpy(h->dt_sched, dts, n * sizeof(double), cudaMemcpyHostToDevice));
         h->dt_sched_i0 = h->scal_host->i_step;
         h->dt_sched_n = n;
@@ -2250,6 +2338,7 @@ int salec_gpu_set_dt_schedule(salec_gpu *h, const double *dts, int n)
 int salec_gpu_adjoint_reset(salec_gpu *h)
 {
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
+    const auto lock = salec_internal_enter(h);
     if (int rc = adjoint_check(h)) return rc;
     if (int rc = adjoint_zero(h)) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -2259,6 +2348,7 @@ int salec_gpu_adjoint_reset(salec_gpu *h)
 int salec_gpu_adjoint_set_field(salec_gpu *h, int field, const double *host, long long n)
 {
     if (!h || !host || !h->adj || !h->adj->pool) return fail(SALEC_ERR_STATE, "call salec_gpu_adjoint_reset first");
+    const auto lock = salec_internal_enter(h);
     if (field < 0 || field >= kNumFields) return fail(SALEC_ERR_ARG, "unknown field");
     return adjoint_transfer(h, field, const_cast<double *>(host), n, true);
 }
@@ -2266,6 +2356,7 @@ int salec_gpu_adjoint_set_field(salec_gpu *h, int field, const double *host, lon
 int salec_gpu_adjoint_get_field(salec_gpu *h, int field, double *host, long long n)
 {
     if (!h || !host || !h->adj || !h->adj->pool) return fail(SALEC_ERR_STATE, "call salec_gpu_adjoint_reset first");
+    const auto lock = salec_internal_enter(h);
     if (field < 0 || field >= kNumFields) return fail(SALEC_ERR_ARG, "unknown field");
     return adjoint_transfer(h, field, host, n, false);
 }
@@ -2273,6 +2364,7 @@ int salec_gpu_adjoint_get_field(salec_gpu *h, int field, double *host, long long
 int salec_gpu_adjoint_phase(salec_gpu *h, int phase)
 {
     if (!h || !h->adj || !h->adj->pool) return fail(SALEC_ERR_STATE, "call salec_gpu_adjoint_reset first");
+    const auto lock = salec_internal_enter(h);
     if (phase < 0 || phase > 15) return fail(SALEC_ERR_ARG, "phase out of range");
     if (int rc = settle(h)) return rc;
     if (int rc = adjoint_phase(h, phase)) return rc;
@@ -2292,6 +2384,7 @@ int salec_gpu_adjoint_window(salec_gpu *h, int nsteps, int every, const double *
                              int ncols, double *grad_density, long long n_density, salec_adjoint_result *out)
 {
     if (!h || nsteps < 1 || every < 1 || !target || !out) return fail(SALEC_ERR_ARG, "bad argument");
+    const auto lock = salec_internal_enter(h);
     if (ncols != h->d.enx - 4) return fail(SALEC_ERR_ARG, "target and weights need one value per interior column");
     if (grad_density && n_density != (long long)h->d.enx * h->d.eny)
         return fail(SALEC_ERR_ARG, "grad_density needs (nx+4)*(ny+4) doubles");
@@ -2324,7 +2417,7 @@ int salec_gpu_adjoint_window(salec_gpu *h, int nsteps, int every, const double *
     if (st->mis_doubles < md) {
         cudaFree(st->mis);
         st->mis = nullptr;
-        CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&st->mis), md * sizeof(double)));
+        CUDA_TRY(device_malloc(h, reinterpret_cast<void **>(&st->mis), md * sizeof(double)));
         st->mis_doubles = md;
     }
     if (int rc = adjoint_graphs(h, ub, uoff)) return rc;
