@@ -238,6 +238,10 @@ def make_deck(n: int, folder: str) -> str:
 
 
 # ---------------------------------------------------------------- CPU reference leg
+class ReferenceUnavailable(RuntimeError):
+    """The reference cannot be run on this machine."""
+
+
 def _cpu_reference_worker(deck: str, eos_dir: str, steps: int, warmup: int, barrier, results) -> None:
     """One reference process of cpu_reference_cores: its own oracle instance (the reference
     keeps global state), started by the reference's own initialisation of the deck
@@ -269,8 +273,13 @@ def cpu_reference_cores(n: int, steps: int, warmup: int, folder: str, procs: int
     best, with no halo exchange). Each process starts from the reference's own initialisation of
     the same deck, steps `warmup` cycles, meets the others at a barrier and steps `steps` cycles;
     the rate is procs x n^2 x steps over the slowest process's time. Returns the rate, the
-    slowest timed window and the slowest initialisation."""
+    slowest timed window and the slowest initialisation; raises ReferenceUnavailable where the
+    reference is not built on this machine or one of the processes ends early."""
     import multiprocessing as mp
+    import queue
+    from oracle import ref
+    if not ref.available():
+        raise ReferenceUnavailable("oracle/_ref/libsalec_ref.so is not built (it needs the reference's sources)")
     deck = make_deck(n, folder)
     ctx = mp.get_context("spawn")
     barrier = ctx.Barrier(procs)
@@ -279,7 +288,17 @@ def cpu_reference_cores(n: int, steps: int, warmup: int, folder: str, procs: int
                for _ in range(procs)]
     for w in workers:
         w.start()
-    got = [results.get(timeout=3600) for _ in workers]
+    got, until = [], time.monotonic() + 3600
+    while len(got) < procs:
+        try:
+            got.append(results.get(timeout=1.0))
+        except queue.Empty:
+            ended = [w.exitcode for w in workers if w.exitcode is not None]
+            if len(ended) > len(got) or time.monotonic() > until:
+                # the others wait for it at the barrier
+                for w in workers:
+                    w.terminate()
+                raise ReferenceUnavailable("a reference process ended without a result (exit codes %s)" % ended)
     for w in workers:
         w.join()
     secs = max(g[0] for g in got)
@@ -298,8 +317,12 @@ def run_reference_arm(args):
         return
     n = args.cpu_n
     procs = host_cores()
-    with tempfile.TemporaryDirectory() as tmp:
-        rate, secs, init_s = cpu_reference_cores(n, args.steps, args.warmup, tmp, procs)
+    try:
+        with tempfile.TemporaryDirectory() as tmp:
+            rate, secs, init_s = cpu_reference_cores(n, args.steps, args.warmup, tmp, procs)
+    except ReferenceUnavailable as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     line = {"impl": "reference", "metric": METRIC, "value": rate, "unit": "cell-updates/s", "n_gpus": args.gpus,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1000.0 * secs / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
@@ -690,12 +713,15 @@ def run_gpu_arm(args):
     cpu = None
     if rank == 0 and not args.no_cpu:
         procs = host_cores()
-        with tempfile.TemporaryDirectory() as ctmp:
-            rate, secs, cinit = cpu_reference_cores(args.cpu_n, args.cpu_steps, 2, ctmp, procs)
-        cpu = {"value": rate, "unit": "cell-updates/s", "cores": procs, "kind": "reference",
-               "sample": "%d steps of a %dx%d-cell copy of the workload on each of %d reference processes, "
-                         "one per host core, each started by the reference's own initialisation (%.0f s); "
-                         "timed window %.1f s" % (args.cpu_steps, args.cpu_n, args.cpu_n, procs, cinit, secs)}
+        try:
+            with tempfile.TemporaryDirectory() as ctmp:
+                rate, secs, cinit = cpu_reference_cores(args.cpu_n, args.cpu_steps, 2, ctmp, procs)
+            cpu = {"value": rate, "unit": "cell-updates/s", "cores": procs, "kind": "reference",
+                   "sample": "%d steps of a %dx%d-cell copy of the workload on each of %d reference processes, "
+                             "one per host core, each started by the reference's own initialisation (%.0f s); "
+                             "timed window %.1f s" % (args.cpu_steps, args.cpu_n, args.cpu_n, procs, cinit, secs)}
+        except ReferenceUnavailable as e:
+            cpu = {"unavailable": str(e)}
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": "cell-updates/s", "n_gpus": world, "steps": args.steps,
