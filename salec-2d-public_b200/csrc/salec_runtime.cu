@@ -198,6 +198,11 @@ struct salec_gpu {
     std::atomic<bool> spare{false};
     int device = 0;
     bool fractions_known = false;   // Scal::odd_fractions is what the last graph cycle left
+    // A caller captured cycles or phases of this handle into a graph of its own (salec_gpu_stream). Its replays
+    // change the fields where they were at the capture and nothing here learns of them: from then on
+    // the handle works in place, on the copy that was current, without a quiet map.
+    bool in_place = false, graphs_stale = false;
+    bool dual() const { return alt_pool && !in_place; }
     bool in_graph = false;       // the cycle graph is being captured: its kernels take the quiet map
     bool volumes_only = false;   // the face records hold the last cycle's volumes but not its donors
     // pipelined read-back (salec_gpu_step_report_async): per slot a pinned copy of the scalars,
@@ -255,7 +260,7 @@ struct salec_gpu {
         c.next_list = c.next_count = nullptr;
         c.vacuum = c.quiet = nullptr;
         c.profile = in_graph ? profile_acc : nullptr;
-        if (in_graph && quiet_map) {
+        if (in_graph && quiet_map && !in_place) {
             c.vacuum = quiet_map;
             c.quiet = quiet_map + segment_bytes();
             c.tile_list = tile_list(flip);
@@ -543,7 +548,7 @@ double *&alt_ptr(salec_gpu *h, int k)
 int forget_quiet(salec_gpu *h)
 {
     h->fractions_known = false;
-    if (!h->quiet_map || !h->quiet_known) return SALEC_OK;
+    if (!h->quiet_map || !h->quiet_known || h->in_place) return SALEC_OK;
     h->quiet_known = false;
     launch_forget_quiet(h->quiet_map, h->tiles() * SALEC_TILE_ROWS, h->quiet_map + h->segment_bytes(), h->tiles_x(),
                         h->tiles_y(), h->tile_list(0), h->tile_count(0), h->tile_list(1), h->tile_count(1), h->stream);
@@ -605,11 +610,29 @@ int complete_records(salec_gpu *h)
     return SALEC_OK;
 }
 
+void destroy_cycle_graphs(salec_gpu *h)
+{
+    for (auto &g : h->cycle_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
+bool caller_captures(const salec_gpu *h)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool known = cudaStreamIsCapturing(h->stream, &capture) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    return !known || capture != cudaStreamCaptureStatusNone;
+}
+
 // Full face records, the donor state in the pool's own planes and no segment taken for quiet.
 int settle(salec_gpu *h)
 {
     if (int rc = complete_records(h)) return rc;
     if (h->flip) {
+        if (h->in_place)
+            return fail(SALEC_ERR_STATE, "not after a caller's capture that followed an odd number of cycles");
         for (int k : donor_fields(h)) {
             CUDA_TRY(cudaMemcpyAsync(alt_ptr(h, k), field_ptr(h, k),
                                      (size_t)field_ncomp(h, k) * h->d.PL * field_elem(h, k), cudaMemcpyDeviceToDevice,
@@ -621,12 +644,16 @@ int settle(salec_gpu *h)
     return forget_quiet(h);
 }
 
-void destroy_cycle_graphs(salec_gpu *h)
+// The same before phases run one by one. Under a caller's capture, and after one, nothing is moved: a
+// replay would move it again.
+int settle_or_stay(salec_gpu *h)
 {
-    for (auto &g : h->cycle_graph) {
-        if (g) cudaGraphExecDestroy(g);
-        g = nullptr;
+    if (caller_captures(h) && !h->in_place) {
+        h->in_place = true;
+        h->spare = false;
+        h->graphs_stale = true;   // they cannot be destroyed during the capture
     }
+    return h->in_place ? complete_records(h) : settle(h);
 }
 
 // The second copy of the donor state only makes cycles faster: it is given up where the device runs out
@@ -634,9 +661,7 @@ void destroy_cycle_graphs(salec_gpu *h)
 bool release_donor_copy(salec_gpu *h)
 {
     cudaGetLastError();
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!h->alt_pool || cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
-        return false;
+    if (!h->dual() || caller_captures(h)) return false;
     if (settle(h) != SALEC_OK || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
     destroy_cycle_graphs(h);
     cudaFree(h->alt_pool);
@@ -690,7 +715,7 @@ cudaError_t allocate(salec_gpu *h, Request request)
             cudaGetLastError();
         }
     }
-    if (was_spare && h->alt_pool) h->spare = true;
+    if (was_spare && h->dual()) h->spare = true;
     return e;
 }
 
@@ -734,7 +759,7 @@ int run_cycle_t(salec_gpu *h)
         if (int rc = run_phase(h, 9, true)) return rc;
         if (int rc = run_gather(h, h->g_flux_state)) return rc;
     }
-    const bool dual = h->alt_pool != nullptr;
+    const bool dual = h->dual();
     launch_step_kernel(SK_FLUX, c, s, h->blk[SK_FLUX], 1, dual ? 1 : 0);
     CUDA_TRY(cudaGetLastError());
     if (int rc = run_phase(h, 13, true)) return rc;
@@ -1385,7 +1410,7 @@ int salec_gpu_phases(salec_gpu *h, int first, int last)
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
     const auto lock = salec_internal_enter(h);
     if (first < 0 || last > 15 || first > last) return fail(SALEC_ERR_ARG, "phase range must lie in [0, 15]");
-    if (int rc = settle(h)) return rc;
+    if (int rc = settle_or_stay(h)) return rc;
     for (int p = first; p <= last; ++p) {
         if (h->profiling) {
             if (h->ev_used == h->ev_a.size()) {
@@ -1463,16 +1488,27 @@ int salec_gpu_step(salec_gpu *h, int nsteps)
     if (!h) return fail(SALEC_ERR_ARG, "null handle");
     const auto lock = salec_internal_enter(h);
     if (nsteps < 0) return fail(SALEC_ERR_ARG, "negative step count");
+    // sweep by sweep while profiling, and under a caller's capture as long as there is no graph (launching
+    // one is an error there)
+    bool sweeps = h->profiling;
+    if (!sweeps && nsteps > 0) {
+        const bool captures = caller_captures(h);
+        if (h->graphs_stale && !captures) {
+            destroy_cycle_graphs(h);
+            h->graphs_stale = false;
+        }
+        sweeps = captures && !h->cycle_graph[h->flip];
+    }
     for (int k = 0; k < nsteps; ++k) {
-        if (!h->profiling && !h->cycle_graph[h->flip]) capture_cycle_graph(h);
-        if (!h->profiling && h->cycle_graph[h->flip]) {
-            if (!h->fractions_known) {
+        if (!sweeps && !h->cycle_graph[h->flip]) capture_cycle_graph(h);
+        if (!sweeps && h->cycle_graph[h->flip]) {
+            if (h->dual() && !h->fractions_known) {
                 CUDA_TRY(cudaMemsetAsync(&h->scal->odd_fractions, 1, sizeof(unsigned), h->stream));
                 h->fractions_known = true;
             }
             CUDA_TRY(cudaGraphLaunch(h->cycle_graph[h->flip], h->stream));
             h->launches += h->cycle_graph_launches[h->flip];
-            if (h->alt_pool) {
+            if (h->dual()) {
                 for (int f : donor_fields(h)) std::swap(field_ptr(h, f), alt_ptr(h, f));
                 h->flip ^= 1;
                 h->volumes_only = true;
