@@ -117,7 +117,10 @@ typedef struct salec_material_desc {
     const double *xtem, *yden, *data;
 } salec_material_desc;
 
-/* Create a handle on the current CUDA device. mats has nmat entries (entry 0 unused). */
+/* Create a handle on the current CUDA device. mats has nmat entries (entry 0 unused). Beside its fields a
+ * handle keeps, where there is room, a second copy of the fields that advection moves (2 nmat + 8 planes,
+ * 3 nmat + 9 with porosity), which makes cycles faster. When the device is out of memory for anything a
+ * handle asks for, these copies are given up, the handle's own first and then other handles'. */
 int salec_gpu_create(const salec_run_desc *run, const salec_material_desc *mats, salec_gpu **out);
 int salec_gpu_destroy(salec_gpu *h);
 
@@ -151,9 +154,11 @@ int salec_gpu_step(salec_gpu *h, int nsteps);
 /* salec_gpu_step, then the per-cycle quantities of the reference's loop: dt and the simulated
  * time (the MIN-reduced ccl.dt and ccl.step_time, src/salec2d.c:167-168; either pointer may be
  * NULL) and, when profile is not NULL, the surface profile y_profile (the MIN-reduced
- * sale2d.y_profile, src/salec2d.c:120, 232; profile_n doubles, its field shape). The read-backs are queued
- * behind the cycles and the call synchronises once, where salec_gpu_get_scalar and
- * salec_gpu_get_field would synchronise once each. Results equal those calls'. */
+ * sale2d.y_profile, src/salec2d.c:120, 232; profile_n doubles, its field shape). One kernel behind the
+ * cycles writes them to page-locked memory of the handle. The call polls there for up to 2 ms, which
+ * keeps a host core busy, and then waits for the stream. When it returns, everything queued on the
+ * handle's stream before it is done. Results equal those of salec_gpu_get_scalar and salec_gpu_get_field,
+ * which synchronise once each. */
 int salec_gpu_step_report(salec_gpu *h, int nsteps, double *dt, double *time, double *profile, long long profile_n);
 /* The same, pipelined: queue nsteps cycles and the read-back of dt, time and (when profile is not
  * NULL) the surface profile into report slot `slot` (0 or 1), and return without waiting.
@@ -179,21 +184,27 @@ int salec_gpu_step_many(salec_gpu *const *handles, int n, int nsteps, int chunk)
  * energy, 11 tracers, 12 face fluxes (+ ghosts), 13 strength condition, 14 remap, damping,
  * ejecta drag and EOS, 15 cycle control. */
 int salec_gpu_phases(salec_gpu *h, int first, int last);
-/* Pick the block shape of every 2-D sweep for this handle's mesh: each candidate shape is
- * timed per phase over `cycles` cycles (after one warm-up cycle) from a device snapshot of the
+/* Pick the block shape of every 2-D sweep for this handle's mesh: each candidate shape (32x4, 32x8,
+ * 32x2) is timed per phase over `cycles` cycles (after one warm-up cycle) from a device snapshot of the
  * state, the fastest is kept per sweep, and the snapshot is restored, so the simulation is left
- * exactly where it was. The shape changes no result (one thread per point, exact reductions).
+ * exactly where it was. The shape changes no result (one thread per point, exact reductions). The
+ * sweeps that are timed are those of salec_gpu_phases; salec_gpu_step takes their shapes for its own
+ * forms of them, and has none of phases 4 and 10.
  * Takes a device copy of the field pool for its duration. If shapes is not NULL it receives 10
  * triples (phase, block x, block y). No counterpart in the reference. */
 int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes);
 /* Set the block shapes of the tunable 2-D sweeps from n triples (phase, block x, block y), as
  * salec_gpu_autotune returns them, e.g. to reuse one member's tuning for others of the same
  * mesh. Block x must be a multiple of 32 and x*y at most 256; any invalid triple rejects the
- * whole call (SALEC_ERR_ARG) with no shape changed. No counterpart in the reference. */
+ * whole call (SALEC_ERR_ARG) with no shape changed. A shape stands for its thread count: the sweeps
+ * run in blocks of 32 x r threads, r the largest of 1, 2, 4 and 8 with 32 r <= x*y (64x2 and 128x1 run
+ * as 32x4, 96x1 as 32x2). No counterpart in the reference. */
 int salec_gpu_set_block_shapes(salec_gpu *h, const int *shapes, int n);
 /* Block until the handle's stream is idle. */
 int salec_gpu_sync(salec_gpu *h);
-/* The CUDA stream (cudaStream_t) all work of the handle is queued on. */
+/* The CUDA stream (cudaStream_t) all work of the handle is queued on. A caller may capture salec_gpu_phases
+ * on it into a graph of its own; from the capture on the handle's cycles work in place and visit every
+ * cell, which is slower, as replays change the fields without the library knowing. */
 int salec_gpu_stream(salec_gpu *h, void **stream);
 /* Per-phase device timing: when enabled, every phase run is bracketed by CUDA events on the
  * handle's stream; salec_gpu_phase_times() waits for the stream and returns, per phase 0..15,

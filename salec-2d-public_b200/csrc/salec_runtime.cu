@@ -586,7 +586,8 @@ void allocate_donor_copy(salec_gpu *h)
     cudaMemsetAsync(h->alt_pool, 0, bytes, h->stream);
     // The quiet map needs a cycle whose vacuum is the same whatever the time step (count_quiet). Small
     // meshes fill the device for a moment only, whatever they visit, and looking the tile up costs
-    // them more than it saves (64x80: 81 us a cycle without, 86 with; 517x771: 194 and 184).
+    // them more than it saves (64x80: 81 us a cycle without, 86 with; 517x771: 194 and 184). Measured on single
+    // meshes, where latency counts; of members that fill the device together there is no figure.
     if (h->rp.damp_type == SALEC_DAMP_PML2 || (long long)h->d.enx * h->d.eny < SALEC_QUIET_MIN_CELLS ||
         !tiles_fit_a_list(h->tiles_x(), h->tiles_y()))
         return;
@@ -1684,7 +1685,8 @@ int salec_gpu_autotune(salec_gpu *h, int cycles, int *shapes)
     const auto lock = salec_internal_enter(h);
     // a shape stands for its thread count (launch_step_kernel). 32x1 is not offered: timed sweep by sweep
     // it ties with the others, but one block per row segment of a listed tile costs the cycle graph
-    // up to 30 us a sweep (2048x2048: 956-996 us a cycle with one sweep at 32x1, 920-930 without)
+    // 26 to 76 us for one sweep (2048x2048: 956-996 us a cycle with one sweep at 32x1, 920-930 without).
+    // What is timed is the phase-by-phase path's form of each sweep, whole mesh, in place
     static const dim3 cand[] = {dim3(32, 4), dim3(32, 8), dim3(32, 2)};
     constexpr int ncand = sizeof(cand) / sizeof(cand[0]);
     const int *tuned_phase = kTunedPhase;

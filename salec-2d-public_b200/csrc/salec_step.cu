@@ -44,7 +44,9 @@ __device__ __forceinline__ void grid_dependency()
 #define SALEC_REGS_FLUX 80
 #endif
 // the flux that stores volumes only (the cycle graph's): us at 2048x2048 FP64 with three materials,
-// layered 1024x1024 and 1536x1536 mixed: 104/54/58 at 64, 102/57/59 at 72, 110/57/62 at 80
+// layered 1024x1024 (four materials, porous) and 1536x1536 mixed (three): 104/54/58 at 64, 102/57/59 at 72,
+// 110/57/62 at 80. The other numbers of materials, and porosity or none with these, follow the nearest of
+// them unmeasured
 #ifndef SALEC_REGS_FLUX_VOLUMES
 #define SALEC_REGS_FLUX_VOLUMES (NM == 0 || NM >= 4 || sizeof(R) == 4 ? 64 : 72)
 #endif
@@ -54,7 +56,8 @@ __device__ __forceinline__ void grid_dependency()
 // the remap that reads its donors from the neighbours: 96 for up to three materials and the mixed
 // form, 112 for more in FP64 (2048x2048, three materials: 1243, 1214 and 1254 us a cycle at 80, 96
 // and 112; layered 1024x1024, four porous materials: 558, 507 and 493; layered 600x450 mixed: 210,
-// 192 and 202)
+// 192 and 202). Those are the measured instances: porosity with two or three materials, four materials
+// without it and five or more follow the nearest of them unmeasured
 #ifndef SALEC_REGS_REMAP_DUAL
 #define SALEC_REGS_REMAP_DUAL (NM == 2 || NM == 3 || sizeof(R) == 4 ? 96 : 112)
 #endif
@@ -1196,12 +1199,6 @@ __global__ void k_strength_condition(const CtxT<R> c)
 }
 
 // ============================================================ phase 12: face flux volumes
-// calculate_flux_mixed (src/advect.c:861-1136) with _calculate_flux_set_bphi (:1138-1223):
-// swept face volumes, geometric cut-line reconstruction of the primary material, algebraic
-// (MSTACS) fractions of the others, and the upwind state written on each outflow face.
-// A face with zero swept volume gets zero material volumes, which stands in for the
-// reference's clean_flux (src/advect.c:597-626): the other members of such a record are only
-// ever multiplied by those zero volumes.
 // The donor members of a face record, from the state `d` of cell p.
 template <class R, int NM, bool POR, class State>
 __device__ __forceinline__ void store_donor(const CtxT<R> &c, const State &d, double *f, long long p, int nmat)
@@ -1269,12 +1266,18 @@ __device__ __forceinline__ void cell_swept_volumes(const C &c, int i, int j, dou
     uv = swept_volume(px[3], py[3], px[2], py[2], dx[3], dy[3], dx[2], dy[2]);
 }
 
+// calculate_flux_mixed (src/advect.c:861-1136) with _calculate_flux_set_bphi (:1138-1223):
+// swept face volumes, geometric cut-line reconstruction of the primary material, algebraic
+// (MSTACS) fractions of the others, and the upwind state written on each outflow face.
+// A face with zero swept volume gets zero material volumes, which stands in for the
+// reference's clean_flux (src/advect.c:597-626): the other members of such a record are only
+// ever multiplied by those zero volumes.
 // Every cell in one launch, after the ghost fills: no interior cell's flux reads a ghost member that
 // the fills write, and no flux writes what the fills read, so this computes what the reference's
 // interior pass, ghost update and pad pass compute, and the pad cells hide in the interior's waves.
-// The first `tracer_blocks` blocks (rows of blocks, on a two-dimensional grid) move the tracers instead (they read nothing the fluxes write and
-// write only tracer arrays), so that their chain of dependent loads runs beside the fluxes: as a
-// launch of their own they cost 41 us of the 2048x2048 impact's cycle.
+// The first `tracer_blocks` blocks (rows of blocks, on a two-dimensional grid) move the tracers instead:
+// they read nothing the fluxes write and write only tracer arrays, so that their chain of dependent loads
+// runs beside the fluxes. As a launch of their own they cost 41 us of the 2048x2048 impact's cycle.
 template <class R, int NM, bool POR, bool REC = true>
 __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int tracer_blocks)
 {
@@ -2215,7 +2218,7 @@ __device__ __forceinline__ void edge_copy(const EdgeField &f, const EdgeEntry &e
 
 // One lane per entry. A batch takes a few microseconds whatever its size: a launch, the entry, its
 // sources. One thread per component, walking up to 16 entries through index arrays, took 2-3 us
-// more (64x80: 35 us a cycle in eight batches, 12 in the five that are left).
+// more (64x80: 35 us a cycle in eight batches; the six that are left take 2.4 to 3.2 us each at 200x400).
 __global__ void __launch_bounds__(256) k_edges(const __grid_constant__ EdgeBatch g)
 {
     grid_dependency();
