@@ -427,9 +427,9 @@ __global__ void SALEC_BOUNDS_VOFMOM k_vertex_vof_momentum(const CtxT<R> c)
 {
     grid_dependency();
     for_points<true>(c, 0, [&](int i, int j) {
-    if (!vert_active(c, i, j)) return;
-    vertex_vof(c, i, j);
-    vertex_momentum(c, i, j);
+        if (!vert_active(c, i, j)) return;
+        vertex_vof(c, i, j);
+        vertex_momentum(c, i, j);
     });
 }
 
@@ -440,38 +440,38 @@ __global__ void k_cell_velocity(const CtxT<R> c)
 {
     grid_dependency();
     for_points<true>(c, 0, [&](int i, int j) {
-    if (!cell_interior(c, i, j)) return;
-    const long long p = KIDX(i, j);
-    const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
-    double ex = 0., ey = 0.;
-    const double rho = c.f.e_den[p];
-    if (!(rho < SALEC_TOLRHO)) {
-        int vac = 0;
-        double wpt[4];
-        for (int k = 0; k < 4; ++k) {
-            wpt[k] = PLN(c.f.e_wpt, k)[p];
-            const double nvoid = PLN(c.f.v_mass, 1)[vl[k]];
-            if (nvoid >= 4.0 || (nvoid >= 3.0 && wpt[k] < 0.)) vac++;
-        }
-        if (vac != 4) {
-            double sm = 0.;
+        if (!cell_interior(c, i, j)) return;
+        const long long p = KIDX(i, j);
+        const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
+        double ex = 0., ey = 0.;
+        const double rho = c.f.e_den[p];
+        if (!(rho < SALEC_TOLRHO)) {
+            int vac = 0;
+            double wpt[4];
             for (int k = 0; k < 4; ++k) {
-                if (wpt[k] > 0.0 || rho < SALEC_TOLRHO) continue;
-                const double mk = c.f.v_mass[vl[k]];
-                ex += mk * c.f.v_vel[vl[k]];
-                ey += mk * PLN(c.f.v_vel, 1)[vl[k]];
-                sm += mk;
+                wpt[k] = PLN(c.f.e_wpt, k)[p];
+                const double nvoid = PLN(c.f.v_mass, 1)[vl[k]];
+                if (nvoid >= 4.0 || (nvoid >= 3.0 && wpt[k] < 0.)) vac++;
             }
-            if (sm > 0.) {
-                const double s = 1.0 / sm;
-                ex *= s; ey *= s;
-            } else {
-                ex = 0.; ey = 0.;
+            if (vac != 4) {
+                double sm = 0.;
+                for (int k = 0; k < 4; ++k) {
+                    if (wpt[k] > 0.0 || rho < SALEC_TOLRHO) continue;
+                    const double mk = c.f.v_mass[vl[k]];
+                    ex += mk * c.f.v_vel[vl[k]];
+                    ey += mk * PLN(c.f.v_vel, 1)[vl[k]];
+                    sm += mk;
+                }
+                if (sm > 0.) {
+                    const double s = 1.0 / sm;
+                    ex *= s; ey *= s;
+                } else {
+                    ex = 0.; ey = 0.;
+                }
             }
         }
-    }
-    c.f.e_vel[p] = ex;
-    PLN(c.f.e_vel, 1)[p] = ey;
+        c.f.e_vel[p] = ex;
+        PLN(c.f.e_vel, 1)[p] = ey;
     });
 }
 
@@ -533,65 +533,65 @@ __global__ void SALEC_BOUNDS_GRAD k_gradient_viscosity_cfl(const CtxT<R> c)
     using A = R;   // arithmetic of the gradient and the viscosity: FP64, or FP32 in the mixed form
     unsigned long long cand = ~0ULL;
     for_points<VOID>(c, 0, [&](int i, int j) {
-    if (VOID && vert_active(c, i, j)) {
-        const long long p = KIDX(i, j);
-        double x, y;
-        if (void_velocity(c, i, j, PLN(c.f.v_mass, 1)[p], x, y)) {
-            c.f.v_vel[p] = x;
-            PLN(c.f.v_vel, 1)[p] = y;
-        }
-    }
-    if (cell_interior(c, i, j)) {
-        const long long p = KIDX(i, j);
-        const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
-        A vx[4], vy[4];
-        for (int k = 0; k < 4; ++k) { vx[k] = c.f.v_vel[vl[k]]; vy[k] = PLN(c.f.v_vel, 1)[vl[k]]; }
-        if (VOID) {
-            R corners[4];
-            for (int k = 0; k < 4; ++k) corners[k] = PLN(c.f.v_mass, 1)[vl[k]];
-            for (int k = 0; k < 4; ++k) {
-                double x, y;
-                const int di = k == 1 || k == 2, dj = k >= 2;
-                if (void_velocity(c, i + di, j + dj, corners[k], x, y)) { vx[k] = R(x); vy[k] = R(y); }
+        if (VOID && vert_active(c, i, j)) {
+            const long long p = KIDX(i, j);
+            double x, y;
+            if (void_velocity(c, i, j, PLN(c.f.v_mass, 1)[p], x, y)) {
+                c.f.v_vel[p] = x;
+                PLN(c.f.v_vel, 1)[p] = y;
             }
         }
-        A g[12];
-        for (int k = 0; k < 12; ++k) g[k] = GEO(c.g_e_grad, k);
-        A d0 = A(0.), d1 = A(0.), d2 = A(0.), d3 = A(0.), d4 = A(0.);
-        for (int k = 0; k < 4; ++k) d0 += g[k] * vx[k];        // dv_r/dr
-        for (int k = 0; k < 4; ++k) d2 += g[k] * vy[k];        // dv_z/dr
-        for (int k = 0; k < 4; ++k) d1 += g[4 + k] * vx[k];    // dv_r/dz
-        for (int k = 0; k < 4; ++k) d3 += g[4 + k] * vy[k];    // dv_z/dz
-        for (int k = 0; k < 4; ++k) d4 += g[8 + k] * vx[k];    // v_r/r
-        PLN(c.f.e_grad_vel, 0)[p] = d0;
-        PLN(c.f.e_grad_vel, 1)[p] = d1;
-        PLN(c.f.e_grad_vel, 2)[p] = d2;
-        PLN(c.f.e_grad_vel, 3)[p] = d3;
-        PLN(c.f.e_grad_vel, 4)[p] = d4;
-        const A div = d0 + d3 + d4;
-        c.f.e_div_vel[p] = div;
-        const double vof0 = c.f.m_vof[p];
-        const A csd = c.f.e_csd[p];
-        A q;
-        if (vof0 > SALEC_TOLVOF || c.f.e_pre[p] <= A(0.0)) {
-            q = A(0.);
-        } else {
-            double aread = GEO(c.g_e_vol, 0) / c.f.e_pos[p];
-            const A area = A(fabs(aread));
-            const A ql = A(c.rp.avis1) * csd * sqrt(area);
-            const A qq = A(c.rp.avis2) * div * area;
-            q = amin(A(0.), div) * A(c.f.e_den[p]) * (qq - ql);
-            if (q < A(SALEC_TOLQPRE)) q = A(0.);
+        if (cell_interior(c, i, j)) {
+            const long long p = KIDX(i, j);
+            const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
+            A vx[4], vy[4];
+            for (int k = 0; k < 4; ++k) { vx[k] = c.f.v_vel[vl[k]]; vy[k] = PLN(c.f.v_vel, 1)[vl[k]]; }
+            if (VOID) {
+                R corners[4];
+                for (int k = 0; k < 4; ++k) corners[k] = PLN(c.f.v_mass, 1)[vl[k]];
+                for (int k = 0; k < 4; ++k) {
+                    double x, y;
+                    const int di = k == 1 || k == 2, dj = k >= 2;
+                    if (void_velocity(c, i + di, j + dj, corners[k], x, y)) { vx[k] = R(x); vy[k] = R(y); }
+                }
+            }
+            A g[12];
+            for (int k = 0; k < 12; ++k) g[k] = GEO(c.g_e_grad, k);
+            A d0 = A(0.), d1 = A(0.), d2 = A(0.), d3 = A(0.), d4 = A(0.);
+            for (int k = 0; k < 4; ++k) d0 += g[k] * vx[k];        // dv_r/dr
+            for (int k = 0; k < 4; ++k) d2 += g[k] * vy[k];        // dv_z/dr
+            for (int k = 0; k < 4; ++k) d1 += g[4 + k] * vx[k];    // dv_r/dz
+            for (int k = 0; k < 4; ++k) d3 += g[4 + k] * vy[k];    // dv_z/dz
+            for (int k = 0; k < 4; ++k) d4 += g[8 + k] * vx[k];    // v_r/r
+            PLN(c.f.e_grad_vel, 0)[p] = d0;
+            PLN(c.f.e_grad_vel, 1)[p] = d1;
+            PLN(c.f.e_grad_vel, 2)[p] = d2;
+            PLN(c.f.e_grad_vel, 3)[p] = d3;
+            PLN(c.f.e_grad_vel, 4)[p] = d4;
+            const A div = d0 + d3 + d4;
+            c.f.e_div_vel[p] = div;
+            const double vof0 = c.f.m_vof[p];
+            const A csd = c.f.e_csd[p];
+            A q;
+            if (vof0 > SALEC_TOLVOF || c.f.e_pre[p] <= A(0.0)) {
+                q = A(0.);
+            } else {
+                double aread = GEO(c.g_e_vol, 0) / c.f.e_pos[p];
+                const A area = A(fabs(aread));
+                const A ql = A(c.rp.avis1) * csd * sqrt(area);
+                const A qq = A(c.rp.avis2) * div * area;
+                q = amin(A(0.), div) * A(c.f.e_den[p]) * (qq - ql);
+                if (q < A(SALEC_TOLQPRE)) q = A(0.);
+            }
+            c.f.e_q[p] = q;
+            // CFL candidate over cells that are not pure vacuum, in FP64; a NaN candidate is recorded
+            // by its position in the reference's traversal order instead (see k_finalize_dt)
+            if (!(vof0 > 1.0 - SALEC_TOLVOF)) {
+                const double dt_rz = cfl_candidate(c, p, (double)csd);
+                if (dt_rz == dt_rz) cand = min(cand, ord_encode(dt_rz));
+                else atomicMax(&c.scal->dt_nan_last, (long long)j * c.d.enx + i);
+            }
         }
-        c.f.e_q[p] = q;
-        // CFL candidate over cells that are not pure vacuum, in FP64; a NaN candidate is recorded
-        // by its position in the reference's traversal order instead (see k_finalize_dt)
-        if (!(vof0 > 1.0 - SALEC_TOLVOF)) {
-            const double dt_rz = cfl_candidate(c, p, (double)csd);
-            if (dt_rz == dt_rz) cand = min(cand, ord_encode(dt_rz));
-            else atomicMax(&c.scal->dt_nan_last, (long long)j * c.d.enx + i);
-        }
-    }
     });
     // block MIN, one atomic per block
     for (int o = 16; o > 0; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
@@ -694,204 +694,204 @@ __global__ void SALEC_BOUNDS_STRESS k_stress(const CtxT<R> c)
     using A = R;   // arithmetic of stress, strength and damage: FP64, or FP32 in the mixed form
     constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
     for_points<false>(c, 0, [&](int i, int j) {
-    if (!cell_interior(c, i, j)) return;
-    const long long p = KIDX(i, j);
-    const int nmat = NM > 0 ? NM : c.d.nmat;
-    const A dt = A(c.scal->dt);
-    const double vof0 = c.f.m_vof[p];
-    A dam = c.f.e_dam[p];
+        if (!cell_interior(c, i, j)) return;
+        const long long p = KIDX(i, j);
+        const int nmat = NM > 0 ? NM : c.d.nmat;
+        const A dt = A(c.scal->dt);
+        const double vof0 = c.f.m_vof[p];
+        A dam = c.f.e_dam[p];
 
-    // --- acoustic fluidisation (block model)
-    if (c.rp.acoustic_fluid) {
-        A vib = c.f.e_vib[p];
-        if (vof0 > SALEC_TOLVOF || dam < A(0.5)) {
-            vib = A(0.);
-        } else {
-            A tdec = A(-1.0), cvib = A(0.0), toff = A(-1.0), vmax = A(0.0), pvl = A(0.0);
-            for (int m = 1; m < nmat; ++m) {
-                if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
-                const DevMat &s = c.mat[m];
-                tdec = amax(A(s.Tdamp), tdec);
-                cvib = amax(A(s.Cvib), cvib);
-                toff = amax(A(s.Toff), toff);
-                vmax = amax(A(s.VibMax), vmax);
-                pvl = amax(A(s.Pvlim), pvl);
-            }
-            if (tdec <= A(0.) || toff <= A(0.)) {
+        // --- acoustic fluidisation (block model)
+        if (c.rp.acoustic_fluid) {
+            A vib = c.f.e_vib[p];
+            if (vof0 > SALEC_TOLVOF || dam < A(0.5)) {
                 vib = A(0.);
             } else {
-                const A evx = c.f.e_vel[p], evy = PLN(c.f.e_vel, 1)[p];
-                A len = A(0.);
-                len += evx * evx;
-                len += evy * evy;
-                const A nv = cvib * sqrt(len);
-                const A nv2 = nv * nv;
-                const A t = A(c.scal->time);
-                if ((t <= toff) && (nv2 >= vib) && (nv >= A(1.0)) && (c.f.e_q[p] > A(0.)))
-                    vib = amin(nv2, vmax * vmax);
-                else
-                    vib = amax(vib * (A(1.0) - A(2.0) * dt / tdec + A(2.0) * (dt / tdec) * (dt / tdec)), A(0.0));
+                A tdec = A(-1.0), cvib = A(0.0), toff = A(-1.0), vmax = A(0.0), pvl = A(0.0);
+                for (int m = 1; m < nmat; ++m) {
+                    if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
+                    const DevMat &s = c.mat[m];
+                    tdec = amax(A(s.Tdamp), tdec);
+                    cvib = amax(A(s.Cvib), cvib);
+                    toff = amax(A(s.Toff), toff);
+                    vmax = amax(A(s.VibMax), vmax);
+                    pvl = amax(A(s.Pvlim), pvl);
+                }
+                if (tdec <= A(0.) || toff <= A(0.)) {
+                    vib = A(0.);
+                } else {
+                    const A evx = c.f.e_vel[p], evy = PLN(c.f.e_vel, 1)[p];
+                    A len = A(0.);
+                    len += evx * evx;
+                    len += evy * evy;
+                    const A nv = cvib * sqrt(len);
+                    const A nv2 = nv * nv;
+                    const A t = A(c.scal->time);
+                    if ((t <= toff) && (nv2 >= vib) && (nv >= A(1.0)) && (c.f.e_q[p] > A(0.)))
+                        vib = amin(nv2, vmax * vmax);
+                    else
+                        vib = amax(vib * (A(1.0) - A(2.0) * dt / tdec + A(2.0) * (dt / tdec) * (dt / tdec)), A(0.0));
+                }
             }
+            c.f.e_vib[p] = vib;
         }
-        c.f.e_vib[p] = vib;
-    }
 
-    // --- stress update
-    if (vof0 > SALEC_TOLVOF) {
-        c.f.e_ste[p] = 0.; PLN(c.f.e_ste, 1)[p] = 0.; PLN(c.f.e_ste, 2)[p] = 0.; PLN(c.f.e_ste, 3)[p] = 0.;
-        c.f.e_ste2s[p] = 0.; c.f.e_sta2s[p] = 0.; c.f.e_strength[p] = 0.;
-        return;
-    }
-    // every input of a full cell, issued in one batch
-    A s0 = c.f.e_ste[p], s1 = PLN(c.f.e_ste, 1)[p], s2 = PLN(c.f.e_ste, 2)[p], s3 = PLN(c.f.e_ste, 3)[p];
-    A ste2s = c.f.e_ste2s[p], sta2s = c.f.e_sta2s[p], tps = c.f.e_tps[p], strength = c.f.e_strength[p];
-    A vmat[MM], ptm[MM];
-    #pragma unroll
-    for (int m = 1; m < nmat; ++m) {
-        vmat[m] = A(PLN(c.f.m_vof, m)[p]);
-        ptm[m] = POR ? A(PLN(c.f.m_pty, m)[p]) : A(1.0);
-    }
-    const A rho = c.f.e_den[p];
-    const A g0 = c.f.e_grad_vel[p], g1 = PLN(c.f.e_grad_vel, 1)[p], g2 = PLN(c.f.e_grad_vel, 2)[p],
-            g3 = PLN(c.f.e_grad_vel, 3)[p], g4 = PLN(c.f.e_grad_vel, 4)[p];
-    const A mu = c.f.e_mu[p];
-    const A pre = c.f.e_pre[p], tem = c.f.e_tem[p], csd = c.f.e_csd[p];
-    A vapor_ref = A(0.), melt_ref = A(0.);
-    #pragma unroll
-    for (int m = 1; m < nmat; ++m) {
-        const A vm = vmat[m];
-        if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
-        vapor_ref += vm * A(c.mat[m].VaporDen);
-        melt_ref += vm * A(c.mat[m].MeltDen);
-    }
-    A porosity = A(0.0);
-    if (POR) {
-        A mv = A(0.0);
+        // --- stress update
+        if (vof0 > SALEC_TOLVOF) {
+            c.f.e_ste[p] = 0.; PLN(c.f.e_ste, 1)[p] = 0.; PLN(c.f.e_ste, 2)[p] = 0.; PLN(c.f.e_ste, 3)[p] = 0.;
+            c.f.e_ste2s[p] = 0.; c.f.e_sta2s[p] = 0.; c.f.e_strength[p] = 0.;
+            return;
+        }
+        // every input of a full cell, issued in one batch
+        A s0 = c.f.e_ste[p], s1 = PLN(c.f.e_ste, 1)[p], s2 = PLN(c.f.e_ste, 2)[p], s3 = PLN(c.f.e_ste, 3)[p];
+        A ste2s = c.f.e_ste2s[p], sta2s = c.f.e_sta2s[p], tps = c.f.e_tps[p], strength = c.f.e_strength[p];
+        A vmat[MM], ptm[MM];
+        #pragma unroll
+        for (int m = 1; m < nmat; ++m) {
+            vmat[m] = A(PLN(c.f.m_vof, m)[p]);
+            ptm[m] = POR ? A(PLN(c.f.m_pty, m)[p]) : A(1.0);
+        }
+        const A rho = c.f.e_den[p];
+        const A g0 = c.f.e_grad_vel[p], g1 = PLN(c.f.e_grad_vel, 1)[p], g2 = PLN(c.f.e_grad_vel, 2)[p],
+                g3 = PLN(c.f.e_grad_vel, 3)[p], g4 = PLN(c.f.e_grad_vel, 4)[p];
+        const A mu = c.f.e_mu[p];
+        const A pre = c.f.e_pre[p], tem = c.f.e_tem[p], csd = c.f.e_csd[p];
+        A vapor_ref = A(0.), melt_ref = A(0.);
         #pragma unroll
         for (int m = 1; m < nmat; ++m) {
             const A vm = vmat[m];
             if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
-            porosity += vm * ptm[m];
-            mv += vm;
+            vapor_ref += vm * A(c.mat[m].VaporDen);
+            melt_ref += vm * A(c.mat[m].MeltDen);
         }
-        porosity /= mv;
-    } else {
-        porosity = A(1.0);
-    }
-    porosity = amax(porosity, A(1.0));
-    vapor_ref /= porosity;
-    melt_ref /= porosity;
-
-    const A ste2s_old = ste2s;
-    int state; // 0 solid, 1 melt, 2 vapour
-    if (rho <= vapor_ref) {
-        state = 2;
-        s0 = s1 = s2 = s3 = A(0.);
-        ste2s = A(0.);
-        tps = A(0.);
-        dam = A(0.);
-        strength = A(0.);
-    } else {
-        A e0 = g0, e1 = A(0.5) * g1 + A(0.5) * g2, e2 = g3, e3 = g4;
-        const A tr = e0 + e2 + e3;
-        e0 -= tr / A(3.0);
-        e2 -= tr / A(3.0);
-        e3 -= tr / A(3.0);
-        if (rho <= melt_ref) {
-            state = 1;
-            s0 = s1 = s2 = s3 = A(0.);
-            ste2s = A(0.);
-            sta2s = sqrt(second_inv(e0, e1, e2, e3));
-            tps = amin(tps + sta2s * dt, A(10.));
-            dam = A(1.);
-            strength = A(0.);
-        } else {
-            state = 0;
-            // Wilkins rotation
-            A sin2o = (g2 - g1) * dt;
-            sin2o = awind(sin2o, A(-1.), A(1.));
-            const A cos2o1 = sqrt(A(1.0) - sin2o * sin2o) - A(1.0);
-            const A ss2 = (s0 - s2) / A(2.0);
-            const A r0 = ss2 * cos2o1 + s1 * sin2o;
-            const A r1 = s1 * cos2o1 - ss2 * sin2o;
-            const A r2 = -ss2 * cos2o1 - s1 * sin2o;
-            s0 += A(1.0) * r0; s1 += A(1.0) * r1; s2 += A(1.0) * r2; s3 += A(1.0) * A(0.0);
-            const A k2 = A(2.0) * mu * dt;
-            s0 += k2 * e0; s1 += k2 * e1; s2 += k2 * e2; s3 += k2 * e3;
-            ste2s = sqrt(second_inv(s0, s1, s2, s3));
-            sta2s = sqrt(second_inv(e0, e1, e2, e3));
-        }
-    }
-
-    if (state == 2) {
-        dam = A(0.);
-    } else if (state == 1) {
-        dam = A(1.0);
-    } else {
-        A shear = A(0.0), tensile = A(0.);
-        #pragma unroll
-        for (int m = 1; m < nmat; ++m) {
-            const A vm = vmat[m];
-            if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
-            const DevMat &s = c.mat[m];
-            A my = strength_fn<A>(s.yfunc, pre, dam, tps, sta2s, tem, A(0.), s);
-            if (c.rp.acoustic_fluid && pre >= A(0.)) {
-                const A vibp = amin(rho * csd * sqrt(A(c.f.e_vib[p])), pre);
-                const A tm = simon_melt<A>(pre, s);
-                A soft = ohnaka_soft<A>(tem, s, tm);
-                soft = awind(soft, A(0.0), A(1.0));
-                const A lp = pre - vibp * dam * dam * sqrt(soft);
-                const A myv = strength_fn<A>(s.yfunc, lp, dam, tps, sta2s, tem, A(0.), s) + rho * A(s.Acvis) * sta2s;
-                my = amin(myv, my);
-            }
-            shear += vm * amax(my, A(0.0));
-            if (c.rp.tensile_failure) tensile += vm * strength_fn<A>(s.tfunc, pre, dam, tps, sta2s, tem, A(0.), s);
-        }
-        if (c.rp.tracer_lubrication >= 1 && c.f.e_cnd[p] >= A(1.0)) {
-            const A lub = amin(pre * A(c.rp.tracer_lub_frac) + A(c.rp.tracer_lub_y0), A(0.0));
-            shear = amin(shear, lub);
-        }
-        strength = shear;
-        if (shear < ste2s) {
-            sta2s = sta2s / amax(A(0.5), (ste2s - ste2s_old) / (ste2s - shear));
-            const A sfac = shear / ste2s;
-            s0 *= sfac; s1 *= sfac; s2 *= sfac; s3 *= sfac;
-            ste2s = shear;
-            A dsd = A(0.);
+        A porosity = A(0.0);
+        if (POR) {
+            A mv = A(0.0);
             #pragma unroll
             for (int m = 1; m < nmat; ++m) {
+                const A vm = vmat[m];
+                if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
+                porosity += vm * ptm[m];
+                mv += vm;
+            }
+            porosity /= mv;
+        } else {
+            porosity = A(1.0);
+        }
+        porosity = amax(porosity, A(1.0));
+        vapor_ref /= porosity;
+        melt_ref /= porosity;
+
+        const A ste2s_old = ste2s;
+        int state; // 0 solid, 1 melt, 2 vapour
+        if (rho <= vapor_ref) {
+            state = 2;
+            s0 = s1 = s2 = s3 = A(0.);
+            ste2s = A(0.);
+            tps = A(0.);
+            dam = A(0.);
+            strength = A(0.);
+        } else {
+            A e0 = g0, e1 = A(0.5) * g1 + A(0.5) * g2, e2 = g3, e3 = g4;
+            const A tr = e0 + e2 + e3;
+            e0 -= tr / A(3.0);
+            e2 -= tr / A(3.0);
+            e3 -= tr / A(3.0);
+            if (rho <= melt_ref) {
+                state = 1;
+                s0 = s1 = s2 = s3 = A(0.);
+                ste2s = A(0.);
+                sta2s = sqrt(second_inv(e0, e1, e2, e3));
+                tps = amin(tps + sta2s * dt, A(10.));
+                dam = A(1.);
+                strength = A(0.);
+            } else {
+                state = 0;
+                // Wilkins rotation
+                A sin2o = (g2 - g1) * dt;
+                sin2o = awind(sin2o, A(-1.), A(1.));
+                const A cos2o1 = sqrt(A(1.0) - sin2o * sin2o) - A(1.0);
+                const A ss2 = (s0 - s2) / A(2.0);
+                const A r0 = ss2 * cos2o1 + s1 * sin2o;
+                const A r1 = s1 * cos2o1 - ss2 * sin2o;
+                const A r2 = -ss2 * cos2o1 - s1 * sin2o;
+                s0 += A(1.0) * r0; s1 += A(1.0) * r1; s2 += A(1.0) * r2; s3 += A(1.0) * A(0.0);
+                const A k2 = A(2.0) * mu * dt;
+                s0 += k2 * e0; s1 += k2 * e1; s2 += k2 * e2; s3 += k2 * e3;
+                ste2s = sqrt(second_inv(s0, s1, s2, s3));
+                sta2s = sqrt(second_inv(e0, e1, e2, e3));
+            }
+        }
+
+        if (state == 2) {
+            dam = A(0.);
+        } else if (state == 1) {
+            dam = A(1.0);
+        } else {
+            A shear = A(0.0), tensile = A(0.);
+            #pragma unroll
+            for (int m = 1; m < nmat; ++m) {
+                const A vm = vmat[m];
+                if (PLN(c.f.m_vof, m)[p] < SALEC_TOLVOF) continue;
                 const DevMat &s = c.mat[m];
-                dsd += vmat[m] * strength_fn<A>(s.dsdf, pre, dam, A(0.), A(0.), A(0.), A(0.), s);
+                A my = strength_fn<A>(s.yfunc, pre, dam, tps, sta2s, tem, A(0.), s);
+                if (c.rp.acoustic_fluid && pre >= A(0.)) {
+                    const A vibp = amin(rho * csd * sqrt(A(c.f.e_vib[p])), pre);
+                    const A tm = simon_melt<A>(pre, s);
+                    A soft = ohnaka_soft<A>(tem, s, tm);
+                    soft = awind(soft, A(0.0), A(1.0));
+                    const A lp = pre - vibp * dam * dam * sqrt(soft);
+                    const A myv = strength_fn<A>(s.yfunc, lp, dam, tps, sta2s, tem, A(0.), s) + rho * A(s.Acvis) * sta2s;
+                    my = amin(myv, my);
+                }
+                shear += vm * amax(my, A(0.0));
+                if (c.rp.tensile_failure) tensile += vm * strength_fn<A>(s.tfunc, pre, dam, tps, sta2s, tem, A(0.), s);
             }
-            dam = awind(dam + sta2s * dsd * dt, A(0.0), A(1.0));
-            tps = amin(tps + sta2s * dt, A(10.));
-        }
-        if (c.rp.tensile_failure) {
-            const A sxx = s0, szz = s2, sxz = s1, sth = s3;
-            const A ts = sqrt(sxz * sxz + A(0.25) * (sxx - szz) * (sxx - szz));
-            A tmax = amax(A(0.5) * (sxx + szz) - ts, A(0.5) * (sxx + szz) + ts);
-            tmax = amax(tmax, sth);
-            if ((tmax - pre) > tensile) {
-                // the reference divides by Min(e_pos[1], e_pos[2]) (centre y and scale x)
-                const A dinc = A(0.4) * csd / A(dmin(PLN(c.f.e_pos, 1)[p], PLN(c.f.e_pos, 2)[p]));
-                const A dold = dam;
-                A third = pow(dold, A(1.0 / 3.));
-                third += dinc;
-                dam = awind(pow(third, A(3.0)), A(0.), A(1.));
-                const A sfac = dold < A(0.98) ? (A(1.0) - dam) / (A(1.0) - dold) : A(0.0);
+            if (c.rp.tracer_lubrication >= 1 && c.f.e_cnd[p] >= A(1.0)) {
+                const A lub = amin(pre * A(c.rp.tracer_lub_frac) + A(c.rp.tracer_lub_y0), A(0.0));
+                shear = amin(shear, lub);
+            }
+            strength = shear;
+            if (shear < ste2s) {
+                sta2s = sta2s / amax(A(0.5), (ste2s - ste2s_old) / (ste2s - shear));
+                const A sfac = shear / ste2s;
                 s0 *= sfac; s1 *= sfac; s2 *= sfac; s3 *= sfac;
-                ste2s *= sfac;
+                ste2s = shear;
+                A dsd = A(0.);
+                #pragma unroll
+                for (int m = 1; m < nmat; ++m) {
+                    const DevMat &s = c.mat[m];
+                    dsd += vmat[m] * strength_fn<A>(s.dsdf, pre, dam, A(0.), A(0.), A(0.), A(0.), s);
+                }
+                dam = awind(dam + sta2s * dsd * dt, A(0.0), A(1.0));
+                tps = amin(tps + sta2s * dt, A(10.));
+            }
+            if (c.rp.tensile_failure) {
+                const A sxx = s0, szz = s2, sxz = s1, sth = s3;
+                const A ts = sqrt(sxz * sxz + A(0.25) * (sxx - szz) * (sxx - szz));
+                A tmax = amax(A(0.5) * (sxx + szz) - ts, A(0.5) * (sxx + szz) + ts);
+                tmax = amax(tmax, sth);
+                if ((tmax - pre) > tensile) {
+                    // the reference divides by Min(e_pos[1], e_pos[2]) (centre y and scale x)
+                    const A dinc = A(0.4) * csd / A(dmin(PLN(c.f.e_pos, 1)[p], PLN(c.f.e_pos, 2)[p]));
+                    const A dold = dam;
+                    A third = pow(dold, A(1.0 / 3.));
+                    third += dinc;
+                    dam = awind(pow(third, A(3.0)), A(0.), A(1.));
+                    const A sfac = dold < A(0.98) ? (A(1.0) - dam) / (A(1.0) - dold) : A(0.0);
+                    s0 *= sfac; s1 *= sfac; s2 *= sfac; s3 *= sfac;
+                    ste2s *= sfac;
+                }
             }
         }
-    }
-    c.f.e_ste[p] = s0; PLN(c.f.e_ste, 1)[p] = s1; PLN(c.f.e_ste, 2)[p] = s2; PLN(c.f.e_ste, 3)[p] = s3;
-    c.f.e_ste2s[p] = ste2s;
-    c.f.e_sta2s[p] = sta2s;
-    c.f.e_tps[p] = tps;
-    c.f.e_dam[p] = dam;
-    c.f.e_strength[p] = strength;
-    if (EN && !(rho < SALEC_TOLRHO))
-        energy_cell<R, NM, POR>(c, p, R(s0), R(s1), R(s2), R(s3), g0, g1, g2, g3, g4, pre);
+        c.f.e_ste[p] = s0; PLN(c.f.e_ste, 1)[p] = s1; PLN(c.f.e_ste, 2)[p] = s2; PLN(c.f.e_ste, 3)[p] = s3;
+        c.f.e_ste2s[p] = ste2s;
+        c.f.e_sta2s[p] = sta2s;
+        c.f.e_tps[p] = tps;
+        c.f.e_dam[p] = dam;
+        c.f.e_strength[p] = strength;
+        if (EN && !(rho < SALEC_TOLRHO))
+            energy_cell<R, NM, POR>(c, p, R(s0), R(s1), R(s2), R(s3), g0, g1, g2, g3, g4, pre);
     });
 }
 
@@ -905,104 +905,104 @@ __global__ void SALEC_BOUNDS_ACCEL k_vertex_acceleration(const CtxT<R> c)
     grid_dependency();
     using A = R;   // arithmetic of the stress divergence: FP64, or FP32 in the mixed form
     for_points<false>(c, 0, [&](int i, int j) {
-    if (!vert_active(c, i, j)) return;
-    const long long p = KIDX(i, j);
-    const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
-    const bool pml = (c.rp.damp_type == 1 || c.rp.damp_type == 2);
-    const A dt = A(c.scal->dt);
-    A ax = A(0.), ay = A(0.), vmass = A(0.), vvol = A(0.);
-    A sub[4];
-    for (int k = 0; k < 4; ++k) sub[k] = GEO(c.g_v_subvol, k);
-    A sigx = A(0.), sigy = A(0.);
-    A alx = A(0.), aly = A(0.);
-    if (pml) {
+        if (!vert_active(c, i, j)) return;
+        const long long p = KIDX(i, j);
+        const long long cl[4] = {KIDX(i - 1, j - 1), KIDX(i, j - 1), KIDX(i, j), KIDX(i - 1, j)};
+        const bool pml = (c.rp.damp_type == 1 || c.rp.damp_type == 2);
+        const A dt = A(c.scal->dt);
+        A ax = A(0.), ay = A(0.), vmass = A(0.), vvol = A(0.);
+        A sub[4];
+        for (int k = 0; k < 4; ++k) sub[k] = GEO(c.g_v_subvol, k);
+        A sigx = A(0.), sigy = A(0.);
+        A alx = A(0.), aly = A(0.);
+        if (pml) {
+            for (int k = 0; k < 4; ++k) {
+                sigx += A(0.25) * A(c.f.e_sigma[cl[k]]);
+                sigy += A(0.25) * A(PLN(c.f.e_sigma, 1)[cl[k]]);
+            }
+            alx = c.f.v_alpha[p];
+            aly = PLN(c.f.v_alpha, 1)[p];
+        }
+        const bool damped = pml && (sigx > A(0.) || sigy > A(0.));
         for (int k = 0; k < 4; ++k) {
-            sigx += A(0.25) * A(c.f.e_sigma[cl[k]]);
-            sigy += A(0.25) * A(PLN(c.f.e_sigma, 1)[cl[k]]);
-        }
-        alx = c.f.v_alpha[p];
-        aly = PLN(c.f.v_alpha, 1)[p];
-    }
-    const bool damped = pml && (sigx > A(0.) || sigy > A(0.));
-    for (int k = 0; k < 4; ++k) {
-        const long long e = cl[k];
-        const A sfx = GEO(c.g_v_suf, 2 * k), sfy = GEO(c.g_v_suf, 2 * k + 1);
-        const A lp = A(c.f.e_pre[e]) + A(c.f.e_q[e]);
-        const A ste0 = c.f.e_ste[e], ste1 = PLN(c.f.e_ste, 1)[e], ste2 = PLN(c.f.e_ste, 2)[e],
-                ste3 = PLN(c.f.e_ste, 3)[e];
-        if (!pml) {
-            A fpx = A(0.), fpy = A(0.);
-            fpx += lp * sfx;
-            fpy += lp * sfy;
-            fpx += sub[k] * lp;
-            const A sxx = ste0, szz = ste2, sxz = ste1, sth = ste3;
-            A fsx = A(0.), fsy = A(0.);
-            fsx += sfx * sxx; fsx += sfy * sxz;
-            fsy += sfx * sxz; fsy += sfy * szz;
-            fsx += sub[k] * sth;
-            ax += A(-1.0) * fsx; ay += A(-1.0) * fsy;
-            ax += A(1.0) * fpx; ay += A(1.0) * fpy;
-        } else {
-            const A lpr = PLN(c.f.e_dampref, 2)[e];
-            A sxx = ste0 - lp, szz = ste2 - lp, sxz = ste1, sth = ste3 - lp;
-            A fsx = A(0.), fsy = A(0.);
-            fsx += sfx * sxx; fsx += sfy * sxz;
-            fsy += sfx * sxz; fsy += sfy * szz;
-            fsx += sub[k] * sth;
-            ax += A(-1.0) * fsx; ay += A(-1.0) * fsy;
-            if (damped) {
-                sxx += lpr; szz += lpr; sth += lpr;
-                A t0 = A(0.); t0 += sfx * (sigy * sxx); t0 += sfy * (sigx * sxz);
-                alx += t0 * dt;
-                A t1 = A(0.); t1 += sfx * (sigy * sxz); t1 += sfy * (sigx * szz);
-                aly += t1 * dt;
-                alx += (sigx + sigy) * sub[k] * sth * dt;
+            const long long e = cl[k];
+            const A sfx = GEO(c.g_v_suf, 2 * k), sfy = GEO(c.g_v_suf, 2 * k + 1);
+            const A lp = A(c.f.e_pre[e]) + A(c.f.e_q[e]);
+            const A ste0 = c.f.e_ste[e], ste1 = PLN(c.f.e_ste, 1)[e], ste2 = PLN(c.f.e_ste, 2)[e],
+                    ste3 = PLN(c.f.e_ste, 3)[e];
+            if (!pml) {
+                A fpx = A(0.), fpy = A(0.);
+                fpx += lp * sfx;
+                fpy += lp * sfy;
+                fpx += sub[k] * lp;
+                const A sxx = ste0, szz = ste2, sxz = ste1, sth = ste3;
+                A fsx = A(0.), fsy = A(0.);
+                fsx += sfx * sxx; fsx += sfy * sxz;
+                fsy += sfx * sxz; fsy += sfy * szz;
+                fsx += sub[k] * sth;
+                ax += A(-1.0) * fsx; ay += A(-1.0) * fsy;
+                ax += A(1.0) * fpx; ay += A(1.0) * fpy;
+            } else {
+                const A lpr = PLN(c.f.e_dampref, 2)[e];
+                A sxx = ste0 - lp, szz = ste2 - lp, sxz = ste1, sth = ste3 - lp;
+                A fsx = A(0.), fsy = A(0.);
+                fsx += sfx * sxx; fsx += sfy * sxz;
+                fsy += sfx * sxz; fsy += sfy * szz;
+                fsx += sub[k] * sth;
+                ax += A(-1.0) * fsx; ay += A(-1.0) * fsy;
+                if (damped) {
+                    sxx += lpr; szz += lpr; sth += lpr;
+                    A t0 = A(0.); t0 += sfx * (sigy * sxx); t0 += sfy * (sigx * sxz);
+                    alx += t0 * dt;
+                    A t1 = A(0.); t1 += sfx * (sigy * sxz); t1 += sfy * (sigx * szz);
+                    aly += t1 * dt;
+                    alx += (sigx + sigy) * sub[k] * sth * dt;
+                }
             }
+            const A lv = GEO(c.g_v_vol, 1 + k);
+            vmass += lv * A(c.f.e_den[e]);
+            vvol += lv;
         }
-        const A lv = GEO(c.g_v_vol, 1 + k);
-        vmass += lv * A(c.f.e_den[e]);
-        vvol += lv;
-    }
-    if (damped) {
-        alx -= A(c.rp.alpha_damp_x) * alx * dt;
-        aly -= A(c.rp.alpha_damp_y) * aly * dt;
-        ax += A(-1.0) * alx; ay += A(-1.0) * aly;
-    }
-    if (pml) { c.f.v_alpha[p] = alx; PLN(c.f.v_alpha, 1)[p] = aly; }
+        if (damped) {
+            alx -= A(c.rp.alpha_damp_x) * alx * dt;
+            aly -= A(c.rp.alpha_damp_y) * aly * dt;
+            ax += A(-1.0) * alx; ay += A(-1.0) * aly;
+        }
+        if (pml) { c.f.v_alpha[p] = alx; PLN(c.f.v_alpha, 1)[p] = aly; }
 
-    A ancx = A(0.), ancy = A(0.);
-    // where all nine weights are zero (outside the ANC band) the stencil sums to +0 and the term
-    // is +0: the weights are not read there
-    const bool lap = (c.lap_mask[(long long)j * (c.d.P >> 5) + (i >> 5)] >> (i & 31)) & 1u;
-    if (!vert_pad(c, i, j) && lap) {
-        A lvx = A(0.), lvy = A(0.);
-        int k = 0;
-        for (int dj = -1; dj <= 1; ++dj)
-            for (int di = -1; di <= 1; ++di, ++k) {
-                const long long q = KIDX(i + di, j + dj);
-                const A w = PLN(c.f.v_laplace, k)[p];
-                lvx += w * A(c.f.v_vel[q]);
-                lvy += w * A(PLN(c.f.v_vel, 1)[q]);
-            }
-        const A sc = A(5.0e3) * sqrt(fabs(sub[0]) + fabs(sub[2]));
-        ancx = sc * lvx;
-        ancy = sc * lvy;
-    }
-    if (PLN(c.f.v_mass, 1)[p] >= A(1.)) { ancx = A(0.); ancy = A(0.); }
-    if (vmass > A(SALEC_TOLRHO) * vvol) {
-        const A s = A(1.0) / vmass;
-        ax *= s; ay *= s;
-        ax += A(1.0) * A(c.f.v_bf[p]); ay += A(1.0) * A(PLN(c.f.v_bf, 1)[p]);
-        ax += A(c.rp.anc) * ancx; ay += A(c.rp.anc) * ancy;
-    } else if (pml) {
-        ax = c.f.v_bf[p]; ay = PLN(c.f.v_bf, 1)[p];
-    } else {
-        ax = A(0.); ay = A(0.);
-    }
-    if (fabs(ax) < A(c.rp.acceleration_min * 1)) ax = A(0.);
-    if (fabs(ay) < A(c.rp.acceleration_min * 1)) ay = A(0.);
-    c.f.v_acc[p] = ax;
-    PLN(c.f.v_acc, 1)[p] = ay;
+        A ancx = A(0.), ancy = A(0.);
+        // where all nine weights are zero (outside the ANC band) the stencil sums to +0 and the term
+        // is +0: the weights are not read there
+        const bool lap = (c.lap_mask[(long long)j * (c.d.P >> 5) + (i >> 5)] >> (i & 31)) & 1u;
+        if (!vert_pad(c, i, j) && lap) {
+            A lvx = A(0.), lvy = A(0.);
+            int k = 0;
+            for (int dj = -1; dj <= 1; ++dj)
+                for (int di = -1; di <= 1; ++di, ++k) {
+                    const long long q = KIDX(i + di, j + dj);
+                    const A w = PLN(c.f.v_laplace, k)[p];
+                    lvx += w * A(c.f.v_vel[q]);
+                    lvy += w * A(PLN(c.f.v_vel, 1)[q]);
+                }
+            const A sc = A(5.0e3) * sqrt(fabs(sub[0]) + fabs(sub[2]));
+            ancx = sc * lvx;
+            ancy = sc * lvy;
+        }
+        if (PLN(c.f.v_mass, 1)[p] >= A(1.)) { ancx = A(0.); ancy = A(0.); }
+        if (vmass > A(SALEC_TOLRHO) * vvol) {
+            const A s = A(1.0) / vmass;
+            ax *= s; ay *= s;
+            ax += A(1.0) * A(c.f.v_bf[p]); ay += A(1.0) * A(PLN(c.f.v_bf, 1)[p]);
+            ax += A(c.rp.anc) * ancx; ay += A(c.rp.anc) * ancy;
+        } else if (pml) {
+            ax = c.f.v_bf[p]; ay = PLN(c.f.v_bf, 1)[p];
+        } else {
+            ax = A(0.); ay = A(0.);
+        }
+        if (fabs(ax) < A(c.rp.acceleration_min * 1)) ax = A(0.);
+        if (fabs(ay) < A(c.rp.acceleration_min * 1)) ay = A(0.);
+        c.f.v_acc[p] = ax;
+        PLN(c.f.v_acc, 1)[p] = ay;
     });
 }
 
@@ -1013,15 +1013,15 @@ __global__ void k_vertex_displacement(const CtxT<R> c)
 {
     grid_dependency();
     for_points<true>(c, 0, [&](int i, int j) {
-    if (!vert_active(c, i, j)) return;
-    const long long p = KIDX(i, j);
-    const double dt = c.scal->dt;
-    const double hdt2 = 0.5 * dt * dt;
-    for (int k = 0; k < 2; ++k) {
-        const double v = PLN(c.f.v_vel, k)[p], a = PLN(c.f.v_acc, k)[p];
-        PLN(c.f.v_dis, k)[p] = dt * v + hdt2 * a;
-        PLN(c.f.v_vel, k)[p] = v + dt * a;
-    }
+        if (!vert_active(c, i, j)) return;
+        const long long p = KIDX(i, j);
+        const double dt = c.scal->dt;
+        const double hdt2 = 0.5 * dt * dt;
+        for (int k = 0; k < 2; ++k) {
+            const double v = PLN(c.f.v_vel, k)[p], a = PLN(c.f.v_acc, k)[p];
+            PLN(c.f.v_dis, k)[p] = dt * v + hdt2 * a;
+            PLN(c.f.v_vel, k)[p] = v + dt * a;
+        }
     });
 }
 
@@ -1288,164 +1288,164 @@ __global__ void SALEC_BOUNDS_FLUX k_flux(const CtxT<R> c, int tracer_blocks)
         return;
     }
     for_points<false>(c, tracer_blocks, [&](int i, int j) {
-    if (i >= c.d.enx || j >= c.d.eny) return;
-    constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
-    const int nmat = NM > 0 ? NM : c.d.nmat;
-    const long long p = KIDX(i, j);
-    const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
-    double px[4], py[4], dx[4], dy[4], lv, bv, rv, uv;
-    cell_swept_volumes(c, i, j, px, py, dx, dy, lv, bv, rv, uv);
-    double vof[MM];
-    #pragma unroll
-    for (int m = 0; m < nmat; ++m) vof[m] = PLN(c.f.m_vof, m)[p];
-    const double evol = c.f.e_vol[p];
-    double flux[MM][4];
-    #pragma unroll
-    for (int m = 0; m < nmat; ++m) flux[m][0] = flux[m][1] = flux[m][2] = flux[m][3] = 0.;
-
-    // primary material: vacuum, or the largest fraction when the cell holds no vacuum; selected
-    // with compare loops so that the per-material arrays stay in registers
-    int prim = 0;
-    double vprim = vof[0];
-    if (vof[0] < SALEC_TOLVOF) {
-#pragma unroll
-        for (int m = 1; m < nmat; ++m)
-            if (vof[m] > vprim) { prim = m; vprim = vof[m]; }
-    }
-
-    double wpt[4];
-    if (vprim > 1.0 - SALEC_TOLVOF) {
-#pragma unroll
-        for (int m = 0; m < nmat; ++m)
-            if (m == prim) {
-                flux[m][0] = dmin(lv, 0);
-                flux[m][2] = -1.0 * dmin(rv, 0);
-                flux[m][1] = dmin(bv, 0);
-                flux[m][3] = -1.0 * dmin(uv, 0);
-            }
-        const double w = prim == 0 ? 1.0 : -0.25;
-        wpt[0] = wpt[1] = wpt[2] = wpt[3] = w;
-    } else {
-        double grd[12];
+        if (i >= c.d.enx || j >= c.d.eny) return;
+        constexpr int MM = NM > 0 ? NM : SALEC_MAXMAT;
+        const int nmat = NM > 0 ? NM : c.d.nmat;
+        const long long p = KIDX(i, j);
+        const long long vl[4] = {KIDX(i, j), KIDX(i + 1, j), KIDX(i + 1, j + 1), KIDX(i, j + 1)};
+        double px[4], py[4], dx[4], dy[4], lv, bv, rv, uv;
+        cell_swept_volumes(c, i, j, px, py, dx, dy, lv, bv, rv, uv);
+        double vof[MM];
         #pragma unroll
-        for (int k = 0; k < 8; ++k) grd[k] = GEO(c.g_e_grad, k);
-        double gx = 0., gy = 0.;
-        {
-            const auto *vv = PLN(c.f.v_vof, prim);
-            double vq[4];
-            #pragma unroll
-            for (int k = 0; k < 4; ++k) vq[k] = vv[vl[k]];
-            #pragma unroll
-            for (int k = 0; k < 4; ++k) gx += vq[k] * grd[k];
-            #pragma unroll
-            for (int k = 0; k < 4; ++k) gy += vq[k] * grd[4 + k];
+        for (int m = 0; m < nmat; ++m) vof[m] = PLN(c.f.m_vof, m)[p];
+        const double evol = c.f.e_vol[p];
+        double flux[MM][4];
+        #pragma unroll
+        for (int m = 0; m < nmat; ++m) flux[m][0] = flux[m][1] = flux[m][2] = flux[m][3] = 0.;
+
+        // primary material: vacuum, or the largest fraction when the cell holds no vacuum; selected
+        // with compare loops so that the per-material arrays stay in registers
+        int prim = 0;
+        double vprim = vof[0];
+        if (vof[0] < SALEC_TOLVOF) {
+    #pragma unroll
+            for (int m = 1; m < nmat; ++m)
+                if (vof[m] > vprim) { prim = m; vprim = vof[m]; }
         }
-        normalise2(gx, gy);
-        double ca = PLN(c.f.e_pos, 2)[p] * fabs(gx);
-        double cb = PLN(c.f.e_pos, 3)[p] * fabs(gy);
-        if (ca < cb) { double t = ca; ca = cb; cb = t; }
-        const double dstar = cut_length(vprim, ca, cb);
-        double lw[4];
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) { double s = 0.; s += gx * px[k]; s += gy * py[k]; lw[k] = s; }
-        const double mw = dmax(dmax(lw[0], lw[1]), dmax(lw[2], lw[3]));
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) lw[k] = lw[k] - mw + dstar;
-        if (prim == 0) { for (int k = 0; k < 4; ++k) wpt[k] = lw[k]; }
-        else wpt[0] = wpt[1] = wpt[2] = wpt[3] = -0.25;
-        double fp[4];
-        fp[0] = face_ratio(lw[3], lw[0]);
-        fp[2] = face_ratio(lw[2], lw[1]);
-        fp[1] = face_ratio(lw[0], lw[1]);
-        fp[3] = face_ratio(lw[3], lw[2]);
-        double cr = dmin(lv, 0.0) + dmin(rv, 0) + dmin(bv, 0) + dmin(uv, 0);
-        cr = fabs(cr) / evol;
-        // neighbours l, b, r, u (the cell itself where the neighbour is off the mesh)
-        long long nb[4] = {KIDX(i - 1, j), KIDX(i, j - 1), KIDX(i + 1, j), KIDX(i, j + 1)};
-        if (i - 1 < 0) nb[0] = p;
-        if (j - 1 < 0) nb[1] = p;
-        if (i + 1 >= c.d.enx) nb[2] = p;
-        if (j + 1 >= c.d.eny) nb[3] = p;
-        // face normals l, b, r, u
-        const long long fb[4] = {KIDX(i, j), KIDX(i, j), KIDX(i + 1, j), KIDX(i, j + 1)};
-        double fnx[4], fny[4];
-        fnx[0] = c.f.bx_normal[fb[0]]; fny[0] = PLN(c.f.bx_normal, 1)[fb[0]];
-        fnx[2] = c.f.bx_normal[fb[2]]; fny[2] = PLN(c.f.bx_normal, 1)[fb[2]];
-        fnx[1] = c.f.by_normal[fb[1]]; fny[1] = PLN(c.f.by_normal, 1)[fb[1]];
-        fnx[3] = c.f.by_normal[fb[3]]; fny[3] = PLN(c.f.by_normal, 1)[fb[3]];
-        double fnp[MM][4];
-        double snp[4] = {0., 0., 0., 0.};
-        #pragma unroll
-        for (int m = 0; m < nmat; ++m) fnp[m][0] = fnp[m][1] = fnp[m][2] = fnp[m][3] = 0.;
-        #pragma unroll
-        for (int m = 1; m < nmat; ++m) {
-            if (m == prim) continue;
-            const auto *vv = PLN(c.f.v_vof, m);
-            double vq[4];
+
+        double wpt[4];
+        if (vprim > 1.0 - SALEC_TOLVOF) {
+    #pragma unroll
+            for (int m = 0; m < nmat; ++m)
+                if (m == prim) {
+                    flux[m][0] = dmin(lv, 0);
+                    flux[m][2] = -1.0 * dmin(rv, 0);
+                    flux[m][1] = dmin(bv, 0);
+                    flux[m][3] = -1.0 * dmin(uv, 0);
+                }
+            const double w = prim == 0 ? 1.0 : -0.25;
+            wpt[0] = wpt[1] = wpt[2] = wpt[3] = w;
+        } else {
+            double grd[12];
             #pragma unroll
-            for (int k = 0; k < 4; ++k) vq[k] = vv[vl[k]];
-            double ngx = 0., ngy = 0.;
+            for (int k = 0; k < 8; ++k) grd[k] = GEO(c.g_e_grad, k);
+            double gx = 0., gy = 0.;
+            {
+                const auto *vv = PLN(c.f.v_vof, prim);
+                double vq[4];
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) vq[k] = vv[vl[k]];
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) gx += vq[k] * grd[k];
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) gy += vq[k] * grd[4 + k];
+            }
+            normalise2(gx, gy);
+            double ca = PLN(c.f.e_pos, 2)[p] * fabs(gx);
+            double cb = PLN(c.f.e_pos, 3)[p] * fabs(gy);
+            if (ca < cb) { double t = ca; ca = cb; cb = t; }
+            const double dstar = cut_length(vprim, ca, cb);
+            double lw[4];
             #pragma unroll
-            for (int k = 0; k < 4; ++k) ngx += vq[k] * grd[k];
+            for (int k = 0; k < 4; ++k) { double s = 0.; s += gx * px[k]; s += gy * py[k]; lw[k] = s; }
+            const double mw = dmax(dmax(lw[0], lw[1]), dmax(lw[2], lw[3]));
             #pragma unroll
-            for (int k = 0; k < 4; ++k) ngy += vq[k] * grd[4 + k];
-            normalise2(ngx, ngy);
-            const double *ev = PLN(c.f.m_vof, m);
-            const double up[4] = {ev[nb[0]], ev[nb[1]], ev[nb[2]], ev[nb[3]]};
-            const double ac[4] = {up[2], up[3], up[0], up[1]};
+            for (int k = 0; k < 4; ++k) lw[k] = lw[k] - mw + dstar;
+            if (prim == 0) { for (int k = 0; k < 4; ++k) wpt[k] = lw[k]; }
+            else wpt[0] = wpt[1] = wpt[2] = wpt[3] = -0.25;
+            double fp[4];
+            fp[0] = face_ratio(lw[3], lw[0]);
+            fp[2] = face_ratio(lw[2], lw[1]);
+            fp[1] = face_ratio(lw[0], lw[1]);
+            fp[3] = face_ratio(lw[3], lw[2]);
+            double cr = dmin(lv, 0.0) + dmin(rv, 0) + dmin(bv, 0) + dmin(uv, 0);
+            cr = fabs(cr) / evol;
+            // neighbours l, b, r, u (the cell itself where the neighbour is off the mesh)
+            long long nb[4] = {KIDX(i - 1, j), KIDX(i, j - 1), KIDX(i + 1, j), KIDX(i, j + 1)};
+            if (i - 1 < 0) nb[0] = p;
+            if (j - 1 < 0) nb[1] = p;
+            if (i + 1 >= c.d.enx) nb[2] = p;
+            if (j + 1 >= c.d.eny) nb[3] = p;
+            // face normals l, b, r, u
+            const long long fb[4] = {KIDX(i, j), KIDX(i, j), KIDX(i + 1, j), KIDX(i, j + 1)};
+            double fnx[4], fny[4];
+            fnx[0] = c.f.bx_normal[fb[0]]; fny[0] = PLN(c.f.bx_normal, 1)[fb[0]];
+            fnx[2] = c.f.bx_normal[fb[2]]; fny[2] = PLN(c.f.bx_normal, 1)[fb[2]];
+            fnx[1] = c.f.by_normal[fb[1]]; fny[1] = PLN(c.f.by_normal, 1)[fb[1]];
+            fnx[3] = c.f.by_normal[fb[3]]; fny[3] = PLN(c.f.by_normal, 1)[fb[3]];
+            double fnp[MM][4];
+            double snp[4] = {0., 0., 0., 0.};
+            #pragma unroll
+            for (int m = 0; m < nmat; ++m) fnp[m][0] = fnp[m][1] = fnp[m][2] = fnp[m][3] = 0.;
+            #pragma unroll
+            for (int m = 1; m < nmat; ++m) {
+                if (m == prim) continue;
+                const auto *vv = PLN(c.f.v_vof, m);
+                double vq[4];
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) vq[k] = vv[vl[k]];
+                double ngx = 0., ngy = 0.;
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) ngx += vq[k] * grd[k];
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) ngy += vq[k] * grd[4 + k];
+                normalise2(ngx, ngy);
+                const double *ev = PLN(c.f.m_vof, m);
+                const double up[4] = {ev[nb[0]], ev[nb[1]], ev[nb[2]], ev[nb[3]]};
+                const double ac[4] = {up[2], up[3], up[0], up[1]};
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    fnp[m][k] = algebraic_ratio(up[k], vof[m], ac[k], cr, fnx[k], fny[k], ngx, ngy);
+                    snp[k] += fnp[m][k];
+                }
+            }
             #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                fnp[m][k] = algebraic_ratio(up[k], vof[m], ac[k], cr, fnx[k], fny[k], ngx, ngy);
-                snp[k] += fnp[m][k];
+                if (snp[k] > SALEC_TOLVOF) {
+                    #pragma unroll
+                    for (int m = 1; m < nmat; ++m) fnp[m][k] = fnp[m][k] / snp[k];
+                } else {
+                    #pragma unroll
+                    for (int m = 1; m < nmat; ++m) fnp[m][k] = vof[m] / (1.0 - vprim);
+                }
             }
-        }
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (snp[k] > SALEC_TOLVOF) {
-                #pragma unroll
-                for (int m = 1; m < nmat; ++m) fnp[m][k] = fnp[m][k] / snp[k];
-            } else {
-                #pragma unroll
-                for (int m = 1; m < nmat; ++m) fnp[m][k] = vof[m] / (1.0 - vprim);
-            }
-        }
-        #pragma unroll
-        for (int m = 0; m < nmat; ++m) {
-            if (m == prim) {
-                flux[m][0] = dmin(lv, 0.0) * fp[0];
-                flux[m][2] = -1.0 * dmin(rv, 0.0) * fp[2];
-                flux[m][1] = dmin(bv, 0.0) * fp[1];
-                flux[m][3] = -1.0 * dmin(uv, 0.0) * fp[3];
-            } else {
-                flux[m][0] = dmin(lv, 0.0) * (1.0 - fp[0]) * fnp[m][0];
-                flux[m][2] = -1.0 * dmin(rv, 0.0) * (1.0 - fp[2]) * fnp[m][2];
-                flux[m][1] = dmin(bv, 0.0) * (1.0 - fp[1]) * fnp[m][1];
-                flux[m][3] = -1.0 * dmin(uv, 0.0) * (1.0 - fp[3]) * fnp[m][3];
-            }
-        }
-    }
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) PLN(c.f.e_wpt, k)[p] = wpt[k];
-
-    // cap the out-flux of each material by its content
-    #pragma unroll
-    for (int m = 1; m < nmat; ++m) {
-        double d = 0.;
-        d += flux[m][0] * 1.0; d += flux[m][1] * 1.0; d += flux[m][2] * -1.0; d += flux[m][3] * -1.0;
-        const double out = -1.0 * d;
-        if (out > vof[m] * evol) {
-            const double s = vof[m] * evol / out;
             #pragma unroll
-            for (int k = 0; k < 4; ++k) flux[m][k] *= s;
+            for (int m = 0; m < nmat; ++m) {
+                if (m == prim) {
+                    flux[m][0] = dmin(lv, 0.0) * fp[0];
+                    flux[m][2] = -1.0 * dmin(rv, 0.0) * fp[2];
+                    flux[m][1] = dmin(bv, 0.0) * fp[1];
+                    flux[m][3] = -1.0 * dmin(uv, 0.0) * fp[3];
+                } else {
+                    flux[m][0] = dmin(lv, 0.0) * (1.0 - fp[0]) * fnp[m][0];
+                    flux[m][2] = -1.0 * dmin(rv, 0.0) * (1.0 - fp[2]) * fnp[m][2];
+                    flux[m][1] = dmin(bv, 0.0) * (1.0 - fp[1]) * fnp[m][1];
+                    flux[m][3] = -1.0 * dmin(uv, 0.0) * (1.0 - fp[3]) * fnp[m][3];
+                }
+            }
         }
-    }
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) PLN(c.f.e_wpt, k)[p] = wpt[k];
 
-    const bool odd = !REC && c.scal->odd_fractions;
-    // faces l, b, r, u
-    store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i, j), lv, flux, 0, p, nmat, odd);
-    store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j), bv, flux, 1, p, nmat, odd);
-    store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i + 1, j), rv, flux, 2, p, nmat, odd);
-    store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j + 1), uv, flux, 3, p, nmat, odd);
+        // cap the out-flux of each material by its content
+        #pragma unroll
+        for (int m = 1; m < nmat; ++m) {
+            double d = 0.;
+            d += flux[m][0] * 1.0; d += flux[m][1] * 1.0; d += flux[m][2] * -1.0; d += flux[m][3] * -1.0;
+            const double out = -1.0 * d;
+            if (out > vof[m] * evol) {
+                const double s = vof[m] * evol / out;
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) flux[m][k] *= s;
+            }
+        }
+
+        const bool odd = !REC && c.scal->odd_fractions;
+        // faces l, b, r, u
+        store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i, j), lv, flux, 0, p, nmat, odd);
+        store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j), bv, flux, 1, p, nmat, odd);
+        store_face<R, NM, POR, REC>(c, c.f.bx_phi + KIDX(i + 1, j), rv, flux, 2, p, nmat, odd);
+        store_face<R, NM, POR, REC>(c, c.f.by_phi + KIDX(i, j + 1), uv, flux, 3, p, nmat, odd);
     });
 }
 
@@ -2021,44 +2021,44 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
 {
     grid_dependency();
     for_points<false>(c, 0, [&](int i, int j) {
-    if (i >= c.d.enx || j >= c.d.eny) return;
-    const long long p = KIDX(i, j);
-    const bool interior = cell_interior(c, i, j);
-    const double dt = c.scal->dt;
-    const bool remap = do_remap && interior;
-    const bool damp = do_damp && c.rp.damp_time > c.scal->time && c.rp.damp_type != 4 && c.rp.damp_type != 5;
-    const bool ejecta = do_ejecta && interior;
-    const bool state = do_state && interior;
-    if (!DUAL && !(remap || damp || ejecta || state)) return;
-    CellState<NM, POR> s;
-    if (remap && DUAL && c.scal->odd_fractions) remap_cell<R, NM, POR, P3, DUAL, DUAL>(c, i, j, p, s);
-    else if (remap) remap_cell<R, NM, POR, P3, DUAL>(c, i, j, p, s);
-    else load_cell<R, NM, POR>(c, p, s);
-    bool dirty = remap || DUAL;
-    if (damp) dirty |= damp_cell<R, NM, POR>(c, p, dt, s);
-    if (ejecta) {
-        ejecta_drag_cell<R, NM, POR>(c, i, j, p, dt, s);
-        dirty = true;
-    }
-    if (dirty) store_cell<R, NM, POR>(c, p, s, !state);   // the EOS pass writes e_den itself
-    if (DUAL) {
-        bool odd = false;
-        #pragma unroll
-        for (int m = 0; m < (NM > 0 ? NM : c.d.nmat); ++m) odd = odd || !(s.vof[m] >= 0.);
-        if (odd) c.scal->odd_next = 1u;
-    }
-    if (state) state_cell<R, NM, POR>(c, p, s);
-    if (DUAL && c.vacuum) {
-        // a warp covers one segment; only whole interior ones count
-        const int i0 = i & ~31;
-        if (i0 < 2 || i0 + 31 > c.d.enx - 3 || j < 2 || j > c.d.eny - 3) return;
-        bool empty = s.vof[0] == 1.0 && s.eden == 0.0;
-        #pragma unroll
-        for (int m = 1; m < (NM > 0 ? NM : c.d.nmat); ++m)
-            empty = empty && s.vof[m] == 0.0 && s.rho[m] == 0.0 && s.eng[m] == 0.0;
-        empty = __all_sync(0xffffffffu, empty);
-        if (i == i0) c.vacuum[c.tx * j + (i >> 5)] = empty;
-    }
+        if (i >= c.d.enx || j >= c.d.eny) return;
+        const long long p = KIDX(i, j);
+        const bool interior = cell_interior(c, i, j);
+        const double dt = c.scal->dt;
+        const bool remap = do_remap && interior;
+        const bool damp = do_damp && c.rp.damp_time > c.scal->time && c.rp.damp_type != 4 && c.rp.damp_type != 5;
+        const bool ejecta = do_ejecta && interior;
+        const bool state = do_state && interior;
+        if (!DUAL && !(remap || damp || ejecta || state)) return;
+        CellState<NM, POR> s;
+        if (remap && DUAL && c.scal->odd_fractions) remap_cell<R, NM, POR, P3, DUAL, DUAL>(c, i, j, p, s);
+        else if (remap) remap_cell<R, NM, POR, P3, DUAL>(c, i, j, p, s);
+        else load_cell<R, NM, POR>(c, p, s);
+        bool dirty = remap || DUAL;
+        if (damp) dirty |= damp_cell<R, NM, POR>(c, p, dt, s);
+        if (ejecta) {
+            ejecta_drag_cell<R, NM, POR>(c, i, j, p, dt, s);
+            dirty = true;
+        }
+        if (dirty) store_cell<R, NM, POR>(c, p, s, !state);   // the EOS pass writes e_den itself
+        if (DUAL) {
+            bool odd = false;
+            #pragma unroll
+            for (int m = 0; m < (NM > 0 ? NM : c.d.nmat); ++m) odd = odd || !(s.vof[m] >= 0.);
+            if (odd) c.scal->odd_next = 1u;
+        }
+        if (state) state_cell<R, NM, POR>(c, p, s);
+        if (DUAL && c.vacuum) {
+            // a warp covers one segment; only whole interior ones count
+            const int i0 = i & ~31;
+            if (i0 < 2 || i0 + 31 > c.d.enx - 3 || j < 2 || j > c.d.eny - 3) return;
+            bool empty = s.vof[0] == 1.0 && s.eden == 0.0;
+            #pragma unroll
+            for (int m = 1; m < (NM > 0 ? NM : c.d.nmat); ++m)
+                empty = empty && s.vof[m] == 0.0 && s.rho[m] == 0.0 && s.eng[m] == 0.0;
+            empty = __all_sync(0xffffffffu, empty);
+            if (i == i0) c.vacuum[c.tx * j + (i >> 5)] = empty;
+        }
     });
 }
 
