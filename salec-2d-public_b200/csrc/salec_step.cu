@@ -1527,6 +1527,28 @@ __device__ __forceinline__ void store_cell(const CtxT<R> &c, long long p, const 
     if (den) c.f.e_den[p] = s.eden;
 }
 
+// Which of a cell's donors lie across its faces l, b, r, u (bits 0 to 3), in a cycle that begins with a NaN or
+// a negative fraction somewhere, or with fractions that the graph has not seen (a caller's, or the phases').
+// The side is the sign of the volumes that are not NaN, or, where they differ in sign, the one that the flux
+// stored; volumes that are all NaN or zero make every member they touch NaN, whichever cell they leave.
+// Out of line and ahead of the remap's loads, so that the rare case takes one register of the common one.
+// us a cycle without and with it: layered 1024x1024 389 and 387, layered 600x450 mixed 149.5 and 150.4,
+// 12 meshes of 128 to 512 mixed 10.5 and 10.6 ms for 32. A second instance of the remap took 393, 151.6 and
+// 10.8, looking at the signs in every cycle 1 to 2 percent.
+#define SALEC_PLAIN_SIDES 0x80000000u
+__device__ __noinline__ unsigned odd_sides(const double *left, const double *bottom, long long pitch, long long PL, int nmat)
+{
+    unsigned sides = 0u;
+    for (int k = 0; k < 4; ++k) {
+        const double *f = (k & 1 ? bottom : left) + (k < 2 ? 0 : k == 2 ? 1 : pitch);
+        bool pos = false, neg = false;
+        for (int m = 0; m < nmat; ++m) { pos = pos || f[m * PL] > 0.; neg = neg || f[m * PL] < 0.; }
+        const double side = pos && neg ? f[nmat * PL] : pos ? 1. : neg ? -1. : 0.;
+        if ((k < 2 ? side : -side) > 0.) sides |= 1u << k;
+    }
+    return sides;
+}
+
 // advect_flux_default (src/advect.c:26-302) for one interior cell, into registers. The loads
 // that do not depend on the flow (the cell's own state and the material volumes of its four
 // faces) are all issued before the first dependent one, the own state only where that leaves
@@ -1535,14 +1557,8 @@ __device__ __forceinline__ void store_cell(const CtxT<R> &c, long long p, const 
 // record; the net volume of the face says which cell that is. With fractions between 0 and 1 its material
 // volumes have one sign, but for roundings of the algebraic ones: those are nonzero only for a material
 // the cell holds, and no cap scales a held material's volume down to a rounding.
-// ODD: the remap of a cycle that begins with a NaN or a negative fraction somewhere, or with fractions
-// that the graph has not seen (a caller's, or the phases'). The side is then the sign of the volumes that are
-// not NaN, or, where they differ in sign, the one that the flux stored; volumes that are all NaN or zero
-// make every member they touch NaN, whichever cell they leave. An instance of its own beside the other:
-// us a cycle, layered 1024x1024 and layered 600x450 mixed, 385 and 147.5 without it, 389 and 149 with it,
-// 1 to 2 percent more with the signs looked at in every cycle (spills), 396 and 149.7 with its faces in a
-// loop.
-template <class R, int NM, bool POR, bool P3, bool DUAL, bool ODD = false>
+// A cycle with odd fractions asks odd_sides() instead.
+template <class R, int NM, bool POR, bool P3, bool DUAL>
 __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long long p, CellState<NM, POR> &s)
 {
     constexpr int MM = CellState<NM, POR>::MM;
@@ -1553,6 +1569,8 @@ __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long 
     const double *face[4] = {c.f.bx_phi + KIDX(i, j), c.f.by_phi + KIDX(i, j), c.f.bx_phi + KIDX(i + 1, j),
                              c.f.by_phi + KIDX(i, j + 1)};
     const double dir[4] = {1.0, 1.0, -1.0, -1.0};
+    unsigned sides = SALEC_PLAIN_SIDES;
+    if (DUAL && c.scal->odd_fractions) sides = odd_sides(face[0], face[1], c.d.P, PL, nmat);
     double fv[4][MM];
     #pragma unroll
     for (int k = 0; k < 4; ++k)
@@ -1608,13 +1626,7 @@ __device__ __forceinline__ void remap_cell(const CtxT<R> &c, int i, int j, long 
             #pragma unroll
             for (int m = 0; m < nmat; ++m) { in += dir[k] * fv[k][m]; flow = flow || fv[k][m] != 0.0; }
             if (!flow) continue;
-            if (ODD) {
-                bool pos = false, neg = false;
-                #pragma unroll
-                for (int m = 0; m < nmat; ++m) { pos = pos || fv[k][m] > 0.; neg = neg || fv[k][m] < 0.; }
-                in = dir[k] * (pos && neg ? face[k][nmat * PL] : pos ? 1. : neg ? -1. : 0.);
-            }
-            const long long q = in > 0. ? nb[k] : p;
+            const long long q = (sides & SALEC_PLAIN_SIDES ? in > 0. : (sides >> k & 1u) != 0u) ? nb[k] : p;
             // the donor's members in one batch, then every material's share
             double rf[MM], ef[MM], pf[MM], g[11];
             #pragma unroll
@@ -2031,8 +2043,7 @@ __global__ void SALEC_BOUNDS_REMAP k_remap_damp_state(const CtxT<R> c, int do_re
         const bool state = do_state && interior;
         if (!DUAL && !(remap || damp || ejecta || state)) return;
         CellState<NM, POR> s;
-        if (remap && DUAL && c.scal->odd_fractions) remap_cell<R, NM, POR, P3, DUAL, DUAL>(c, i, j, p, s);
-        else if (remap) remap_cell<R, NM, POR, P3, DUAL>(c, i, j, p, s);
+        if (remap) remap_cell<R, NM, POR, P3, DUAL>(c, i, j, p, s);
         else load_cell<R, NM, POR>(c, p, s);
         bool dirty = remap || DUAL;
         if (damp) dirty |= damp_cell<R, NM, POR>(c, p, dt, s);
